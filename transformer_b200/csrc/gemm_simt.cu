@@ -12,7 +12,13 @@
 //  * DUAL: B[g] is [2N, K]; the block computes gate = A.B[g][n] and up = A.B[g][N + n] together and
 //    stores silu(gate) * up  (swiglu, compute.rs:324-326), in float, rounded once.
 //  Any M, N, K >= 1; edges are predicated.
+//
+// Three kernels: gemm_simt_kernel takes anything; for float with 16-byte rows, gemm_rows_f32_kernel streams the weights
+// past a few rows (decoding), and gemm_tile_f32_kernel multiplies tiles fed by cp.async (prompts).
+#include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
 #include "common.cuh"
+
+#include <type_traits>
 
 struct GemmArgs {
     const void* A;
@@ -28,6 +34,36 @@ struct GemmArgs {
     long long c_batch_stride;   // zero without batches
 };
 
+// Which rows does tile `tile` of BM rows hold?  False: none.
+template <int BM>
+__device__ __forceinline__ bool gemm_tile_rows(const GemmArgs& a, int tile, int& g, int& row0, int& row_end) {
+    g = 0;
+    row0 = tile * BM;
+    row_end = a.M;
+    if (!a.group_offsets) return row0 < a.M;
+    int cum = 0;
+    for (g = 0; g < a.G; ++g) {
+        const int lo = a.group_offsets[g], hi = a.group_offsets[g + 1];
+        const int tiles = (hi - lo + BM - 1) / BM;
+        if (tile < cum + tiles) {
+            row0 = lo + (tile - cum) * BM;
+            row_end = hi;
+            return true;
+        }
+        cum += tiles;
+    }
+    return false;
+}
+
+__device__ __forceinline__ float gemm_act(float v, float v2, bool dual, const GluRule r) {
+    if (dual) return glu_apply(v, v2, r);
+    if (r.kind == TB_ACT_RELU2) {
+        v = fmaxf(v, 0.f);
+        v *= v;
+    }
+    return v;
+}
+
 #define GB_N 64
 #define GB_K 16
 
@@ -39,27 +75,8 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmArgs a) {
     __shared__ float Bs[GB_K][GB_N + 1];
     __shared__ float B2s[DUAL ? GB_K : 1][GB_N + 1];
 
-    // which group and rows does this block own?
-    int g = 0, row0 = 0, row_end = a.M;
-    if (a.group_offsets) {
-        int tile = blockIdx.x, cum = 0;
-        bool found = false;
-        for (g = 0; g < a.G; ++g) {
-            const int lo = a.group_offsets[g], hi = a.group_offsets[g + 1];
-            const int tiles = (hi - lo + BM - 1) / BM;
-            if (tile < cum + tiles) {
-                row0 = lo + (tile - cum) * BM;
-                row_end = hi;
-                found = true;
-                break;
-            }
-            cum += tiles;
-        }
-        if (!found) return;
-    } else {
-        row0 = blockIdx.x * BM;
-        if (row0 >= a.M) return;
-    }
+    int g, row0, row_end;
+    if (!gemm_tile_rows<BM>(a, blockIdx.x, g, row0, row_end)) return;
     const int n0 = blockIdx.y * GB_N;
     if (gridDim.z > 1) g = blockIdx.z;      // batches: every batch has a matrix of its own and all the rows
     const T* A = static_cast<const T*>(a.A) + (size_t)blockIdx.z * a.a_batch_stride;
@@ -131,22 +148,259 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmArgs a) {
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
             if (n >= a.N) continue;
-            float v = acc[i][j];
-            if (DUAL) {
-                v = glu_apply(v, acc2[i][j], a.glu);
-            } else if (a.glu.kind == TB_ACT_RELU2) {
-                v = fmaxf(v, 0.f);
-                v *= v;
-            }
-            stf(C + (size_t)m * a.ldc + n, v);
+            stf(C + (size_t)m * a.ldc + n, gemm_act(acc[i][j], acc2[DUAL ? i : 0][j], DUAL, a.glu));
         }
     }
+}
+
+// ---- a few rows (decoding) -----------------------------------------------------------------------------------------
+// Bound by reading the weights once.  A warp owns CT rows of W (DUAL: CT / 2 gate rows and their up rows) and every
+// WK-th piece of 128 entries of K: a lane holds 16 bytes of each row, so a warp has CT x 512 bytes in flight, and the
+// rows of A (up to MT at a time, from L1) meet them in registers.  WK warps of a block share its columns; a warp's
+// MT x CT sums are joined by a reduce-scatter (31 shuffles for 32 sums), the warps' through shared memory.  The general
+// kernel walks K in steps of 16 with two barriers each and was bound by that chain: 3 rows x 1,536
+// x 1,024 took 55.7 us and take 3.0 (2.1 TB/s), x 32,000 x 1,024 275 and 34 us (3.9 TB/s), 16 rows x 1,536 x 1,024 56.4
+// and 7.1 us; a decode step of three sequences (width 1,024, 8 layers, 8 experts of 512) 4.6 and 0.58 ms.
+template <int MT, int CT, bool DUAL>
+__global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, int wk_count) {
+    constexpr int COLS = DUAL ? CT / 2 : CT;
+    constexpr int SETS = MT * CT / 32;
+    static_assert(MT * CT % 32 == 0, "the reduce-scatter takes 32 sums at a time");
+    __shared__ float red[8][MT * CT];
+    pdl_sync();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wk = warp % wk_count, wn = warp / wk_count, wn_count = (blockDim.x >> 5) / wk_count;
+    const int g = blockIdx.y, n0 = (blockIdx.x * wn_count + wn) * COLS;
+    const int row_lo = a.group_offsets ? a.group_offsets[g] : 0, row_hi = a.group_offsets ? a.group_offsets[g + 1] : a.M;
+    if (row_lo >= row_hi) return;
+    const float* B = static_cast<const float*>(a.B) + (size_t)g * a.b_group_stride;
+    const float* A = static_cast<const float*>(a.A);
+    const float* wp[CT];
+#pragma unroll
+    for (int c = 0; c < CT; ++c) {      // columns past the end repeat the last one and are not stored
+        const int n = min(n0 + c % COLS, a.N - 1) + (DUAL && c >= COLS ? a.N : 0);
+        wp[c] = B + (size_t)n * a.ldb;
+    }
+    for (int chunk = row_lo; chunk < row_hi; chunk += MT) {
+        const int rows = min(MT, row_hi - chunk);
+        float acc[MT * CT];
+        const float* xp[MT];            // rows past the end repeat the last one and are not stored
+#pragma unroll
+        for (int i = 0; i < MT * CT; ++i) acc[i] = 0.f;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            const int r = chunk + min(m, rows - 1);
+            xp[m] = A + (size_t)(a.a_rows ? a.a_rows[r] : r) * a.lda;
+        }
+        for (int k = wk * 128 + lane * 4; k < a.K; k += wk_count * 128) {
+            float4 w[CT];
+#pragma unroll
+            for (int c = 0; c < CT; ++c) w[c] = __ldcs(reinterpret_cast<const float4*>(wp[c] + k));
+#pragma unroll
+            for (int m0 = 0; m0 < MT; m0 += 4) {
+                if (m0 < rows) {
+                    float4 x[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) x[m] = *reinterpret_cast<const float4*>(xp[m0 + m] + k);
+#pragma unroll
+                    for (int m = 0; m < 4; ++m)
+#pragma unroll
+                        for (int c = 0; c < CT; ++c) {
+                            float& v = acc[(m0 + m) * CT + c];
+                            v = fmaf(x[m].x, w[c].x, v);
+                            v = fmaf(x[m].y, w[c].y, v);
+                            v = fmaf(x[m].z, w[c].z, v);
+                            v = fmaf(x[m].w, w[c].w, v);
+                        }
+                }
+            }
+        }
+        if (chunk != row_lo) __syncthreads();       // the sums of the rows before have been read
+#pragma unroll
+        for (int set = 0; set < SETS; ++set) {
+            float* v = acc + set * 32;
+#pragma unroll
+            for (int half = 16; half > 0; half >>= 1) {      // a lane keeps the half of the sums that its bit names
+                const bool up = lane & half;
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                    const float keep = up ? v[i + half] : v[i], give = up ? v[i] : v[i + half];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+                }
+            }
+            red[warp][set * 32 + lane] = v[0];
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < wn_count * rows * COLS; idx += blockDim.x) {
+            const int c = idx % COLS, m = idx / COLS % rows, w_n = idx / (COLS * rows);
+            const int n = (blockIdx.x * wn_count + w_n) * COLS + c;
+            if (n >= a.N) continue;
+            float v = 0.f, v2 = 0.f;
+            for (int w = 0; w < wk_count; ++w) {
+                v += red[w_n * wk_count + w][m * CT + c];
+                if (DUAL) v2 += red[w_n * wk_count + w][m * CT + COLS + c];
+            }
+            static_cast<float*>(a.C)[(size_t)(chunk + m) * a.ldc + n] = gemm_act(v, v2, DUAL, a.glu);
+        }
+    }
+}
+
+template <int MT, int CT, bool DUAL>
+static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
+    // as many warps on K as it has pieces of 128 entries, up to eight; with fewer than four, more columns a block
+    const int wk = a.K >= 1024 ? 8 : a.K >= 512 ? 4 : a.K >= 256 ? 2 : 1;
+    const int warps = wk == 8 ? 8 : 4, cols = (DUAL ? CT / 2 : CT) * (warps / wk);
+    TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL>), dim3((a.N + cols - 1) / cols, a.G), warps * 32, 0, s, a, wk);
+}
+
+// ---- many rows (prompts) -------------------------------------------------------------------------------------------
+// 64 x 64 outputs a block, 32 x 32 a warp, 8 x 4 a thread; K in steps of 32 through a ring of three stages filled by
+// cp.async.  Four warps take the first 16 entries of a step and four the others, and their sums are joined at the end:
+// a prompt of a few hundred tokens has fewer tiles than the GPU has SMs, and one warp a scheduler does not hide the
+// latencies of its own loads (254 rows x 1,536 x 1,024: 85 us with four warps a block, 61 with eight; an expert's pair
+// for 254 tokens 110 and 73; 2,048 x 4,096 x 4,096, where tiles abound, 1,510 and 1,674).  Tiles lie in shared memory as in memory (K innermost, rows 36 floats apart: the eight
+// rows that a quarter of a warp reads start in different banks), so a thread's operands are 16-byte loads of four
+// entries of K: 12 of them feed 128 multiply-adds.  Bound by FFMA issue; the general kernel reads one float at a time
+// (8 loads for 16 multiply-adds) and waits for global memory in every step: 148, 274 and 3,236 us for these three.
+#define GT_BK 32
+#define GT_PITCH (GT_BK + 4)
+#define GT_STAGES 3
+template <bool DUAL>
+__global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
+    constexpr int NB = DUAL ? 2 : 1;
+    extern __shared__ __align__(16) float gt[];
+    constexpr int STAGE = (1 + NB) * 64 * GT_PITCH;        // A, then the one or two tiles of B
+    pdl_sync();
+    int g, row0, row_end;
+    if (!gemm_tile_rows<64>(a, blockIdx.x, g, row0, row_end)) return;
+    const int n0 = blockIdx.y * 64, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float* A = static_cast<const float*>(a.A);
+    const float* B = static_cast<const float*>(a.B) + (size_t)g * a.b_group_stride;
+    // a thread copies 16 bytes of rows r0 and r0 + 32 of each tile; rows and columns past the end repeat the last one
+    const int r0 = tid >> 3, kq = (tid & 7) * 4;
+    const float* src[(1 + NB) * 2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int m = min(row0 + r0 + 32 * i, row_end - 1), n = min(n0 + r0 + 32 * i, a.N - 1);
+        src[i] = A + (size_t)(a.a_rows ? a.a_rows[m] : m) * a.lda + kq;
+        src[2 + i] = B + (size_t)n * a.ldb + kq;
+        if (DUAL) src[2 * NB + i] = B + (size_t)(a.N + n) * a.ldb + kq;
+    }
+    const int steps = (a.K + GT_BK - 1) / GT_BK;
+    auto issue = [&](int step) {
+        float* st = gt + (step % GT_STAGES) * STAGE;
+        const int k = step * GT_BK;
+#pragma unroll
+        for (int i = 0; i < (1 + NB) * 2; ++i) {
+            float* dst = st + ((i >> 1) * 64 + r0 + 32 * (i & 1)) * GT_PITCH + kq;
+            if (k + kq < a.K) cp_async16((uint32_t)__cvta_generic_to_shared(dst), src[i] + k);
+            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float acc[NB][8][4];
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[b][i][j] = 0.f;
+#pragma unroll
+    for (int st = 0; st < GT_STAGES - 1; ++st) {
+        if (st < steps) issue(st);
+        cp_async_commit();
+    }
+    const int ty = lane >> 3, tx = lane & 7, wm = (warp >> 1 & 1) * 32, wn = (warp & 1) * 32;
+    const int k_half = warp >> 2;
+    for (int st = 0; st < steps; ++st) {
+        cp_async_wait<GT_STAGES - 2>();
+        __syncthreads();            // this stage is there for everyone, and everyone is done with the one before
+        if (st + GT_STAGES - 1 < steps) issue(st + GT_STAGES - 1);
+        cp_async_commit();
+        const float* As = gt + (st % GT_STAGES) * STAGE + (wm + ty) * GT_PITCH + k_half * (GT_BK / 2);
+        const float* Bs = gt + (st % GT_STAGES) * STAGE + (64 + wn + tx) * GT_PITCH + k_half * (GT_BK / 2);
+#pragma unroll 2
+        for (int k = 0; k < GT_BK / 2; k += 4) {
+            float4 av[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float4*>(As + 4 * i * GT_PITCH + k);
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 bv = *reinterpret_cast<const float4*>(Bs + (b * 64 + 8 * j) * GT_PITCH + k);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        float& v = acc[b][i][j];
+                        v = fmaf(av[i].x, bv.x, v);
+                        v = fmaf(av[i].y, bv.y, v);
+                        v = fmaf(av[i].z, bv.z, v);
+                        v = fmaf(av[i].w, bv.w, v);
+                    }
+                }
+        }
+    }
+    // the second half's sums to shared memory (a warp's 32 x NB values a lane, lane innermost), the first half adds them
+    __syncthreads();
+    float* part = gt + (warp & 3) * (NB * 1024) + lane;
+    if (k_half) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) part[(b * 32 + i) * 32] = acc[b][i >> 2][i & 3];
+    }
+    __syncthreads();
+    if (k_half) return;
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[b][i >> 2][i & 3] += part[(b * 32 + i) * 32];
+    float* C = static_cast<float*>(a.C);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = row0 + wm + ty + 4 * i;
+        if (m >= row_end) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + wn + tx + 8 * j;
+            if (n < a.N) C[(size_t)m * a.ldc + n] = gemm_act(acc[0][i][j], acc[NB - 1][i][j], DUAL, a.glu);
+        }
+    }
+}
+
+// The float kernels with 16-byte loads, for rows that start on such a boundary and K in multiples of four; false: the
+// caller takes the general kernel.  Up to 16 rows (a group, on average) the weights are what is read, and the rows are
+// taken 4, 8 or 16 at a time by what most groups hold, as gemm_skinny does; above, tiles.  Measured at the border: 16
+// rows x 1,536 x 1,024 7.1 us here, 17 rows 39 us in tiles; a pair of 8 experts (1,024 -> 512) 25 us for groups of 15 rows
+// here, 73 for groups of 25 in tiles (one tile a group, mostly empty, and the general kernel's 200 and 219).
+static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
+    if (a.K % 4 || a.lda % 4 || a.ldb % 4 || a.b_group_stride % 4 || (((uintptr_t)a.A | (uintptr_t)a.B) & 15)) return false;
+    if (a.M <= 16 * a.G && a.G <= 65535) {
+        const int usual = a.G > 1 ? (3 * a.M / a.G + 1) / 2 : a.M;
+        if (usual <= 4) dual ? gemm_rows_f32_go<4, 8, true>(a, s) : gemm_rows_f32_go<4, 8, false>(a, s);
+        else if (usual <= 8) dual ? gemm_rows_f32_go<8, 8, true>(a, s) : gemm_rows_f32_go<8, 8, false>(a, s);
+        else dual ? gemm_rows_f32_go<16, 4, true>(a, s) : gemm_rows_f32_go<16, 4, false>(a, s);
+        return true;
+    }
+    const int tiles = (a.M + 63) / 64 + (a.group_offsets ? a.G : 0), cols = (a.N + 63) / 64;
+    if (cols > 65535) return false;
+    const size_t smem = (size_t)GT_STAGES * (dual ? 3 : 2) * 64 * GT_PITCH * sizeof(float);
+    static std::once_flag raised;
+    std::call_once(raised, [] {
+        tb_note_error(cudaFuncSetAttribute(gemm_tile_f32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        tb_note_error(cudaFuncSetAttribute(gemm_tile_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    });
+    if (dual) TB_LAUNCH((gemm_tile_f32_kernel<true>), dim3(tiles, cols), 256, smem, s, a);
+    else TB_LAUNCH((gemm_tile_f32_kernel<false>), dim3(tiles, cols), 256, smem, s, a);
+    return true;
 }
 
 template <typename T, typename TC, bool DUAL>
 static int gemm_simt_launch(const GemmArgs& a, cudaStream_t s, int batches = 1) {
     if (a.M < 0 || a.N <= 0 || a.K <= 0 || a.G <= 0 || batches <= 0 || batches > 65535) return TB_ERR_ARG;
     if (a.M == 0) return 0;
+    if constexpr (std::is_same<T, float>::value) {
+        if (batches == 1 && gemm_f32_launch(a, DUAL, s)) return tb_last_error();
+    }
     const bool small = a.M <= 16 * a.G;
     const int bm = small ? 16 : 64;
     // every group may end in a partly filled tile
