@@ -1,0 +1,82 @@
+"""The delta rule 16 tokens at a time against the recurrence in 64 bits: sequences around a chunk's edges, one in two
+steps, heads that share a key, one decay per head, and decays from 1 down to 0.
+
+The bound: results are sums of at most (tokens + dim) float terms whose sizes the values bound (unit keys, beta <= 1,
+decays <= 1), so 1e-5 of the largest value, as for the token-by-token kernel; bfloat16 inputs are exact here."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _plain(x, conv, a, beta, G, H, dim, vdim):
+    """x [n, C] inputs, a [n, H, dim] decays, beta [n, H], float64 -> (o [n, H, vdim], S [H, dim, vdim])."""
+    n, C = x.shape
+    xp = torch.cat([torch.zeros(3, C, dtype=x.dtype), x])
+    y = sum(conv[:, j] * xp[j:j + n] for j in range(4))
+    y = y * torch.sigmoid(y)
+    unit = lambda t: t / (t.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt()
+    q = unit(y[:, :G * dim].view(n, G, dim)).repeat_interleave(H // G, 1) * dim ** -0.5
+    k = unit(y[:, G * dim:2 * G * dim].view(n, G, dim)).repeat_interleave(H // G, 1)
+    v = y[:, 2 * G * dim:].view(n, H, vdim)
+    S = torch.zeros(H, dim, vdim, dtype=x.dtype)
+    out = []
+    for t in range(n):
+        S = a[t][:, :, None] * S
+        u = beta[t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], S))
+        S = S + k[t][:, :, None] * u[:, None]
+        out.append(torch.einsum("hd,hdv->hv", q[t], S))
+    return torch.stack(out), S
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("G,H,dim,vdim,per_head,steep", [(2, 4, 64, 48, False, 0.0), (1, 1, 128, 128, True, 0.0),
+                                                         (2, 2, 128, 16, False, 6.0), (1, 2, 64, 256, False, -12.0)])
+def test_chunks(dtype, G, H, dim, vdim, per_head, steep):
+    from transformer_b200.csrc import lib
+    gen = torch.Generator().manual_seed(dim + vdim)
+    lens, later = [1, 16, 17, 50, 3, 32], [40, 1, 15, 33, 16, 2]        # two steps of the same sequences
+    B, C, sfx = len(lens), 2 * G * dim + H * vdim, "f32" if dtype == torch.float32 else "bf16"
+    size, n_a = lib.delta_state_size(G, H, dim, vdim, 4), H if per_head else H * dim
+    state = torch.randn(B + 1, size, generator=gen)
+    slots = torch.tensor([3, 1, 0, 5, 2, 6], dtype=torch.int32)
+    state[slots.long()] = 0.0
+    untouched = state[4].clone()
+    state, slots = state.cuda(), slots.cuda()
+    x = [torch.randn(m + n, C, generator=gen).to(dtype) for m, n in zip(lens, later)]
+    pre = [torch.randn(m + n, n_a, generator=gen) * 3 + steep for m, n in zip(lens, later)]
+    bz = [torch.randn(m + n, H, generator=gen) * 2 for m, n in zip(lens, later)]
+    for i in (1, 3):                                    # a sequence whose tokens are all alike: keys repeat
+        x[i][:] = x[i][0]
+    conv, A_log = torch.randn(C, 4, generator=gen) * 0.6, torch.rand(H, generator=gen) * 3 - 2.5
+    bias = torch.randn(n_a, generator=gen) - 1
+    d_conv, d_A, d_bias = conv.cuda(), A_log.cuda(), bias.cuda()
+    per = lib.delta_chunk_record_size(dim, vdim, 4)
+    got = [[] for _ in lens]
+    for first, ns in ((0, lens), (1, later)):
+        pick = lambda rows: torch.cat([r[m:] if first else r[:m] for r, m in zip(rows, lens)])
+        z = torch.zeros(sum(ns), C + 6, dtype=dtype)
+        z[:, :C] = pick(x)
+        z, a, b = z.cuda(), pick(pre).cuda(), pick(bz).cuda()
+        starts = torch.tensor([0] + ns).cumsum(0).to(torch.int32).cuda()
+        chunks = sum(ns) // 16 + B
+        rec = torch.full((H, chunks, per), float("nan"), device="cuda")
+        o = torch.full((sum(ns), H, vdim), float("nan"), device="cuda")
+        where = (lib.ptr(starts), lib.ptr(slots), sum(ns), B, G, H, dim, vdim, 4, chunks)
+        lib.call("tb_delta_chunk_" + sfx, lib.ptr(z), C + 6, lib.ptr(d_conv), lib.ptr(state), lib.ptr(a), lib.ptr(d_bias),
+                 lib.ptr(d_A), lib.ptr(b), lib.ptr(rec), *where, n_a, H, int(per_head))
+        lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where)
+        torch.cuda.synchronize()
+        for i, part in enumerate(o.cpu().split(ns)):
+            got[i].append(part)
+    assert not lib.library().tb_gemm_tc_status()
+    assert torch.equal(state[4].cpu(), untouched)
+    for i in range(B):
+        rate = torch.exp(A_log.double())[None, :, None]
+        decay = torch.exp(-rate * torch.nn.functional.softplus(pre[i].double() + bias.double()).view(len(x[i]), H, -1))
+        want, S = _plain(x[i].double(), conv.double(), decay.expand(-1, -1, dim), torch.sigmoid(bz[i].double()), G, H, dim, vdim)
+        scale = float(want.abs().max()) + 1.0
+        assert float((torch.cat(got[i]).double() - want).abs().max()) <= 1e-5 * scale
+        row = state[int(slots[i])].cpu().double()
+        assert float((row[:H * dim * vdim].view(H, dim, vdim) - S).abs().max()) <= 1e-5 * (float(S.abs().max()) + 1.0)
+        assert torch.equal(row[H * dim * vdim:].view(3, C), x[i][-3:].double())

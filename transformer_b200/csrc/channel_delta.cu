@@ -19,12 +19,10 @@
 // four to sixteen adjacent lanes, which split the rows (chunks of four rows, interleaved), RPT rows each in
 // registers.  The first kernel leaves one contiguous record per (token, head), so the scan's staging is a plain
 // 16-byte copy.
-#include "common.cuh"
+#include "channel_delta.cuh"
 #include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
 
-#define CD_UNIT_EPS 1e-6f
 #define CD_THREADS 128
-#define CD_MAX_TAPS 16
 #define CD_TOK 4            // tokens staged in shared memory per barrier
 
 // Rows that the scan's lanes cover for heads of `dim` key channels (dim rounded up to what its forms take), and the
@@ -33,27 +31,6 @@
 __host__ __device__ inline int cd_rows(int dim) { return dim <= 16 ? 16 : dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
 __host__ __device__ inline int cd_record(int dim) { return 3 * cd_rows(dim) + 4; }
 __host__ __device__ inline int cd_vpitch(int vdim) { return (vdim + 31) / 32 * 32; }
-
-struct DeltaPrepArgs {
-    const void* z;          // [nt, ldz]: q (G dim) | k (G dim) | v (H vdim) | whatever else the product made
-    const float* wconv;     // [C, taps], the last column is the current token's
-    float* state;           // [slots, state_stride]
-    const float* a;         // [nt, H dim]  pre-activation of the decay
-    const float* dt_bias;   // [H dim]
-    const float* A_log;     // [H]
-    const float* bz;        // [nt, H]      pre-activation of beta
-    float* rec;             // out [nt, H, cd_record(dim)]
-    float* vbuf;            // out [nt, H, cd_vpitch(vdim)]
-    const int* tok_seq;
-    const int* seq_start;
-    const int* slots;
-    long long state_stride, conv_offset;
-    int ldz, G, H, dim, vdim, taps, update_state;
-    int lda, ldb;           // row pitches of a and bz (floats)
-    int head_decay;         // 1: one decay per head: a [nt, H], dt_bias [H], the same g for every key channel
-};
-
-__device__ __forceinline__ float cd_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
 // A block = up to four consecutive tokens of the step x one key head g: the convolutions of that head's query and
 // key channels and of the value channels of the heads that read it (a thread keeps a channel's taps for the block's
@@ -157,26 +134,6 @@ __global__ void __launch_bounds__(32 * CD_PT) delta_prep_kernel(const DeltaPrepA
             for (int c = lane; c < VP; c += 32) vb[c] = c < vdim ? y[2 * dim + h * vdim + c] : 0.f;
         }
     }
-}
-
-// After a step that brought a sequence more than one token: the last taps - 1 inputs of every channel, from the
-// step's rows and, where the step was shorter than that, from what the state held.
-template <typename T>
-__global__ void __launch_bounds__(256) delta_conv_state_kernel(const DeltaPrepArgs p) {
-    pdl_sync();
-    const int b = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
-    const int C = 2 * p.G * p.dim + p.H * p.vdim, keep = p.taps - 1;
-    if (c >= C) return;
-    const int t0 = p.seq_start[b], n = p.seq_start[b + 1] - t0;
-    if (n <= 0) return;
-    const T* z = static_cast<const T*>(p.z);
-    float* cs = p.state + (size_t)p.slots[b] * p.state_stride + p.conv_offset;
-    float fresh[CD_MAX_TAPS];
-    for (int r = 0; r < keep; ++r) {
-        const int li = n - keep + r;
-        fresh[r] = li >= 0 ? ldf(z + (size_t)(t0 + li) * p.ldz + c) : cs[(size_t)(keep + li) * C + c];
-    }
-    for (int r = 0; r < keep; ++r) cs[(size_t)r * C + c] = fresh[r];
 }
 
 struct DeltaScanArgs {

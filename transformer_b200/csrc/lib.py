@@ -72,6 +72,8 @@ _SIGNATURES: Dict[str, str] = {
     "tb_delta_prep_f32": "pipppppppppppiiiiiiiiiii",
     "tb_delta_prep_bf16": "pipppppppppppiiiiiiiiiii",
     "tb_delta_scan": "ppppppiiiiiii",
+    "tb_delta_chunk_f32": "pipppppppppiiiiiiiiiii", "tb_delta_chunk_bf16": "pipppppppppiiiiiiiiiii",
+    "tb_delta_chunk_scan": "pppppiiiiiiii",
     "tb_bias_glu_f32": "pppiii", "tb_bias_glu_bf16": "pppiii",
     "tb_router_sigmoid_f32": "ppppppppiiii", "tb_router_sigmoid_bf16": "ppppppppiiii",
     "tb_router_rows_sigmoid_bf16": "ppppppppiiii",
@@ -127,7 +129,7 @@ class TapeMap(ctypes.Structure):
 
 _NO_STREAM = {"tb_decay_scan_rect_record_size": "ii", "tb_split_delta_record_size": "i",
               "tb_decay_state_size": "iii", "tb_decay_record_size": "i",
-              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_latent_attention_tile_tokens": "i", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
+              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_latent_attention_tile_tokens": "i", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
               "tb_attention_tc_tile_tokens": ""}
 
 _lock = threading.Lock()
@@ -389,7 +391,7 @@ def kernel_status_async(host_int32: torch.Tensor) -> None:
 def _gave_up(code: int) -> str:
     """Which kernel family a wait code belongs to (1..5 tensor-core products, 11..17 tensor-core prompt
     attention, 21..27 decode attention with the page ring, 31..32 the decaying memory's scan, 33..34 the split delta
-    rule's)."""
+    rule's, 35..36 the chunked delta rule's)."""
     if 1 <= code <= 5:
         return "tensor-core matrix product"
     if 11 <= code <= 17:
@@ -400,6 +402,8 @@ def _gave_up(code: int) -> str:
         return "scan of the decaying memory"
     if 33 <= code <= 34:
         return "scan of the split delta rule"
+    if 35 <= code <= 36:
+        return "chunk scan of the delta rule"
     return "unknown kernel"
 
 
@@ -434,6 +438,15 @@ def delta_record_size(dim: int) -> int:
 def delta_value_pitch(vdim: int) -> int:
     """Floats of a (token, head) row of values between the delta rule's two kernels."""
     return library().tb_delta_value_pitch(vdim)
+
+
+def delta_chunk_record_size(dim: int, vdim: int, taps: int) -> int:
+    """Floats of a (head, chunk) record of the chunked delta rule; 0: its kernels do not take such heads."""
+    return library().tb_delta_chunk_record_size(dim, vdim, taps)
+
+
+def delta_chunk_tokens() -> int:
+    return library().tb_delta_chunk_tokens()
 
 
 def decay_state_size(heads: int, dim: int, width: int) -> int:

@@ -17,7 +17,7 @@ S is zero when a sequence starts, float, and carried from step to step together 
 of the convolutions in the engine's per-sequence state (one row per slot).  Decays, their logarithms and
 exponentials, beta, the unit norms, the state and the per-head norm are float on both paths; the bfloat16 path
 differs in the type of the projections' results.  The projections of beta and of the decay write float (their
-error would add up along the sequence).  Kernels: csrc/channel_delta.cu.
+error would add up along the sequence).  Kernels: csrc/channel_delta.cu, prompts: csrc/channel_delta_chunk.cu.
 """
 from __future__ import annotations
 
@@ -81,6 +81,8 @@ class ChannelDelta(Mixer):
 
     def bind(self, tensors) -> None:
         super().bind(tensors)
+        if self.weights["conv"].data_ptr() % 16:
+            self.weights["conv"] = self.weights["conv"].clone()       # the chunk kernel reads a channel's taps in one load
         # the kernel that norms the heads' outputs takes one weight per (head, entry): the shared one, repeated
         self.weights["norm"] = self.weights["norm"].float().repeat(self.H).contiguous()
         if not self.ra:
@@ -110,17 +112,30 @@ class ChannelDelta(Mixer):
             matmul_nt(z[:, self.C + self.ra:], w["g2"], gz)
         else:
             gz = z[:, self.C + self.ra:]
-        # what enters the recurrence, float: one record per (token, head) [q | k | decay | beta, k.q], and the values
-        rec = ctx.scratch("delta.rec", (nt, H, lib.delta_record_size(self.dim)), torch.float32)
-        vals = ctx.scratch("delta.v", (nt, H, lib.delta_value_pitch(self.vdim)), torch.float32)
-        lib.call("tb_delta_prep_" + sfx, lib.ptr(z), self.z_width, lib.ptr(w["conv"]), lib.ptr(state), lib.ptr(a),
-                 lib.ptr(w["dt_bias"]), lib.ptr(w["A_log"]), lib.ptr(bz), lib.ptr(rec), lib.ptr(vals),
-                 lib.ptr(ctx.tok_seq), lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), nt, ctx.B, self.G, H,
-                 self.dim, self.vdim, self.taps, 1 if ctx.decode else 0, a.stride(0), bz.stride(0),
-                 1 if self.decay == "head" else 0)
         o = ctx.scratch("delta.o", (nt, self.hv), torch.float32)
-        lib.call("tb_delta_scan", lib.ptr(rec), lib.ptr(vals), lib.ptr(state), lib.ptr(o),
-                 lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), nt, ctx.B, self.G, H, self.dim, self.vdim, self.taps)
+        where = (lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), nt, ctx.B, self.G, H, self.dim, self.vdim, self.taps)
+        per_head = 1 if self.decay == "head" else 0
+        # long prompts: 16 tokens at a time (csrc/channel_delta_chunk.cu).  It is the faster form from some 20 tokens a
+        # sequence on (16 heads of 128, both kernels: 16 x 8 tokens 65 us here and 63 token by token, 1 x 64 32 and 46,
+        # 8 x 70 91 and 145), but its sums round differently, so it begins where the gain is worth that: at 320 tokens
+        # the two differ by a tenth of a millisecond a layer, at 2,048 by half a millisecond
+        per_chunk = lib.delta_chunk_record_size(self.dim, self.vdim, self.taps)
+        if per_chunk and nt > 320 * ctx.B and self.z_width % 2 == 0:
+            chunks = nt // lib.delta_chunk_tokens() + ctx.B
+            rec = ctx.scratch("delta.rec", (H, chunks, per_chunk), torch.float32)
+            lib.call("tb_delta_chunk_" + sfx, lib.ptr(z), self.z_width, lib.ptr(w["conv"]), lib.ptr(state), lib.ptr(a),
+                     lib.ptr(w["dt_bias"]), lib.ptr(w["A_log"]), lib.ptr(bz), lib.ptr(rec), *where, chunks, a.stride(0),
+                     bz.stride(0), per_head)
+            lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where, chunks)
+        else:
+            # what enters the recurrence, float: one record per (token, head) [q | k | decay | beta, k.q], and the values
+            rec = ctx.scratch("delta.rec", (nt, H, lib.delta_record_size(self.dim)), torch.float32)
+            vals = ctx.scratch("delta.v", (nt, H, lib.delta_value_pitch(self.vdim)), torch.float32)
+            lib.call("tb_delta_prep_" + sfx, lib.ptr(z), self.z_width, lib.ptr(w["conv"]), lib.ptr(state), lib.ptr(a),
+                     lib.ptr(w["dt_bias"]), lib.ptr(w["A_log"]), lib.ptr(bz), lib.ptr(rec), lib.ptr(vals),
+                     lib.ptr(ctx.tok_seq), lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), nt, ctx.B, self.G, H,
+                     self.dim, self.vdim, self.taps, 1 if ctx.decode else 0, a.stride(0), bz.stride(0), per_head)
+            lib.call("tb_delta_scan", lib.ptr(rec), lib.ptr(vals), lib.ptr(state), lib.ptr(o), *where)
         y = ctx.scratch("delta.y", (nt, self.hv), self.dtype)
         lib.call("tb_mlstm_out_" + sfx, lib.ptr(o), lib.ptr(gz), gz.stride(0), lib.ptr(w["norm"]), lib.ptr(y), nt, H,
                  self.vdim, self.eps, 1 if self.gate_act == "silu" else 0, self.hv)
