@@ -77,6 +77,40 @@ __device__ __forceinline__ void lm_cp16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
 }
 
+// The 16 rows' queries to shared memory: the latent's side as it is (16 bytes at a time), the rotated part rotated here,
+// both unscaled.
+__device__ __forceinline__ void lm_load_queries(const LatentMmaArgs& a, __nv_bfloat16* q_s, int pitch, int t0, int n_tok, int h0) {
+    const int hc = a.heads_per_block;
+    const int chunks_q = a.rank / 8;
+    for (int idx = threadIdx.x; idx < LM_ROWS * chunks_q; idx += blockDim.x) {
+        const int row = idx / chunks_q, c = (idx - row * chunks_q) * 8;
+        const int ti = row / hc, h = h0 + row % hc;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (ti < n_tok && h < a.H)
+            v = *reinterpret_cast<const uint4*>(a.qa + ((size_t)(t0 + ti) * a.H + h) * a.rank + c);
+        *reinterpret_cast<uint4*>(q_s + row * pitch + c) = v;
+    }
+    for (int idx = threadIdx.x; idx < LM_ROWS * a.rot; idx += blockDim.x) {
+        const int row = idx / a.rot, r = idx - row * a.rot;
+        const int ti = row / hc, h = h0 + row % hc;
+        float v = 0.f;
+        if (ti < n_tok && h < a.H) {
+            const int t = t0 + ti;
+            const __nv_bfloat16* qr = a.q + (size_t)t * a.ldq + (size_t)h * a.q_head + a.q_plain;
+            const int half = a.rdims / 2, pos = a.tok_pos[t];
+            v = __bfloat162float(qr[r]);
+            if (r < half) {
+                const float co = a.cosT[(size_t)pos * half + r], si = a.sinT[(size_t)pos * half + r];
+                v = v * co - __bfloat162float(qr[r + half]) * si;
+            } else if (r < a.rdims) {
+                const float co = a.cosT[(size_t)pos * half + r - half], si = a.sinT[(size_t)pos * half + r - half];
+                v = v * co + __bfloat162float(qr[r - half]) * si;
+            }
+        }
+        q_s[row * pitch + a.rank + r] = __float2bfloat16_rn(v);
+    }
+}
+
 // NT = n8 tiles of the output per warp (rank / 4 / 8, rounded up to the instantiated sizes)
 template <int NT, int LM_WARPS>
 __global__ void __launch_bounds__(LM_WARPS * 32) latent_mma_kernel(const LatentMmaArgs a) {
@@ -98,37 +132,7 @@ __global__ void __launch_bounds__(LM_WARPS * 32) latent_mma_kernel(const LatentM
     const int seq = a.tile_seq[tile], t0 = a.tile_t0[tile];
     const int hc = a.heads_per_block;
     const int n_tok = min(a.tile_nq[tile], a.tokens_per_block);
-    // ---- queries: the latent's side as it is (16 bytes at a time), the rotated part rotated here, both unscaled ----
-    {
-        const int chunks_q = a.rank / 8;
-        for (int idx = threadIdx.x; idx < LM_ROWS * chunks_q; idx += blockDim.x) {
-            const int row = idx / chunks_q, c = (idx - row * chunks_q) * 8;
-            const int ti = row / hc, h = h0 + row % hc;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (ti < n_tok && h < a.H)
-                v = *reinterpret_cast<const uint4*>(a.qa + ((size_t)(t0 + ti) * a.H + h) * a.rank + c);
-            *reinterpret_cast<uint4*>(q_s + row * pitch + c) = v;
-        }
-        for (int idx = threadIdx.x; idx < LM_ROWS * a.rot; idx += blockDim.x) {
-            const int row = idx / a.rot, r = idx - row * a.rot;
-            const int ti = row / hc, h = h0 + row % hc;
-            float v = 0.f;
-            if (ti < n_tok && h < a.H) {
-                const int t = t0 + ti;
-                const __nv_bfloat16* qr = a.q + (size_t)t * a.ldq + (size_t)h * a.q_head + a.q_plain;
-                const int half = a.rdims / 2, pos = a.tok_pos[t];
-                v = __bfloat162float(qr[r]);
-                if (r < half) {
-                    const float co = a.cosT[(size_t)pos * half + r], si = a.sinT[(size_t)pos * half + r];
-                    v = v * co - __bfloat162float(qr[r + half]) * si;
-                } else if (r < a.rdims) {
-                    const float co = a.cosT[(size_t)pos * half + r - half], si = a.sinT[(size_t)pos * half + r - half];
-                    v = v * co + __bfloat162float(qr[r - half]) * si;
-                }
-            }
-            q_s[row * pitch + a.rank + r] = __float2bfloat16_rn(v);
-        }
-    }
+    lm_load_queries(a, q_s, pitch, t0, n_tok, h0);
     if (threadIdx.x < LM_ROWS) {
         const int ti = threadIdx.x / hc, h = h0 + threadIdx.x % hc;
         pos_s[threadIdx.x] = (ti < n_tok && h < a.H) ? a.tok_pos[t0 + ti] : -1;
@@ -327,6 +331,265 @@ __global__ void __launch_bounds__(LM_WARPS * 32) latent_mma_kernel(const LatentM
     }
 }
 
+// ---- many tokens (prompts): 64 rows a block ------------------------------------------------------------------------
+// The kernel above reads a page (74 KB for a rank of 512 and 64 rotated entries) for 16 rows, waits for it, and feeds every
+// mma from two ldmatrix: 2,039 tokens of 16 heads took 720 us.  Here (439 us; the tensor pipe a quarter busy, bound by latencies with
+// eight warps an SM) four
+// neighbouring tiles share a page and the fragments: a warp's tile of the scores is 32 rows x 32 keys of the even or of
+// the odd k-steps (the two chains of sums of the kernel above, so every bit of the result is the same), 8 mma for 4
+// ldmatrix, and its tile of the values 64 rows x rank / 8 columns, 32 mma for 8.  Pages come as halves of 32 keys through
+// a ring of three: the first half of the next page while this one is multiplied, its second half as soon as this
+// page's first has been used.  One block an SM (230 KB), the latest tiles (the most keys) first.
+// Tiles of several sequences in one block are done one sequence after the other.
+#define LR_TILES 4
+#define LR_ROWS (LR_TILES * LM_ROWS)
+#define LR_HALF (LM_KEYS / 2)
+template <int NT>       // rank = 64 NT
+__global__ void __launch_bounds__(256, 1) latent_rows_kernel(const LatentMmaArgs a, int tiles) {
+    pdl_sync();
+    extern __shared__ __align__(16) unsigned char lm_smem[];
+    const int DK = a.rank + a.rot, pitch = DK + 8;
+    __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(lm_smem);                     // [64][pitch]
+    __nv_bfloat16* k_s = q_s + LR_ROWS * pitch;                                          // [3][32][pitch]
+    float* s_s = reinterpret_cast<float*>(k_s + 3 * LR_HALF * pitch);                    // [2][64][64 + 1]: even, odd k-steps
+    __nv_bfloat16* p_s = reinterpret_cast<__nv_bfloat16*>(s_s + 2 * LR_ROWS * (LM_KEYS + 1));   // [64][64 + 8]
+    float* corr_s = reinterpret_cast<float*>(p_s + LR_ROWS * (LM_KEYS + 8));             // [64]
+    int* pos_s = reinterpret_cast<int*>(corr_s + LR_ROWS);                               // [64] positions, -1: no row
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+    const int first = ((int)gridDim.x - 1 - (int)blockIdx.x) * LR_TILES, count = min(LR_TILES, tiles - first);
+    const int hc = a.heads_per_block, h0 = blockIdx.y * hc;
+    for (int i = 0; i < LR_TILES; ++i) {
+        const bool there = i < count;       // rows of tiles that are not there: zeros
+        const int t0 = there ? a.tile_t0[first + i] : 0, n = there ? min(a.tile_nq[first + i], a.tokens_per_block) : 0;
+        lm_load_queries(a, q_s + i * LM_ROWS * pitch, pitch, t0, n, h0);
+        if (threadIdx.x < LM_ROWS) {
+            const int ti = threadIdx.x / hc, h = h0 + threadIdx.x % hc;
+            pos_s[i * LM_ROWS + threadIdx.x] = (ti < n && h < a.H) ? a.tok_pos[t0 + ti] : -1;
+        }
+    }
+    float acc[LR_TILES][NT][4];
+#pragma unroll
+    for (int m = 0; m < LR_TILES; ++m)
+#pragma unroll
+        for (int i = 0; i < NT; ++i) acc[m][i][0] = acc[m][i][1] = acc[m][i][2] = acc[m][i][3] = 0.f;
+    float mx[8], sum[8];            // of rows 8 warp .. (the same in every lane)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        mx[r] = -INFINITY;
+        sum[r] = 0.f;
+    }
+    const int chunks = DK / 8;
+    const int wr = warp & 1, wk = (warp >> 1) & 1, odd = warp >> 2;     // rows, keys (a half) and k-steps of the scores
+    __syncthreads();
+    for (int s0 = 0; s0 < count;) {
+        const int seq = a.tile_seq[first + s0];
+        int s1 = s0 + 1;
+        while (s1 < count && a.tile_seq[first + s1] == seq) ++s1;
+        // pages of each tile (the others' are none), and of the tiles together
+        int pg_lo[LR_TILES], pg_hi[LR_TILES], pg0 = 0, pg1 = -1;
+#pragma unroll
+        for (int i = 0; i < LR_TILES; ++i) {
+            pg_lo[i] = 0;
+            pg_hi[i] = -1;
+            if (i >= s0 && i < s1) {
+                const int t0 = a.tile_t0[first + i], n = min(a.tile_nq[first + i], a.tokens_per_block);
+                pg_lo[i] = max(a.tok_pos[t0] - a.window + 1, 0) / LM_KEYS;
+                pg_hi[i] = a.tok_pos[t0 + n - 1] / LM_KEYS;
+                if (i == s0) pg0 = pg_lo[i];
+                pg1 = pg_hi[i];
+            }
+        }
+        const int* table = a.page_table + (size_t)seq * a.max_pages;
+        const int halves = 2 * (pg1 - pg0 + 1);
+        auto issue = [&](int half) {
+            if (half < halves) {
+                const __nv_bfloat16* src = a.cache + ((size_t)table[pg0 + (half >> 1)] * TB_PAGE + (half & 1) * LR_HALF) * DK;
+                __nv_bfloat16* dst = k_s + (half % 3) * LR_HALF * pitch;
+                const int kk = threadIdx.x >> 3;                // eight neighbouring threads a row
+                for (int c8 = threadIdx.x & 7; c8 < chunks; c8 += 8)
+                    lm_cp16(dst + kk * pitch + c8 * 8, src + (size_t)kk * DK + c8 * 8);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        issue(0);
+        issue(1);
+        for (int pg = pg0; pg <= pg1; ++pg) {
+            const int half = 2 * (pg - pg0);
+            issue(half + 2);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            // ---- 1. scores
+            {
+                float sc[2][4][4];
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) sc[m][n][0] = sc[m][n][1] = sc[m][n][2] = sc[m][n][3] = 0.f;
+                const __nv_bfloat16* qa_p = q_s + (wr * 32 + (lane & 15)) * pitch + (lane >> 4) * 8;
+                const __nv_bfloat16* kb_p = k_s + ((half + wk) % 3 * LR_HALF + (lane & 7) + ((lane >> 4) << 3)) * pitch +
+                                            ((lane >> 3) & 1) * 8;
+#pragma unroll 2
+                for (int k0 = odd * 16; k0 < DK; k0 += 32) {
+                    unsigned af[2][4], bf[2][4];
+                    lm_ldmatrix_x4(af[0], qa_p + k0);
+                    lm_ldmatrix_x4(af[1], qa_p + 16 * pitch + k0);
+                    lm_ldmatrix_x4(bf[0], kb_p + k0);
+                    lm_ldmatrix_x4(bf[1], kb_p + 16 * pitch + k0);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m)
+#pragma unroll
+                        for (int n = 0; n < 4; ++n) lm_mma(sc[m][n], af[m], bf[n >> 1][(n & 1) * 2], bf[n >> 1][(n & 1) * 2 + 1]);
+                }
+                float* to = s_s + odd * LR_ROWS * (LM_KEYS + 1) + (wr * 32 + g) * (LM_KEYS + 1) + wk * 32 + 2 * t4;
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            to[(m * 16 + (e >> 1) * 8) * (LM_KEYS + 1) + n * 8 + (e & 1)] = sc[m][n][e];
+            }
+            __syncthreads();
+            // ---- 2. softmax of this warp's rows, if their tile sees the page
+            int lo = pg_lo[0], hi = pg_hi[0];
+#pragma unroll
+            for (int i = 1; i < LR_TILES; ++i)
+                if (warp / 2 == i) {
+                    lo = pg_lo[i];
+                    hi = pg_hi[i];
+                }
+            if (pg >= lo && pg <= hi) {
+                // the eight rows step by step side by side: their shuffles' latencies overlap
+                float v0[8], v1[8], red[8];
+                unsigned see0 = 0, see1 = 0;
+                const int j0 = pg * LM_KEYS + lane, j1 = j0 + 32;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int row = warp * 8 + r, pos = pos_s[row];
+                    const bool s0r = pos >= 0 && j0 <= pos && pos - j0 < a.window;
+                    const bool s1r = pos >= 0 && j1 <= pos && pos - j1 < a.window;
+                    see0 |= s0r ? 1u << r : 0u;
+                    see1 |= s1r ? 1u << r : 0u;
+                    const float* sr = s_s + row * (LM_KEYS + 1) + lane;
+                    const float* so = sr + LR_ROWS * (LM_KEYS + 1);
+                    v0[r] = s0r ? __fmul_rn(sr[0] + so[0], a.scale) : -INFINITY;
+                    v1[r] = s1r ? __fmul_rn(sr[32] + so[32], a.scale) : -INFINITY;
+                    red[r] = fmaxf(v0[r], v1[r]);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) red[r] = fmaxf(red[r], __shfl_xor_sync(0xffffffffu, red[r], o));
+                float corr[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const float m_new = fmaxf(mx[r], red[r]);
+                    float p0 = 0.f, p1 = 0.f;
+                    corr[r] = 1.f;
+                    if (m_new > -INFINITY) {
+                        p0 = see0 >> r & 1 ? __expf(v0[r] - m_new) : 0.f;
+                        p1 = see1 >> r & 1 ? __expf(v1[r] - m_new) : 0.f;
+                        corr[r] = __expf(mx[r] - m_new);
+                    }
+                    mx[r] = m_new;
+                    const int row = warp * 8 + r;
+                    p_s[row * (LM_KEYS + 8) + lane] = __float2bfloat16_rn(p0);
+                    p_s[row * (LM_KEYS + 8) + lane + 32] = __float2bfloat16_rn(p1);
+                    if (lane == 0) corr_s[row] = corr[r];
+                    red[r] = p0 + p1;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) red[r] += __shfl_xor_sync(0xffffffffu, red[r], o);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) sum[r] = sum[r] * corr[r] + red[r];
+            }
+            __syncthreads();
+            // ---- 3. this warp's columns of the output; tiles that do not see the page are left alone
+            const __nv_bfloat16* pa_p = p_s + (lane & 15) * (LM_KEYS + 8) + (lane >> 4) * 8;
+            const int vb = ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + warp * (NT * 8) + (lane >> 4) * 8;
+#pragma unroll
+            for (int m = 0; m < LR_TILES; ++m) {
+                if (pg < pg_lo[m] || pg > pg_hi[m]) continue;
+                const float c_lo = corr_s[m * LM_ROWS + g], c_hi = corr_s[m * LM_ROWS + g + 8];
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    acc[m][i][0] *= c_lo;
+                    acc[m][i][1] *= c_lo;
+                    acc[m][i][2] *= c_hi;
+                    acc[m][i][3] *= c_hi;
+                }
+            }
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const __nv_bfloat16* v_p = k_s + (half + hf) % 3 * LR_HALF * pitch + vb;
+#pragma unroll
+                for (int k0 = 0; k0 < LR_HALF; k0 += 16) {
+                    unsigned af[LR_TILES][4];
+#pragma unroll
+                    for (int m = 0; m < LR_TILES; ++m) lm_ldmatrix_x4(af[m], pa_p + m * LM_ROWS * (LM_KEYS + 8) + hf * LR_HALF + k0);
+#pragma unroll
+                    for (int i = 0; i < NT; i += 2) {
+                        unsigned bf[4];
+                        lm_ldmatrix_x4_trans(bf, v_p + k0 * pitch + i * 8);
+#pragma unroll
+                        for (int m = 0; m < LR_TILES; ++m) {
+                            if (pg < pg_lo[m] || pg > pg_hi[m]) continue;
+                            lm_mma(acc[m][i], af[m], bf[0], bf[1]);
+                            lm_mma(acc[m][i + 1], af[m], bf[2], bf[3]);
+                        }
+                    }
+                }
+                __syncthreads();            // this half's rows (and behind the second, the weights) are free again
+                if (hf == 0) issue(half + 3);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        s0 = s1;
+    }
+    // ---- the end: sums to shared memory, then every warp stores its columns
+    float* max_s = s_s;
+    float* sum_s = s_s + LR_ROWS;
+    if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            max_s[warp * 8 + r] = mx[r];
+            sum_s[warp * 8 + r] = sum[r];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < LR_TILES; ++m)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int in_tile = g + 8 * hh, row = m * LM_ROWS + in_tile;
+            if (pos_s[row] < 0) continue;
+            const int t = a.tile_t0[first + m] + in_tile / hc, h = h0 + in_tile % hc;
+            const float inv = lm_finish(max_s[row], sum_s[row], a.sinks, a.gate, a.ldg, t, h);
+            __nv_bfloat16* o = a.out + ((size_t)t * a.H + h) * a.rank + warp * (NT * 8);
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+                *reinterpret_cast<__nv_bfloat162*>(o + i * 8 + 2 * t4) =
+                    __floats2bfloat162_rn(acc[m][i][2 * hh] * inv, acc[m][i][2 * hh + 1] * inv);
+        }
+}
+
+static size_t latent_rows_smem(int DK) {
+    return (size_t)(LR_ROWS + 3 * LR_HALF) * (DK + 8) * 2 + 2 * LR_ROWS * (LM_KEYS + 1) * 4 + LR_ROWS * (LM_KEYS + 8) * 2 + LR_ROWS * 8;
+}
+
+template <int NT>
+static int latent_rows_go(const LatentMmaArgs& a, int tiles, cudaStream_t s) {
+    static std::once_flag raised;
+    std::call_once(raised, [] {
+        tb_note_error(cudaFuncSetAttribute(latent_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    });
+    dim3 grid((tiles + LR_TILES - 1) / LR_TILES, (a.H + a.heads_per_block - 1) / a.heads_per_block);
+    TB_LAUNCH((latent_rows_kernel<NT>), grid, 256, latent_rows_smem(a.rank + a.rot), s, a, tiles);
+    return tb_last_error();
+}
+
 // out[t, h] = sum_s e^{m_s - m} O_s / sum_s e^{m_s - m} l_s        one block per (token, head): the slices' factors
 // once, then every thread its columns with the loads of all slices in flight together
 #define LM_MAX_SPLITS 16
@@ -398,6 +661,14 @@ int tb_latent_attention_mma_bf16(const void* qa, const void* q, void* out, float
                         2 * LM_ROWS * 4 + LM_ROWS * 4;
     if (smem > 120 * 1024) return TB_ERR_UNSUPPORTED;
     int rc;
+    // The rows kernel (its shared memory must fit an SM) for prompts of so many 16-row tiles that its quarter as many blocks
+    // still pay (us, here and with 16 rows a block).  Rank 512 + 64, 16 heads: 300 tiles 52 and 44, 450 66 and 71, 600 85 and
+    // 101, 1,100 148 and 252, 2,039 439 and 720; rank 256 + 32, 8 heads: 450 78 and 63, 600 101 and 93, 800 129 and 139,
+    // 1,020 161 and 205
+    const int all_tiles = tiles * ((H + hc - 1) / hc);
+    if (splits == 1 && all_tiles >= (rank == 512 ? 400 : 700) && (rank == 128 || rank == 256 || rank == 512) && latent_rows_smem(DK) <= 227 * 1024)
+        return rank == 512 ? latent_rows_go<8>(a, tiles, s) : rank == 256 ? latent_rows_go<4>(a, tiles, s)
+                                                                          : latent_rows_go<2>(a, tiles, s);
     if (rank % 64 == 0) {               // eight warps: rank / 8 columns of the output each
         const int nt8 = rank / 8 / 8;
         if (nt8 <= 2) rc = latent_mma_go<2, 8>(a, tiles, smem, s);
