@@ -18,25 +18,9 @@
 // per block of columns, so that no block reads what another has already moved on.
 //
 // State of one (slot, head):  S [dim][vdim], then for each block of 32 columns: n [dim], m.
-#include "common.cuh"
+#include "mlstm.cuh"
 
 #define ML_WARPS 8
-#define ML_COLS 32
-#define ML_DENOM_FLOOR 1e-6f
-
-struct MlstmArgs {
-    const void* qkv;        // [nt, ld]: q heads | k heads | v heads (| anything else)
-    const float* gates;     // [nt, 2 H]: zi of every head, then zf
-    const float* bias;      // [2 H]
-    float* state;           // [slots, H, state_size]
-    float* out;             // [nt, H * vdim] unnormalized o
-    const int* seq_start;   // [B + 1]
-    const int* slots;       // [B]
-    int ld, H, dim, vdim;
-    float cap, qscale;
-};
-
-__device__ __forceinline__ float log_sigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 
 template <typename T, int RPW>
 __global__ void __launch_bounds__(ML_WARPS * 32) mlstm_scan_kernel(const MlstmArgs a) {
@@ -152,25 +136,7 @@ __global__ void __launch_bounds__(ML_WARPS * 32) mlstm_scan_kernel(const MlstmAr
 // C_tj = D_tj (k_j . q_t), then each token's numerator from the old state and from C, then the state's step.
 // Every exponent is <= 0 by the choice of m_t; all arithmetic is float (CUDA cores), on both paths.
 // One block = one sequence x one head x 32 columns of v, the state's layout is that of the kernel above.
-#define MC_L 64
 #define MC_THREADS 256
-
-__device__ __forceinline__ float warp_scan_add(float v, int lane) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-    }
-    return v;
-}
-__device__ __forceinline__ float warp_scan_max(float v, int lane) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = fmaxf(v, u);
-    }
-    return v;
-}
 
 template <typename T, bool FAST>
 __global__ void __launch_bounds__(MC_THREADS) mlstm_chunk_kernel(const MlstmArgs a) {

@@ -10,7 +10,8 @@
 S, n and m are zero when a sequence starts, are float, and are carried from step to step in the
 engine's per-sequence state (one row per slot); the gates' projections are a float product of their
 own, since their error would add up along the sequence.  The kernels are in csrc/mlstm.cu: token by
-token for decoding, 64 tokens at a time (the recurrence's closed form inside a chunk) for prompts.
+token for decoding, 64 tokens at a time (the recurrence's closed form inside a chunk) for prompts; long
+bfloat16 prompts take all chunks at once (csrc/mlstm_parallel.cu, the same bits).
 """
 from __future__ import annotations
 
@@ -22,6 +23,9 @@ from .linear import matmul_nt
 
 
 USE_CHUNKS = True      # prompts: the kernel that takes 64 tokens at a time
+# Tokens a sequence (on average) from which its chunks are done side by side: four launches against 22 us a chunk of 64 tokens
+# (8 heads of 128 x 256, us: 1 x 128 tokens 62 and 49, 1 x 192 67 and 71, 1 x 300 71 and 114, 1 x 2,039 154 and 699)
+PARALLEL_TOKENS = 192
 
 
 @MIXERS.register("mlstm")
@@ -63,11 +67,22 @@ class MatrixMemory(Mixer):
         gates = ctx.scratch("mlstm.gates", (nt, 2 * H), torch.float32)
         matmul_nt(x1, w["wif"], gates)         # float out on both paths
         o = ctx.scratch("mlstm.o", (nt, H * self.vdim), torch.float32)
-        # prompts: 64 tokens of a sequence side by side; decoding: token by token, the state in registers
-        kernel = "tb_mlstm_scan_" if ctx.decode or not USE_CHUNKS else "tb_mlstm_chunk_"
-        lib.call(kernel + sfx, lib.ptr(z), lib.ptr(gates), lib.ptr(w["bif"]), lib.ptr(state), lib.ptr(o),
-                 lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), ctx.B, self.z_width, H, self.dim, self.vdim, self.cap,
-                 self.dim ** -0.5)
+        where = (lib.ptr(ctx.seq_start), lib.ptr(ctx.slots))
+        sizes = (self.z_width, H, self.dim, self.vdim)
+        work = None
+        if self.dtype == torch.bfloat16 and USE_CHUNKS and nt >= PARALLEL_TOKENS * ctx.B and not ctx.decode:
+            per = lib.mlstm_parallel_size(H, self.dim, self.vdim, self.z_width)
+            if per:
+                chunks = nt // lib.mlstm_parallel_tokens() + ctx.B
+                work = ctx.scratch("mlstm.work", (H, chunks, per), torch.float32)
+        if work is not None:       # long prompts: the chunks of a sequence side by side
+            lib.call("tb_mlstm_parallel_" + sfx, lib.ptr(z), lib.ptr(gates), lib.ptr(w["bif"]), lib.ptr(state), lib.ptr(o),
+                     lib.ptr(work), *where, nt, ctx.B, *sizes, chunks, self.cap, self.dim ** -0.5)
+        else:
+            # short ones: 64 tokens of a sequence side by side; decoding: token by token, the state in registers
+            kernel = "tb_mlstm_scan_" if ctx.decode or not USE_CHUNKS else "tb_mlstm_chunk_"
+            lib.call(kernel + sfx, lib.ptr(z), lib.ptr(gates), lib.ptr(w["bif"]), lib.ptr(state), lib.ptr(o), *where, ctx.B,
+                     *sizes, self.cap, self.dim ** -0.5)
         y = ctx.scratch("mlstm.y", (nt, H * self.vdim), self.dtype)
         g = z[:, 2 * H * self.dim + H * self.vdim:]
         lib.call("tb_mlstm_out_" + sfx, lib.ptr(o), lib.ptr(g), self.z_width, lib.ptr(w["norm"]), lib.ptr(y), nt, H,
