@@ -37,6 +37,7 @@
 #define DM_THREADS ((DM_WARPS + 1) * 32)
 #define DM_MAX_STAGES 8
 #define DM_HEADS 16                    // query heads of one key/value head per block
+#define DM_MERGED 128                  // slices whose factors (three floats a head) fit the ring; more: a merge kernel
 
 struct DecodeMmaArgs {
     const __nv_bfloat16* q;   // [nt, q_stride]
@@ -436,20 +437,49 @@ attention_decode_mma_kernel(const __grid_constant__ CUtensorMap mk, const __grid
     __syncthreads();
     if (!last_slice) return;
     __threadfence();
-    for (int idx = threadIdx.x; idx < nheads * DH; idx += DM_THREADS) {
-        const int hc = idx / DH, c = idx - hc * DH, h = h0 + hc;
-        const float* p = a.partial + ((size_t)t * a.nh + h) * a.splits * (DH + 2);
+    // First every slice's maximum and sum, all loads at once, to factors in shared memory (the ring's); then every thread two
+    // channels with the loads of eight slices in flight.  (A loop over the slices per channel, each load waiting for the
+    // one before, was a large part of a step of one sequence; the sums keep their order.)
+    float* f_m = sm_o;                                      // [nheads][slices] maxima
+    float* f_l = f_m + nheads * slices;                     // sums
+    float* f_w = f_l + nheads * slices;                     // factors; -1: the slice saw nothing and is passed over
+    for (int idx = threadIdx.x; idx < nheads * slices; idx += DM_THREADS) {
+        const int hc = idx / slices, s = idx - hc * slices;
+        const float* p = a.partial + (((size_t)t * a.nh + h0 + hc) * a.splits + s) * (DH + 2) + DH;
+        const float2 ml = __ldcg(reinterpret_cast<const float2*>(p));
+        f_m[idx] = ml.x;
+        f_l[idx] = ml.y;
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nheads * slices; idx += DM_THREADS) {
+        const float* row = f_m + idx / slices * slices;
         float mx = -INFINITY;
-        for (int s = 0; s < slices; ++s) mx = fmaxf(mx, __ldcg(p + s * (DH + 2) + DH));
-        float den = 0.f, acc = 0.f;
-        for (int s = 0; s < slices; ++s) {
-            const float ms = __ldcg(p + s * (DH + 2) + DH);
-            if (ms == -INFINITY) continue;
-            const float w = expf(ms - mx);
-            den += __ldcg(p + s * (DH + 2) + DH + 1) * w;
-            acc += __ldcg(p + s * (DH + 2) + c) * w;
+        for (int s = 0; s < slices; ++s) mx = fmaxf(mx, row[s]);
+        f_w[idx] = f_m[idx] == -INFINITY ? -1.f : expf(f_m[idx] - mx);
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nheads * (DH / 2); idx += DM_THREADS) {
+        const int hc = idx / (DH / 2), c = (idx - hc * (DH / 2)) * 2, h = h0 + hc;
+        const float* p = a.partial + ((size_t)t * a.nh + h) * a.splits * (DH + 2) + c;
+        const float* w_row = f_w + hc * slices;
+        const float* l_row = f_l + hc * slices;
+        float den = 0.f, acc0 = 0.f, acc1 = 0.f;
+        for (int s0 = 0; s0 < slices; s0 += 8) {
+            float2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (s0 + u < slices) v[u] = __ldcg(reinterpret_cast<const float2*>(p + (size_t)(s0 + u) * (DH + 2)));
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (s0 + u >= slices) break;
+                const float w = w_row[s0 + u];
+                if (w < 0.f) continue;
+                den += l_row[s0 + u] * w;
+                acc0 += v[u].x * w;
+                acc1 += v[u].y * w;
+            }
         }
-        a.out[((size_t)t * a.nh + h) * DH + c] = __float2bfloat16_rn(acc / den);
+        *reinterpret_cast<__nv_bfloat162*>(a.out + ((size_t)t * a.nh + h) * DH + c) = __floats2bfloat162_rn(acc0 / den, acc1 / den);
     }
 }
 
@@ -464,6 +494,7 @@ static int decode_mma_launch(const CUtensorMap& mk, const CUtensorMap& mv, Decod
     if (stages < 2) stages = 2;
     a.stages = stages;
     // the warps' results (DM_WARPS x DM_HEADS x DH floats) meet in the ring: one stage's worth
+    static_assert((size_t)3 * DM_HEADS * DM_MERGED * sizeof(float) <= (size_t)2 * 2 * TB_PAGE * DH * 2, "ring too small");
     static_assert((size_t)DM_WARPS * DM_HEADS * DH * sizeof(float) <= (size_t)2 * 2 * TB_PAGE * DH * 2, "ring too small");
     const size_t smem = stage * stages + tail + 1024;
     static bool configured = false;
@@ -499,6 +530,7 @@ static int decode_mma(const void* q, void* out, void* kc, void* vc, const int* t
     if (rc) return rc;
     int* err = tc_error_ptr();
     if (!err) return tb_last_error();
+    if (splits > DM_MERGED || ((uintptr_t)partial & 7) || ((uintptr_t)out & 3)) done = nullptr;     // the merge kernel takes anything
     DecodeMmaArgs a{(const __nv_bfloat16*)q, (__nv_bfloat16*)out, tok_seq, tok_pos, page_table, partial, done, err,
                     max_pages, q_stride, nh, nkvh, splits, 0, scale * 1.4426950408889634f,
                     cos_t, sin_t, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, half_pairing, patch};
