@@ -13,6 +13,7 @@
 //   6. draw in ASCENDING id order: the first kept id whose running mass exceeds u * (kept mass).
 // Selection of the edges is exact (a radix select over the order-preserving bit pattern of z),
 // so no sort and no scratch memory is needed; every pass reads the row again (it sits in L2).
+// With a small top_k (1 < top_k <= 256) the row is read twice instead: see sample_few.
 #include "common.cuh"
 
 #define SAMP_THREADS 1024
@@ -125,14 +126,151 @@ __device__ Cut select_cut(const float* __restrict__ row, int V, float inv_t, flo
     return c;
 }
 
+// ---- a small top_k ---------------------------------------------------------------------------------------------
+// The top_k-th largest of the threads' maxima is a lower bound of the top_k-th largest z, so a second pass over the row
+// collects a few more than top_k candidates; these are sorted (key descending, id ascending), and the rest happens in
+// shared memory, its sums in a fixed order.  The radix selects read the row thirteen times, with most of its values in a
+// few bins of the first pass: 145 us for three rows of 32,000 with top_k 40 and top_p 0.9.  Here 17 us.
+#define SAMP_FEW 256            // largest top_k
+#define SAMP_CANDIDATES 1024    // more values than this at or above the bound (ties): the radix selects
+
+// Sorts one value per thread of the first `size` threads (a power of two; all threads call), ascending.
+template <typename K>
+__device__ __forceinline__ K sort_block(K v, int size, K* sm) {
+    const int tid = threadIdx.x;
+    for (int run = 2; run <= size; run <<= 1)
+        for (int stride = run >> 1; stride > 0; stride >>= 1) {
+            K other;
+            if (stride >= 32) {
+                __syncthreads();
+                sm[tid] = v;
+                __syncthreads();
+                other = sm[tid ^ stride];
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, v, stride);
+            }
+            const bool low = !(tid & stride), up = !(tid & run);
+            if (low == up ? other < v : other > v) v = other;
+        }
+    __syncthreads();
+    return v;
+}
+
+// Running sums of v over the first SAMP_FEW threads (all threads call; what the others get is of no use), in `red` [32].
+__device__ __forceinline__ float scan_few(float v, float* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    __syncthreads();
+    if (lane == 31) red[warp] = v;
+    __syncthreads();
+    float before = 0.f;
+    for (int w = 0; w < min(warp, SAMP_FEW / 32); ++w) before += red[w];
+    return before + v;
+}
+
+// True: out_idx and out_val are written.  best: this thread's largest logit; sm: 8 KB, red [33], sh_i [3].
+__device__ bool sample_few(const float* __restrict__ row, int V, float inv_t, float zmax, float best, float u, int top_k, float top_p,
+                           unsigned long long* sm, float* red, int* sh_i, int* __restrict__ out_idx, float* __restrict__ out_val) {
+    const int tid = threadIdx.x;
+    unsigned bound = sort_block<unsigned>(~order_key(best * inv_t), SAMP_THREADS, reinterpret_cast<unsigned*>(sm));
+    if (tid == top_k - 1) sh_i[0] = (int)~bound;
+    if (tid == 0) sh_i[1] = 0;
+    __syncthreads();
+    bound = (unsigned)sh_i[0];
+    auto look = [&](float v, int i) {
+        const unsigned key = order_key(v * inv_t);
+        if (key >= bound) {
+            const int at = atomicAdd(&sh_i[1], 1);
+            if (at < SAMP_CANDIDATES) sm[at] = (unsigned long long)~key << 32 | (unsigned)i;
+        }
+    };
+    int done = 0;
+    if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+        const float4* row4 = reinterpret_cast<const float4*>(row);
+        const int n4 = V >> 2;
+        for (int i0 = tid; i0 < n4; i0 += 4 * SAMP_THREADS) {
+            float4 q[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i0 + j * SAMP_THREADS < n4) q[j] = row4[i0 + j * SAMP_THREADS];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = (i0 + j * SAMP_THREADS) << 2;
+                if (i0 + j * SAMP_THREADS < n4) {
+                    look(q[j].x, i);
+                    look(q[j].y, i + 1);
+                    look(q[j].z, i + 2);
+                    look(q[j].w, i + 3);
+                }
+            }
+        }
+        done = n4 << 2;
+    }
+    for (int i = done + tid; i < V; i += SAMP_THREADS) look(row[i], i);
+    __syncthreads();
+    const int found = sh_i[1];
+    if (found > SAMP_CANDIDATES) return false;
+    int size = 32;
+    while (size < found) size <<= 1;
+    unsigned long long mine = tid < found ? sm[tid] : ~0ull;
+    __syncthreads();
+    mine = sort_block<unsigned long long>(mine, size, sm);
+    // thread tid has the tid-th of the kept, in descending p
+    int kept = min(top_k, found);
+    const int id = (int)(unsigned)mine;
+    const unsigned key = ~(unsigned)(mine >> 32);
+    const float z = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+    const float p = tid < kept ? expf(z - zmax) : 0.f;
+    if (top_p < 1.0f) {
+        const float cum = scan_few(p, red);
+        if (tid == kept - 1) red[32] = cum;
+        if (tid == 0) sh_i[2] = kept;
+        __syncthreads();
+        if (!(red[32] < INFINITY)) return false;        // a NaN or an infinity among them
+        if (tid < kept && cum >= top_p * red[32]) atomicMin(&sh_i[2], tid + 1);
+        __syncthreads();
+        kept = sh_i[2];
+    }
+    // in ascending id
+    int* ids = reinterpret_cast<int*>(sm);
+    float* ps = reinterpret_cast<float*>(sm) + SAMP_FEW;
+    int* by_id = reinterpret_cast<int*>(sm) + 2 * SAMP_FEW;
+    if (tid < kept) ids[tid] = id;
+    __syncthreads();
+    if (tid < kept) {
+        int rank = 0;
+        for (int i = 0; i < kept; ++i) rank += ids[i] < id;
+        ps[rank] = p;
+        by_id[rank] = id;
+    }
+    __syncthreads();
+    const float run = scan_few(tid < kept ? ps[tid] : 0.f, red);
+    if (tid == kept - 1) red[32] = run;
+    if (tid == 0) sh_i[2] = kept - 1;       // rounding left the target at or above the total: the last kept id
+    __syncthreads();
+    if (!(red[32] < INFINITY)) return false;
+    if (tid < kept && run > u * red[32]) atomicMin(&sh_i[2], tid);
+    __syncthreads();
+    if (tid == 0) {
+        const int pick = by_id[sh_i[2]];
+        *out_idx = pick;
+        *out_val = row[pick];
+    }
+    return true;
+}
+
 // logits [rows, V] float (row stride ld); u [rows] uniform numbers in [0, 1);
 // out_idx [rows], out_val [rows] (the chosen token's logit).
 __global__ void __launch_bounds__(SAMP_THREADS)
 sample_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ u, int V, float temperature,
               int top_k, float top_p, int* __restrict__ out_idx, float* __restrict__ out_val) {
     pdl_sync();
-    __shared__ float red_f[SAMP_THREADS];
-    __shared__ int red_i[SAMP_THREADS];
+    __shared__ __align__(8) float red_f[2 * SAMP_THREADS];
+    int* red_i = reinterpret_cast<int*>(red_f) + SAMP_THREADS;
     __shared__ int hist_c[256];
     __shared__ float hist_m[256];
     __shared__ int sh_i[4];
@@ -199,6 +337,11 @@ sample_kernel(const float* __restrict__ logits, long long ld, const float* __res
     }
     const float inv_t = 1.0f / temperature;
     const float zmax = vmax * inv_t;
+    if (top_k > 0 && top_k <= SAMP_FEW && top_k < V &&
+        sample_few(row, V, inv_t, zmax, best, u[blockIdx.x], top_k, top_p, reinterpret_cast<unsigned long long*>(red_f), hist_m, sh_i,
+                   out_idx + blockIdx.x, out_val + blockIdx.x))
+        return;
+    __syncthreads();
     Cut cut{0u, V - 1};   // everything
     if (top_k > 0 && top_k < V)
         cut = select_cut(row, V, inv_t, zmax, cut, false, top_k, 0.f, hist_c, hist_m, sh_i, sh_f);
