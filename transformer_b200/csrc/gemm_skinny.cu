@@ -35,6 +35,7 @@
 
 #define SK_WARPS 8
 #define SK_COLS 16
+#define SK_SMS 148
 
 struct SkinnyArgs {
     const __nv_bfloat16* X;
@@ -48,6 +49,10 @@ struct SkinnyArgs {
     const int* row_group;   // [M] group of every row, rows in any order (instead of group_offsets and x_rows), or null
     int x_div;              // with row_group: row m reads X[m / x_div] and writes Y[m]
     int w_constant;         // W is a weight: nothing the kernel before this one may have written
+    // With row_group and at most half as many rows as groups: a block column per ROW (the first of its group does the group's)
+    // instead of one per group, most of which would be launched to find no row (a step of one sequence, 4 of 16 experts:
+    // 2,106 to 2,039 us in 32 layers).
+    int by_row;
     GluRule glu;            // DUAL: how the (gate, up) pair becomes one value
 };
 
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(WK * WN * 32) gemm_skinny_kernel(const SkinnyA
     __shared__ int list[SK_WARPS * 32];     // with row_group: the rows of this block's group
     __shared__ unsigned list_mask[WK * WN];
 
-    const int g_idx = blockIdx.y;
+    int g_idx = a.by_row ? 0 : blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wk = warp % WK, wn = warp / WK;
     const int n0 = (blockIdx.x * WN + wn) * SK_COLS;
@@ -130,6 +135,19 @@ __global__ void __launch_bounds__(WK * WN * 32) gemm_skinny_kernel(const SkinnyA
     pdl_sync();
     int row_lo = 0, row_hi = a.M;
     const bool listed = a.row_group != nullptr;
+    if (a.by_row) {
+        g_idx = a.row_group[blockIdx.y];
+        if ((unsigned)g_idx >= (unsigned)a.G) return;       // a row of no group
+        for (int m = 0; m < (int)blockIdx.y; ++m)
+            if (a.row_group[m] == g_idx) return;
+        const size_t to = (size_t)g_idx * a.w_group_stride;
+        w0 += to;
+        w1 += to;
+        if (DUAL) {
+            u0 += to;
+            u1 += to;
+        }
+    }
     if (listed) {
         // a thread looks at one row per round of the block's threads (M <= SK_WARPS * 32, the size of the list);
         // rows keep their order inside the group
@@ -257,14 +275,26 @@ template <int NT, bool DUAL, typename TY>
 static int skinny_launch_shape(const SkinnyArgs& a, cudaStream_t s) {
     // long rows: all 8 warps of a block share 16 columns and split K;
     // short rows (an expert's down projection): 2 warps on K
+    //
+    // How many k-steps a thread loads before it multiplies (the order of the sums does not depend on it): where the blocks of
+    // a dense product fit the SMs at once, all of a warp's, so that a block that has waited for the kernel before it has
+    // nothing left to wait for but its activations.  A step of one sequence through a layer of width 1,024, us behind the
+    // kernel before: q-k-v and output products 5.3 to 3.1, gate/up pair 5.6 to 4.3, down product (K 2,816) 4.3 to 4.1.
+    // Where blocks queue for the SMs registers are worth more: an expert's down product (K 688, four experts) 8.4 us with
+    // 4 steps ahead, 10.0 with all 11.
+    const unsigned blocks = (unsigned)((a.N + SK_COLS - 1) / SK_COLS);
+    const bool dense = a.G == 1, few = dense && blocks <= 2 * SK_SMS;
     if (a.K >= 2048) {
         constexpr int WK = 8, WN = 1, UNR = NT >= 4 ? 2 : 4;
-        dim3 grid((a.N + SK_COLS * WN - 1) / (SK_COLS * WN), a.G);
+        dim3 grid(blocks, a.by_row ? a.M : a.G);
         // up to 8 rows and one matrix per group: registers allow twice as many loads in flight per thread
         // (measured in the decode step: -1.5 us per layer on the q-k-v product; for the gate/up pair 4 is best)
-        if constexpr (NT == 1 && !DUAL)
-            TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
-        else
+        if constexpr (NT == 1 && !DUAL) {
+            if (dense && blocks <= SK_SMS && a.K > 8 * WK * 32 && a.K <= 12 * WK * 32)
+                TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 12>), grid, WK * WN * 32, 0, s, a);
+            else
+                TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
+        } else
             TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
     } else {
         // 16 columns per block, as for long rows: few sequences touch few experts, and the smaller the pieces
@@ -272,8 +302,15 @@ static int skinny_launch_shape(const SkinnyArgs& a, cudaStream_t s) {
         // step at batch 8 took 2.4 % longer; 4 or 1 warps on K, or 8 loads ahead, are slower too).  Tried on the
         // gate/up pair as well (8 gate and 8 up rows per tile, half the bytes per block): no gain.
         constexpr int WK = 2, WN = 1, UNR = NT >= 4 ? 2 : 4;
-        dim3 grid((a.N + SK_COLS * WN - 1) / (SK_COLS * WN), a.G);
-        TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
+        dim3 grid(blocks, a.by_row ? a.M : a.G);
+        if constexpr (NT == 1 && DUAL) {
+            if (few) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
+            else TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
+        } else if constexpr (NT == 1) {
+            if (few) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 16>), grid, WK * WN * 32, 0, s, a);
+            else TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
+        } else
+            TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
     }
     return tb_last_error();
 }
@@ -304,7 +341,7 @@ static int skinny_entry(const void* X, const int* x_rows, const void* W, void* Y
     if (((uintptr_t)X | (uintptr_t)W) & 15) return TB_ERR_UNSUPPORTED;
     if (M == 0) return 0;
     SkinnyArgs a{(const __nv_bfloat16*)X, x_rows, (const __nv_bfloat16*)W, Y, group_offsets, w_group_stride,
-                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, glu};
+                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, row_group && 2 * M <= G, glu};
     int rows = (max_group_rows > 0 && max_group_rows < M) ? max_group_rows : M;
     if (G > 1) {
         // A pass takes 8, 16 or 32 rows of a group and a thread's registers are sized by the pass (with 16 rows the
