@@ -2,6 +2,7 @@
 //
 // The residual stream is float on both paths, so the residual sum is a 32-bit sum.
 #include "common.cuh"
+#include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
 #include "router_pick.cuh"
 
 // x[i, :] = table[tokens[i], :]   (models/llama/cuda/src/infer.rs:98-104 copies row by row)
@@ -81,7 +82,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const T* __restrict__ 
 // What a feed-forward may ask the norm before it to do in the same kernel (TAIL): the router of the row it has
 // just normalized, i.e. the row's k experts and their weights, by the rules of router_kernel.  The row goes to
 // shared memory as it goes to y (rounded to T), one warp per expert takes its dot product with the router's
-// matrix (whose first part it has read before the dependency wait), one warp picks.  A router kernel of its
+// matrix (which it has asked for before the dependency wait), one warp picks.  A router kernel of its
 // own would first wait for this kernel to end and then read the row back.
 template <typename T> struct RouterTail {
     const T* w;        // [E, d], or null: none
@@ -89,9 +90,53 @@ template <typename T> struct RouterTail {
     int* idx;          // [rows, k]
     float* wts;        // [rows, k]
     RouterRule rule;   // how the logits become a choice
+    int staged_at = 0; // where in shared memory the first row of the matrix of every warp goes (0: not staged)
 };
 
-template <typename T, int NORM_THREADS, bool EARLY, bool TAIL>
+// acc[0..8) += the weighted sum of row r's k rows of wy at column c: four rows' loads in flight, added in their order.
+template <typename T> struct Raw8;
+template <> struct Raw8<__nv_bfloat16> {
+    uint4 a;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { a = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void get(float (&f)[8]) const { Vec16<__nv_bfloat16>::unpack(a, f); }
+};
+template <> struct Raw8<float> {
+    float4 a, b;
+    __device__ __forceinline__ void load(const float* p) {
+        a = *reinterpret_cast<const float4*>(p);
+        b = *reinterpret_cast<const float4*>(p + 4);
+    }
+    __device__ __forceinline__ void get(float (&f)[8]) const {
+        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    }
+};
+template <typename T>
+__device__ __forceinline__ void experts_sum(const T* __restrict__ wy, const int* __restrict__ pair_row,
+                                            const float* __restrict__ topk_w, int k, int r, int d, int c, float (&acc)[8]) {
+    for (int q0 = 0; q0 < k; q0 += 4) {
+        Raw8<T> raw[4];
+        float wq[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (q0 + u < k) {
+                raw[u].load(wy + (size_t)pair_row[(size_t)r * k + q0 + u] * d + c);
+                wq[u] = topk_w[(size_t)r * k + q0 + u];
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (q0 + u < k) {
+                float t[8];
+                raw[u].get(t);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] += wq[u] * t[e];
+            }
+    }
+}
+
+// CH: pieces of 8 values a thread keeps (NORM_THREADS * 8 * CH >= d), POST: whether post_w is given.  What a width or a form does
+// not need costs registers, hence blocks on an SM, and code: 2,048 rows of 4,096 took 31 us (sums and experts' sums, mean)
+// with room for 8,192 values and the experts' rows loaded one after the other, and take 24.
+template <typename T, int NORM_THREADS, bool EARLY, bool TAIL, int CH, bool POST>
 __global__ void __launch_bounds__(NORM_THREADS)
 add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ wy,
                        const int* __restrict__ pair_row, const float* __restrict__ topk_w, int k,
@@ -99,27 +144,27 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
                        int d, const void* warm, int warm_bytes, const RouterTail<T> tail,
                        const float* __restrict__ post_w, float post_eps) {
     // post_w: the delta is normed by itself first (delta / rms(delta) * post_w, with post_eps) and then added
-    constexpr int EPL = Vec16<T>::N, UN = 8;
-    extern __shared__ __align__(16) unsigned char tail_smem[];      // TAIL: the row as T [d], then logits [E]
-    uint4 first[TAIL ? UN : 1];
+    constexpr int EPL = Vec16<T>::N;
+    // TAIL: the row as T [d], the logits [E] (and scores), and, if `staged`, a row of the router's matrix per warp [warps][d]
+    extern __shared__ __align__(16) unsigned char tail_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T* const ys = reinterpret_cast<T*>(tail_smem);
+    T* const my_w = TAIL ? reinterpret_cast<T*>(tail_smem + tail.staged_at) + (size_t)warp * d : nullptr;
     if (TAIL) {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (warp < tail.E) {
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const int c = (lane + u * 32) * EPL;
-                first[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (c < d) first[u] = *reinterpret_cast<const uint4*>(tail.w + (size_t)warp * d + c);
-            }
+        if (tail.staged_at && warp < tail.E) {
+#pragma unroll 1
+            for (int c = lane * EPL; c < d; c += 32 * EPL)
+                cp_async16((uint32_t)__cvta_generic_to_shared(my_w + c), tail.w + (size_t)warp * d + c);
+            cp_async_commit();
         }
     }
     warm_l2(warm, warm_bytes);
     // this kernel's own weights do not depend on the kernel before it either: they are in registers by the time
     // the wait is over (they are read once per layer and have left L2 since the last step)
-    float ww[EARLY ? NORM_CHUNKS : 1][8];
+    float ww[EARLY ? CH : 1][8];
     if (EARLY && w) {
 #pragma unroll
-        for (int j = 0; j < NORM_CHUNKS; ++j) {
+        for (int j = 0; j < CH; ++j) {
             const int c = (threadIdx.x + j * NORM_THREADS) * 8;
             if (c < d) load8(w + c, ww[j]);
         }
@@ -132,12 +177,12 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
     const T* dr = delta ? delta + (size_t)r * d : nullptr;
     const bool has_delta = dr != nullptr || wy != nullptr;
     const bool write_back = (rows == nullptr) && has_delta;
-    float v[NORM_CHUNKS][8];
+    float v[CH][8];
     float ss = 0.f;
-    if (post_w) {
+    if constexpr (POST) {
         float ss1 = 0.f;
 #pragma unroll
-        for (int j = 0; j < NORM_CHUNKS; ++j) {
+        for (int j = 0; j < CH; ++j) {
             const int c = (threadIdx.x + j * NORM_THREADS) * 8;
             if (c < d) {
                 if (dr) {
@@ -145,13 +190,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
                 } else {
 #pragma unroll
                     for (int e = 0; e < 8; ++e) v[j][e] = 0.f;
-                    for (int q = 0; q < k; ++q) {
-                        float t[8];
-                        load8(wy + (size_t)pair_row[(size_t)r * k + q] * d + c, t);
-                        const float wq = topk_w[(size_t)r * k + q];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[j][e] += wq * t[e];
-                    }
+                    experts_sum(wy, pair_row, topk_w, k, r, d, c, v[j]);
                 }
 #pragma unroll
                 for (int e = 0; e < 8; ++e) ss1 += v[j][e] * v[j][e];
@@ -160,7 +199,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
         ss1 = block_sum(ss1, red);
         const float rs1 = 1.0f / sqrtf(ss1 / (float)d + post_eps);
 #pragma unroll
-        for (int j = 0; j < NORM_CHUNKS; ++j) {
+        for (int j = 0; j < CH; ++j) {
             const int c = (threadIdx.x + j * NORM_THREADS) * 8;
             if (c < d) {
                 float xv[8], pw[8];
@@ -176,9 +215,9 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
         }
     }
 #pragma unroll
-    for (int j = 0; j < NORM_CHUNKS; ++j) {
+    for (int j = 0; j < CH; ++j) {
         const int c = (threadIdx.x + j * NORM_THREADS) * 8;
-        if (c < d && !post_w) {
+        if (c < d && !POST) {
             load8(xr + c, v[j]);
             if (dr) {
                 float t[8];
@@ -187,13 +226,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
                 for (int e = 0; e < 8; ++e) v[j][e] += t[e];
             } else if (wy) {
                 float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                for (int q = 0; q < k; ++q) {
-                    float t[8];
-                    load8(wy + (size_t)pair_row[(size_t)r * k + q] * d + c, t);
-                    const float wq = topk_w[(size_t)r * k + q];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[e] += wq * t[e];
-                }
+                experts_sum(wy, pair_row, topk_w, k, r, d, c, acc);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[j][e] += acc[e];
             }
@@ -206,7 +239,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
     T* yr = y + (size_t)i * d;
     if (!w) {                       // no weights: y is the sum itself, rounded to T (a part that reads the stream as it is)
 #pragma unroll
-        for (int j = 0; j < NORM_CHUNKS; ++j) {
+        for (int j = 0; j < CH; ++j) {
             const int c = (threadIdx.x + j * NORM_THREADS) * 8;
             if (c < d) store8(yr + c, v[j]);
         }
@@ -215,7 +248,7 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
     ss = block_sum(ss, red);
     const float rs = 1.0f / sqrtf(ss / (float)d + eps);
 #pragma unroll
-    for (int j = 0; j < NORM_CHUNKS; ++j) {
+    for (int j = 0; j < CH; ++j) {
         const int c = (threadIdx.x + j * NORM_THREADS) * 8;
         if (c < d) {
             float o[8];
@@ -223,37 +256,25 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
 #pragma unroll
             for (int e = 0; e < 8; ++e) o[e] = v[j][e] * rs * ww[EARLY ? j : 0][e];
             store8(yr + c, o);
-            if (TAIL) store8(reinterpret_cast<T*>(tail_smem) + c, o);
+            if (TAIL) store8(ys + c, o);
         }
     }
     if (!TAIL) return;
     __syncthreads();
-    const T* ys = reinterpret_cast<const T*>(tail_smem);
     float* lg = reinterpret_cast<float*>(tail_smem + (size_t)d * sizeof(T));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (tail.staged_at) cp_async_wait<0>();         // a lane reads what it copied itself
+    // A loop of a few instructions: the block runs once, and code that has to be fetched for it costs more than it saves (a step
+    // of one sequence, width 4,096, 16 experts: 9.0 us behind the kernel before with the row unrolled in registers, 7.7 so)
     for (int e = warp; e < tail.E; e += NORM_THREADS / 32) {
-        const T* we = tail.w + (size_t)e * d;
+        const T* we = tail.staged_at && e == warp ? my_w : tail.w + (size_t)e * d;
         float acc = 0.f;
-        for (int c0 = lane * EPL; c0 < d; c0 += 32 * EPL * UN) {
-            uint4 xv[UN], wv[UN];
-            const bool have = e == warp && c0 == lane * EPL;     // the batch read before the wait
+#pragma unroll 4
+        for (int c = lane * EPL; c < d; c += 32 * EPL) {
+            float xf[EPL], wf[EPL];
+            Vec16<T>::unpack(*reinterpret_cast<const uint4*>(ys + c), xf);
+            Vec16<T>::unpack(*reinterpret_cast<const uint4*>(we + c), wf);
 #pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                const int c = c0 + u * 32 * EPL;
-                xv[u] = wv[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (c < d) {
-                    xv[u] = *reinterpret_cast<const uint4*>(ys + c);
-                    wv[u] = have ? first[u] : *reinterpret_cast<const uint4*>(we + c);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                float xf[EPL], wf[EPL];
-                Vec16<T>::unpack(xv[u], xf);
-                Vec16<T>::unpack(wv[u], wf);
-#pragma unroll
-                for (int q = 0; q < EPL; ++q) acc += xf[q] * wf[q];
-            }
+            for (int q = 0; q < EPL; ++q) acc += xf[q] * wf[q];
         }
         acc = warp_sum(acc);
         if (lane == 0) lg[e] = acc;
@@ -426,6 +447,15 @@ static int embed_launch(const int* tokens, const void* table, float* x, int nt, 
         TB_LAUNCH((embed_kernel<T>), nt, 256, 0, s, tokens, (const T*)table, x, d, scale);
     return tb_last_error();
 }
+#define TAIL_SMEM (200 * 1024)
+#define TAIL_STAGED_ROWS 16     // more rows: the blocks find the router's matrix in L2
+// The kernel, allowed that much shared memory.
+template <auto Kernel> static auto tail_kernel() {
+    static std::once_flag raised;
+    std::call_once(raised, [] { tb_note_error(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM)); });
+    return Kernel;
+}
+
 template <typename T>
 static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const int* pair_row,
                               const float* topk_w, int k, const int* rows, const float* w, float eps,
@@ -444,18 +474,33 @@ static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const
         if (d % 8 || d > 512 * 8 * NORM_CHUNKS || n_out > 256 || smem > 40 * 1024 ||
             (reinterpret_cast<uintptr_t>(tail.w) & 15))
             return TB_ERR_UNSUPPORTED;           // the caller runs the router by itself
-        TB_LAUNCH((add_rmsnorm_vec_kernel<T, 512, true, true>), n_out, 512, smem, s, x, (const T*)delta, (const T*)wy,
-                  pair_row, topk_w, k, rows, w, eps, (T*)y, d, nullptr, 0, tail, post_w, post_eps);
+        // a row of the router's matrix per warp joins them where it fits (128 KB for bfloat16 and a width of 4,096)
+        const size_t at = (smem + 15) / 16 * 16, staged = (size_t)(tail.E < 16 ? tail.E : 16) * d * sizeof(T);
+        if (at + staged <= TAIL_SMEM && n_out <= TAIL_STAGED_ROWS) tail.staged_at = (int)at;
+        auto go = [&](auto kernel) {
+            TB_LAUNCH(kernel, n_out, 512, tail.staged_at ? at + staged : smem, s, x, (const T*)delta, (const T*)wy, pair_row, topk_w, k,
+                      rows, w, eps, (T*)y, d, nullptr, 0, tail, post_w, post_eps);
+        };
+        if (post_w) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, true>>());
+        else if (d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, 1, false>>());
+        else go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, false>>());
         return tb_last_error();
     }
+    auto go = [&](auto kernel, int threads) {
+        TB_LAUNCH(kernel, n_out, threads, 0, s, x, (const T*)delta, (const T*)wy, pair_row, topk_w, k, rows, w, eps, (T*)y, d, warm,
+                  warm_bytes, tail, post_w, post_eps);
+    };
     if (d % 8 == 0 && n_out <= 256 && d <= 512 * 8 * NORM_CHUNKS && y) {
-        TB_LAUNCH((add_rmsnorm_vec_kernel<T, 512, true, false>), n_out, 512, 0, s, x, (const T*)delta, (const T*)wy,
-                  pair_row, topk_w, k, rows, w, eps, (T*)y, d, warm, warm_bytes, tail, post_w, post_eps);
+        if (post_w) go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, true>, 512);
+        else if (d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, false, 1, false>, 512);
+        else go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, false>, 512);
         return tb_last_error();
     }
     if (d % 8 == 0 && d <= 256 * 8 * NORM_CHUNKS) {
-        TB_LAUNCH((add_rmsnorm_vec_kernel<T, 256, false, false>), n_out, 256, 0, s, x, (const T*)delta, (const T*)wy,
-                  pair_row, topk_w, k, rows, w, eps, (T*)y, d, warm, warm_bytes, tail, post_w, post_eps);
+        if (post_w) go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, true>, 256);
+        else if (d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, false, 1, false>, 256);
+        else if (d <= 256 * 8 * 2) go(add_rmsnorm_vec_kernel<T, 256, false, false, 2, false>, 256);
+        else go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, false>, 256);
         return tb_last_error();
     }
     if (post_w) return TB_ERR_UNSUPPORTED;      // the caller takes the kernel that keeps the row in shared memory
