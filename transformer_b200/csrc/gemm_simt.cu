@@ -167,10 +167,21 @@ __global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, in
     constexpr int SETS = MT * CT / 32;
     static_assert(MT * CT % 32 == 0, "the reduce-scatter takes 32 sums at a time");
     __shared__ float red[8][MT * CT];
-    pdl_sync();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wk = warp % wk_count, wn = warp / wk_count, wn_count = (blockDim.x >> 5) / wk_count;
     const int g = blockIdx.y, n0 = (blockIdx.x * wn_count + wn) * COLS;
+    if (!a.group_offsets && lane % 8 == 0) {
+        // Which rows of W a block reads does not depend on the kernel before it: their first pieces are asked into L2 while
+        // that one still runs (into L2 only, where a W that it is writing stays what it is): a request of 3 sequences and 12
+        // sampled tokens, 8 layers of width 1,024, 6.54 to 6.39 ms.
+        const int k = wk * 128 + lane * 4;
+        if (k < a.K)
+#pragma unroll
+            for (int c = 0; c < CT; ++c)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const float*>(a.B) + (size_t)g * a.b_group_stride +
+                             (size_t)(min(n0 + c % COLS, a.N - 1) + (DUAL && c >= COLS ? a.N : 0)) * a.ldb + k));
+    }
+    pdl_sync();
     const int row_lo = a.group_offsets ? a.group_offsets[g] : 0, row_hi = a.group_offsets ? a.group_offsets[g + 1] : a.M;
     if (row_lo >= row_hi) return;
     const float* B = static_cast<const float*>(a.B) + (size_t)g * a.b_group_stride;
