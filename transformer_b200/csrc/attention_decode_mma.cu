@@ -437,12 +437,22 @@ attention_decode_mma_kernel(const __grid_constant__ CUtensorMap mk, const __grid
     __syncthreads();
     if (!last_slice) return;
     __threadfence();
-    // First every slice's maximum and sum, all loads at once, to factors in shared memory (the ring's); then every thread two
-    // channels with the loads of eight slices in flight.  (A loop over the slices per channel, each load waiting for the
+    // Every thread asks for two channels of up to eight slices, then every slice's maximum and sum go to factors in shared memory
+    // (the ring's), all loads at once.  (A loop over the slices per channel, each load waiting for the
     // one before, was a large part of a step of one sequence; the sums keep their order.)
     float* f_m = sm_o;                                      // [nheads][slices] maxima
     float* f_l = f_m + nheads * slices;                     // sums
     float* f_w = f_l + nheads * slices;                     // factors; -1: the slice saw nothing and is passed over
+    constexpr int AHEAD = 8;
+    float2 v[AHEAD];
+    auto fetch = [&](int idx, int s0) {
+        const int hc = idx / (DH / 2), c = (idx - hc * (DH / 2)) * 2;
+        const float* p = a.partial + (((size_t)t * a.nh + h0 + hc) * a.splits + s0) * (DH + 2) + c;
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (s0 + u < slices) v[u] = __ldcg(reinterpret_cast<const float2*>(p + (size_t)u * (DH + 2)));
+    };
+    if (threadIdx.x < nheads * (DH / 2)) fetch(threadIdx.x, 0);
     for (int idx = threadIdx.x; idx < nheads * slices; idx += DM_THREADS) {
         const int hc = idx / slices, s = idx - hc * slices;
         const float* p = a.partial + (((size_t)t * a.nh + h0 + hc) * a.splits + s) * (DH + 2) + DH;
@@ -460,17 +470,13 @@ attention_decode_mma_kernel(const __grid_constant__ CUtensorMap mk, const __grid
     __syncthreads();
     for (int idx = threadIdx.x; idx < nheads * (DH / 2); idx += DM_THREADS) {
         const int hc = idx / (DH / 2), c = (idx - hc * (DH / 2)) * 2, h = h0 + hc;
-        const float* p = a.partial + ((size_t)t * a.nh + h) * a.splits * (DH + 2) + c;
         const float* w_row = f_w + hc * slices;
         const float* l_row = f_l + hc * slices;
         float den = 0.f, acc0 = 0.f, acc1 = 0.f;
-        for (int s0 = 0; s0 < slices; s0 += 8) {
-            float2 v[8];
+        for (int s0 = 0; s0 < slices; s0 += AHEAD) {
+            if (idx != (int)threadIdx.x || s0 > 0) fetch(idx, s0);
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (s0 + u < slices) v[u] = __ldcg(reinterpret_cast<const float2*>(p + (size_t)(s0 + u) * (DH + 2)));
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
+            for (int u = 0; u < AHEAD; ++u) {
                 if (s0 + u >= slices) break;
                 const float w = w_row[s0 + u];
                 if (w < 0.f) continue;
