@@ -481,7 +481,8 @@ static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const
             TB_LAUNCH(kernel, n_out, 512, tail.staged_at ? at + staged : smem, s, x, (const T*)delta, (const T*)wy, pair_row, topk_w, k,
                       rows, w, eps, (T*)y, d, nullptr, 0, tail, post_w, post_eps);
         };
-        if (post_w) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, true>>());
+        if (post_w && d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, 1, true>>());
+        else if (post_w) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, true>>());
         else if (d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, 1, false>>());
         else go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, false>>());
         return tb_last_error();
@@ -491,13 +492,15 @@ static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const
                   warm_bytes, tail, post_w, post_eps);
     };
     if (d % 8 == 0 && n_out <= 256 && d <= 512 * 8 * NORM_CHUNKS && y) {
-        if (post_w) go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, true>, 512);
+        if (post_w && d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, false, 1, true>, 512);
+        else if (post_w) go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, true>, 512);
         else if (d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, false, 1, false>, 512);
         else go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, false>, 512);
         return tb_last_error();
     }
     if (d % 8 == 0 && d <= 256 * 8 * NORM_CHUNKS) {
-        if (post_w) go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, true>, 256);
+        if (post_w && d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, false, 1, true>, 256);
+        else if (post_w) go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, true>, 256);
         else if (d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, false, 1, false>, 256);
         else if (d <= 256 * 8 * 2) go(add_rmsnorm_vec_kernel<T, 256, false, false, 2, false>, 256);
         else go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, false>, 256);
