@@ -16,7 +16,7 @@
 // Three kernels: gemm_simt_kernel takes anything; for float with 16-byte rows, gemm_rows_f32_kernel streams the weights
 // past a few rows (decoding), and gemm_tile_f32_kernel multiplies tiles fed by cp.async (prompts).
 #include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
-#include "common.cuh"
+#include "memory_common.cuh"            // fma2
 
 #include <type_traits>
 
@@ -271,8 +271,9 @@ static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
 // latencies of its own loads (254 rows x 1,536 x 1,024: 85 us with four warps a block, 61 with eight; an expert's pair
 // for 254 tokens 110 and 73; 2,048 x 4,096 x 4,096, where tiles abound, 1,510 and 1,674).  Tiles lie in shared memory as in memory (K innermost, rows 36 floats apart: the eight
 // rows that a quarter of a warp reads start in different banks), so a thread's operands are 16-byte loads of four
-// entries of K: 12 of them feed 128 multiply-adds.  Bound by FFMA issue; the general kernel reads one float at a time
-// (8 loads for 16 multiply-adds) and waits for global memory in every step: 148, 274 and 3,236 us for these three.
+// entries of K: 12 of them feed 128 multiply-adds, two an instruction (one each: 44, 23 and 74 us behind the kernel before for the
+// q-k-v, output and gate/up products of such a prompt, 33, 17 and 65 with two).  Bound by multiply-add issue; the general kernel reads
+// one float at a time (8 loads for 16 multiply-adds) and waits for global memory in every step: 148, 274 and 3,236 us for these three.
 #define GT_BK 32
 #define GT_PITCH (GT_BK + 4)
 #define GT_STAGES 3
@@ -308,13 +309,13 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
             else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    float acc[NB][8][4];
+    F2 acc2[NB][8][4];              // sums over the even and the odd entries of K
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[b][i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc2[b][i][j].f = make_float2(0.f, 0.f);
 #pragma unroll
     for (int st = 0; st < GT_STAGES - 1; ++st) {
         if (st < steps) issue(st);
@@ -322,6 +323,7 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
     }
     const int ty = lane >> 3, tx = lane & 7, wm = (warp >> 1 & 1) * 32, wn = (warp & 1) * 32;
     const int k_half = warp >> 2;
+    union Four { float4 f; F2 p[2]; };
     for (int st = 0; st < steps; ++st) {
         cp_async_wait<GT_STAGES - 2>();
         __syncthreads();            // this stage is there for everyone, and everyone is done with the one before
@@ -331,25 +333,31 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
         const float* Bs = gt + (st % GT_STAGES) * STAGE + (64 + wn + tx) * GT_PITCH + k_half * (GT_BK / 2);
 #pragma unroll 2
         for (int k = 0; k < GT_BK / 2; k += 4) {
-            float4 av[8];
+            Four av[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float4*>(As + 4 * i * GT_PITCH + k);
+            for (int i = 0; i < 8; ++i) av[i].f = *reinterpret_cast<const float4*>(As + 4 * i * GT_PITCH + k);
 #pragma unroll
             for (int b = 0; b < NB; ++b)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 bv = *reinterpret_cast<const float4*>(Bs + (b * 64 + 8 * j) * GT_PITCH + k);
+                    Four bv;
+                    bv.f = *reinterpret_cast<const float4*>(Bs + (b * 64 + 8 * j) * GT_PITCH + k);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        float& v = acc[b][i][j];
-                        v = fmaf(av[i].x, bv.x, v);
-                        v = fmaf(av[i].y, bv.y, v);
-                        v = fmaf(av[i].z, bv.z, v);
-                        v = fmaf(av[i].w, bv.w, v);
+                        F2& v = acc2[b][i][j];
+                        v = fma2(av[i].p[0], bv.p[0], v);
+                        v = fma2(av[i].p[1], bv.p[1], v);
                     }
                 }
         }
     }
+    float acc[NB][8][4];
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[b][i][j] = acc2[b][i][j].f.x + acc2[b][i][j].f.y;
     // the second half's sums to shared memory (a warp's 32 x NB values a lane, lane innermost), the first half adds them
     __syncthreads();
     float* part = gt + (warp & 3) * (NB * 1024) + lane;
