@@ -21,7 +21,9 @@ def _product(a, w):
 @pytest.mark.parametrize("M,N,K", [(1, 8, 4), (3, 1536, 1024), (4, 130, 516), (5, 67, 260), (8, 1, 2048), (9, 33, 124),
                                    (16, 100, 1028), (17, 64, 36), (63, 65, 32), (64, 64, 96), (130, 200, 100), (254, 129, 520),
                                    (3, 20, 1022), (70, 40, 33), (1, 8, 256), (4, 130, 260), (9, 33, 380),
-                                   (17, 64, 292), (63, 65, 288), (64, 64, 352), (130, 200, 356), (254, 129, 260)])
+                                   (17, 64, 292), (63, 65, 288), (64, 64, 352), (130, 200, 356), (254, 129, 260),
+                                   (1, 8, 512), (5, 67, 516), (9, 33, 636), (17, 64, 548), (63, 65, 512), (64, 64, 608),
+                                   (130, 200, 612)])
 @pytest.mark.parametrize("kind", [0, 3])
 def test_dense(M, N, K, kind):
     from transformer_b200.parts.linear import gemm_simt
@@ -38,7 +40,8 @@ def test_dense(M, N, K, kind):
 
 @pytest.mark.parametrize("sizes,N,K", [([1, 0, 2], 512, 1024), ([0, 3, 0, 5, 1], 44, 300), ([40, 0, 3, 1], 33, 260),
                                        ([100, 64, 0, 65, 1], 70, 36), ([6, 6, 6, 6], 24, 22),
-                                       ([100, 64, 0, 65, 1], 70, 292), ([0, 3, 0, 5, 1], 44, 256)])
+                                       ([100, 64, 0, 65, 1], 70, 292), ([0, 3, 0, 5, 1], 44, 256),
+                                       ([100, 64, 0, 65, 1], 70, 548), ([0, 3, 0, 5, 1], 44, 512), ([40, 0, 3, 1], 33, 516)])
 @pytest.mark.parametrize("glu", [None, (1.702, 7.0)])
 def test_grouped_pair_of_gathered_rows(sizes, N, K, glu):
     from transformer_b200.parts.linear import gemm_simt

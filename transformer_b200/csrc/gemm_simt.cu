@@ -391,8 +391,10 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
 // taken 4, 8 or 16 at a time by what most groups hold, as gemm_skinny does; above, tiles.  Measured at the border: 16
 // rows x 1,536 x 1,024 7.1 us here, 17 rows 39 us in tiles; a pair of 8 experts (1,024 -> 512) 25 us for groups of 15 rows
 // here, 73 for groups of 25 in tiles (one tile a group, mostly empty, and the general kernel's 200 and 219).
-// Rows shorter than GF_K stay with the general kernel, whose walk over K is short then.
-#define GF_K 256
+// Rows shorter than GF_K stay with the general kernel, whose walk over K is short then (calls from Python one after the other: 254
+// rows x 1,024 x 252 22.6 us, x 256 in tiles 12.8; 3 rows x 512 x 128 13 us with either): models that small have tokens whose
+// logits another order of the sums moves by several times their mean error, and little to win.
+#define GF_K 512
 static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
     if (a.K < GF_K || a.K % 4 || a.lda % 4 || a.ldb % 4 || a.b_group_stride % 4 || (((uintptr_t)a.A | (uintptr_t)a.B) & 15)) return false;
     if (a.M <= 16 * a.G && a.G <= 65535) {

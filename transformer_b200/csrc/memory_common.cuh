@@ -1,4 +1,5 @@
-// What the kernels of the linear memories (decay_memory.cu, gated_linear.cu, split_delta.cu) share.
+// What the kernels of the linear memories (decay_memory.cu, gated_linear.cu, split_delta.cu) share; the packed multiply-add is
+// used by gemm_simt.cu and channel_delta_chunk.cu as well.
 #pragma once
 #include "common.cuh"
 
