@@ -153,11 +153,16 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
     auto k_empty = [&](int s) { return bar0 + 8u * (AT_STAGES + s); };
     auto v_full = [&](int s) { return bar0 + 8u * (2 * AT_STAGES + s); };
     auto v_empty = [&](int s) { return bar0 + 8u * (3 * AT_STAGES + s); };
-    const uint32_t q_full = bar0 + 8u * (4 * AT_STAGES), o_done = q_full + 16;
-    auto s_full = [&](int i) { return q_full + 24 + 8u * i; };      // one per S buffer
-    // ... and one per S buffer for "P is in it": a softmax warp may be a tile ahead of the others (nothing holds it
-    // back but the scores), and its arrival for the next tile must not count towards this one
-    auto p_ready = [&](int i) { return i == 0 ? q_full + 8 : q_full + 40; };
+    const uint32_t q_full = bar0 + 8u * (4 * AT_STAGES);
+    // Two of each, by the tile's parity.  P ready: a softmax warp may be a tile ahead of the others (nothing holds it
+    // back but the scores), and its arrival for the next tile must not count towards this one.  O done: a warp hands
+    // over P of tile j and then waits for the product of tile j - 1.  Product j may end in between, however long the
+    // warp is held up there, so it completes another barrier: on one for all tiles the warp would find the phase
+    // after the one it wants, take it for the one before, and wait for product j + 1, which waits for this warp.
+    // Product j + 1, the next on the barrier of j - 1, cannot begin before this warp has handed over P of tile j + 1.
+    auto s_full = [&](int i) { return q_full + 8 + 8u * i; };
+    auto p_ready = [&](int i) { return q_full + 24 + 8u * i; };
+    auto o_done = [&](int i) { return q_full + 40 + 8u * i; };
     if (threadIdx.x == 0) {
         for (int s = 0; s < AT_STAGES; ++s) {
             mbar_init(k_full(s), 1);
@@ -170,7 +175,8 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
         mbar_init(s_full(1), 1);
         mbar_init(p_ready(0), 4);    // one arrival per softmax warp
         mbar_init(p_ready(1), 4);
-        mbar_init(o_done, 1);
+        mbar_init(o_done(0), 1);
+        mbar_init(o_done(1), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
@@ -258,7 +264,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
                     umma_bf16_ts(tmem_o, tmem_s + (j & 1) * AT_BN + 8 * k, dv, idesc_o, (j | k) != 0);
                 }
                 umma_commit(v_empty(s));
-                umma_commit(o_done);
+                umma_commit(o_done(j & 1));
             }
         }
     } else {
@@ -341,7 +347,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             // which nothing reads any more: no wait for that)
             const bool touch_o = __any_sync(0xffffffffu, rescale != 1.0f) && j > 0;
             if (touch_o) {
-                ok = mbar_wait(o_done, (j - 1) & 1, a.error, 16);
+                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
                 tc_fence_after();
                 if (!ok) break;
 #pragma unroll
@@ -359,16 +365,16 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             tc_fence_before();
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(p_ready(j & 1)) : "memory");
-            // Keep in step with the products' completions, one phase at a time (a wait on a phase's parity cannot
+            // Keep in step with the products' completions, phase by phase (a wait on a phase's parity cannot
             // tell "two behind" from "done").  Here it costs nothing: P has been handed over, and the product
             // waited for was issued a whole tile ago.
             if (j > 0 && !touch_o) {
-                ok = mbar_wait(o_done, (j - 1) & 1, a.error, 16);
+                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
                 tc_fence_after();
             }
         }
         if (ok) {
-            ok = mbar_wait(o_done, (n_tiles - 1) & 1, a.error, 17);
+            ok = mbar_wait(o_done((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, a.error, 17);
             tc_fence_after();
         }
         if (ok) {
