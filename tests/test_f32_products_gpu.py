@@ -38,6 +38,22 @@ def test_dense(M, N, K, kind):
     assert bool((out[:, N:] == 7.0).all()), "nothing past the last column is written"
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 40, 1024), (17, 70, 512), (45, 33, 516), (48, 64, 64), (49, 65, 520)])
+@pytest.mark.parametrize("kind", [0, 2])
+def test_groups_without_offsets_take_the_first_matrix(M, N, K, kind):
+    """Up to and above 16 rows a group, where another kernel takes over: every block that writes a place has matrix 0."""
+    from transformer_b200.parts.linear import gemm_simt
+    a, w = _rand((M, K), 6), _rand((3, N if kind == 0 else 2 * N, K), 7) * K ** -0.5
+    out, one = torch.full((M, N), 7.0, device="cuda"), torch.full((M, N), 7.0, device="cuda")
+    for _ in range(20):
+        gemm_simt(a, w, out, groups=3, out_kind=kind)
+        gemm_simt(a, w[0], one, out_kind=kind)
+        assert torch.equal(out, one)
+    if kind == 0:
+        want, bound = _product(a, w[0])
+        assert bool(((out.double() - want).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("sizes,N,K", [([1, 0, 2], 512, 1024), ([0, 3, 0, 5, 1], 44, 300), ([40, 0, 3, 1], 33, 260),
                                        ([100, 64, 0, 65, 1], 70, 36), ([6, 6, 6, 6], 24, 22),
                                        ([100, 64, 0, 65, 1], 70, 292), ([0, 3, 0, 5, 1], 44, 256),

@@ -261,7 +261,8 @@ static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
     // as many warps on K as it has pieces of 128 entries, up to eight; with fewer than four, more columns a block
     const int wk = a.K >= 1024 ? 8 : a.K >= 512 ? 4 : a.K >= 256 ? 2 : 1;
     const int warps = wk == 8 ? 8 : 4, cols = (DUAL ? CT / 2 : CT) * (warps / wk);
-    TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL>), dim3((a.N + cols - 1) / cols, a.G), warps * 32, 0, s, a, wk);
+    // without offsets all rows belong to matrix 0, whatever G is: a block for every g would write the same places
+    TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL>), dim3((a.N + cols - 1) / cols, a.group_offsets ? a.G : 1), warps * 32, 0, s, a, wk);
 }
 
 // ---- many rows (prompts) -------------------------------------------------------------------------------------------
@@ -397,8 +398,9 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
 #define GF_K 512
 static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
     if (a.K < GF_K || a.K % 4 || a.lda % 4 || a.ldb % 4 || a.b_group_stride % 4 || (((uintptr_t)a.A | (uintptr_t)a.B) & 15)) return false;
-    if (a.M <= 16 * a.G && a.G <= 65535) {
-        const int usual = a.G > 1 ? (3 * a.M / a.G + 1) / 2 : a.M;
+    const int G = a.group_offsets ? a.G : 1;
+    if (a.M <= 16 * G && G <= 65535) {
+        const int usual = G > 1 ? (3 * a.M / G + 1) / 2 : a.M;
         if (usual <= 4) dual ? gemm_rows_f32_go<4, 8, true>(a, s) : gemm_rows_f32_go<4, 8, false>(a, s);
         else if (usual <= 8) dual ? gemm_rows_f32_go<8, 8, true>(a, s) : gemm_rows_f32_go<8, 8, false>(a, s);
         else dual ? gemm_rows_f32_go<16, 4, true>(a, s) : gemm_rows_f32_go<16, 4, false>(a, s);
