@@ -38,6 +38,26 @@ def test_dense(M, N, K, kind):
     assert bool((out[:, N:] == 7.0).all()), "nothing past the last column is written"
 
 
+@pytest.mark.parametrize("sizes", [[0] * 39 + [640], [300] + [0] * 39, [257, 0, 1, 256] + [0] * 50 + [255, 12],
+                                   [65, 129, 0, 64] + [1] * 76, [130] + [0] * 99, [16] * 40])
+def test_crowded_groups_are_dealt_to_several_blocks(sizes):
+    """Few rows a group on average (the weights' kernel) and one group with many: slices of 16 passes of 4, 8 or 16 rows, found
+    by 32 groups at a time."""
+    from transformer_b200.parts.linear import gemm_simt
+    G, M, N, K = len(sizes), sum(sizes), 37, 516
+    assert 16 * 4 < M <= 16 * G
+    x, w = _rand((M, K), 8), _rand((G, N, K), 9) * K ** -0.5
+    offsets = torch.tensor([0] + sizes).cumsum(0).to(torch.int32).cuda()
+    out = torch.full((M, N), 7.0, device="cuda")
+    gemm_simt(x, w, out, group_offsets=offsets, groups=G)
+    at = 0
+    for g, n in enumerate(sizes):
+        if n:
+            want, bound = _product(x[at:at + n], w[g])
+            assert bool(((out[at:at + n].double() - want).abs() <= bound).all())
+        at += n
+
+
 @pytest.mark.parametrize("M,N,K", [(3, 40, 1024), (17, 70, 512), (45, 33, 516), (48, 64, 64), (49, 65, 520)])
 @pytest.mark.parametrize("kind", [0, 2])
 def test_groups_without_offsets_take_the_first_matrix(M, N, K, kind):

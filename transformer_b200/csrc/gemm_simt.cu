@@ -161,7 +161,12 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmArgs a) {
 // kernel walks K in steps of 16 with two barriers each and was bound by that chain: 3 rows x 1,536
 // x 1,024 took 55.7 us and take 3.0 (2.1 TB/s), x 32,000 x 1,024 275 and 34 us (3.9 TB/s), 16 rows x 1,536 x 1,024 56.4
 // and 7.1 us; a decode step of three sequences (width 1,024, 8 layers, 8 experts of 512) 4.6 and 0.58 ms.
-template <int MT, int CT, bool DUAL>
+// SLICED (many rows, no pair): the rows of a crowded group are dealt to several blocks, 16 passes each.  2,048 rows for 128 experts
+// (512 -> 1,024) that all went to one: 442 us by the blocks of that expert alone (the general kernel: 390), 217 so; evenly
+// spread 223 and 216.  A pair has twice the work a row and stays ahead of the general kernel without (424 and 714 us; dealt out, its
+// registers run out and an even spread costs 7 % more).
+#define GR_PASSES 16
+template <int MT, int CT, bool DUAL, bool SLICED>
 __global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, int wk_count) {
     constexpr int COLS = DUAL ? CT / 2 : CT;
     constexpr int SETS = MT * CT / 32;
@@ -169,7 +174,8 @@ __global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, in
     __shared__ float red[8][MT * CT];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wk = warp % wk_count, wn = warp / wk_count, wn_count = (blockDim.x >> 5) / wk_count;
-    const int g = blockIdx.y, n0 = (blockIdx.x * wn_count + wn) * COLS;
+    int g = blockIdx.y;
+    const int n0 = (blockIdx.x * wn_count + wn) * COLS;
     if (!a.group_offsets && lane % 8 == 0) {
         // Which rows of W a block reads does not depend on the kernel before it: their first pieces are asked into L2 while
         // that one still runs (into L2 only, where a W that it is writing stays what it is): a request of 3 sequences and 12
@@ -182,7 +188,39 @@ __global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, in
                              (size_t)(min(n0 + c % COLS, a.N - 1) + (DUAL && c >= COLS ? a.N : 0)) * a.ldb + k));
     }
     pdl_sync();
-    const int row_lo = a.group_offsets ? a.group_offsets[g] : 0, row_hi = a.group_offsets ? a.group_offsets[g + 1] : a.M;
+    int row_lo = 0, row_hi = a.M;
+    if (!SLICED && a.group_offsets) {
+        row_lo = a.group_offsets[g];
+        row_hi = a.group_offsets[g + 1];
+    }
+    if (SLICED) {
+        constexpr int SLICE = GR_PASSES * MT;
+        int slice = 0;
+        if (g >= a.G) {         // a slice behind some group's first: which?  (32 groups at a time, every warp by itself)
+            int want = g - a.G;
+            g = -1;
+            for (int g0 = 0; g0 < a.G && g < 0; g0 += 32) {
+                int more = 0;
+                if (g0 + lane < a.G) more = (a.group_offsets[g0 + lane + 1] - a.group_offsets[g0 + lane] - 1) / SLICE;
+                int upto = more;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += u;
+                }
+                const unsigned past = __ballot_sync(0xffffffffu, want < upto);
+                if (past) {
+                    const int src = __ffs(past) - 1;
+                    g = g0 + src;
+                    slice = want - __shfl_sync(0xffffffffu, upto - more, src) + 1;
+                }
+                want -= __shfl_sync(0xffffffffu, upto, 31);
+            }
+            if (g < 0) return;
+        }
+        row_lo = a.group_offsets[g] + slice * SLICE;
+        row_hi = min(a.group_offsets[g + 1], row_lo + SLICE);
+    }
     if (row_lo >= row_hi) return;
     const float* B = static_cast<const float*>(a.B) + (size_t)g * a.b_group_stride;
     const float* A = static_cast<const float*>(a.A);
@@ -261,8 +299,11 @@ static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
     // as many warps on K as it has pieces of 128 entries, up to eight; with fewer than four, more columns a block
     const int wk = a.K >= 1024 ? 8 : a.K >= 512 ? 4 : a.K >= 256 ? 2 : 1;
     const int warps = wk == 8 ? 8 : 4, cols = (DUAL ? CT / 2 : CT) * (warps / wk);
-    // without offsets all rows belong to matrix 0, whatever G is: a block for every g would write the same places
-    TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL>), dim3((a.N + cols - 1) / cols, a.group_offsets ? a.G : 1), warps * 32, 0, s, a, wk);
+    // Without offsets all rows belong to matrix 0, whatever G is: a block for every g would write the same places.
+    const int groups = a.group_offsets ? a.G : 1, blocks = (a.N + cols - 1) / cols;
+    const int more = a.group_offsets ? (a.M - 1) / (GR_PASSES * MT) : 0;        // slices behind the groups' first: at most so many
+    if (!DUAL && more > 0) TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL, !DUAL>), dim3(blocks, groups + more), warps * 32, 0, s, a, wk);
+    else TB_LAUNCH((gemm_rows_f32_kernel<MT, CT, DUAL, false>), dim3(blocks, groups), warps * 32, 0, s, a, wk);
 }
 
 // ---- many rows (prompts) -------------------------------------------------------------------------------------------
@@ -399,7 +440,7 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
 static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
     if (a.K < GF_K || a.K % 4 || a.lda % 4 || a.ldb % 4 || a.b_group_stride % 4 || (((uintptr_t)a.A | (uintptr_t)a.B) & 15)) return false;
     const int G = a.group_offsets ? a.G : 1;
-    if (a.M <= 16 * G && G <= 65535) {
+    if (a.M <= 16 * G && G + a.M / (GR_PASSES * 4) <= 65535) {       // blocks in y, with passes of four rows
         const int usual = G > 1 ? (3 * a.M / G + 1) / 2 : a.M;
         if (usual <= 4) dual ? gemm_rows_f32_go<4, 8, true>(a, s) : gemm_rows_f32_go<4, 8, false>(a, s);
         else if (usual <= 8) dual ? gemm_rows_f32_go<8, 8, true>(a, s) : gemm_rows_f32_go<8, 8, false>(a, s);
