@@ -46,10 +46,11 @@ def test_against_the_rules(kind, V, k, p):
             assert (cum[at - 1] if at else 0.0) - 2e-5 <= u <= cum[at] + 2e-5
 
 
-@pytest.mark.parametrize("nt", [1, 3, 40])
-@pytest.mark.parametrize("nh,nkvh,dh", [(4, 1, 128), (5, 1, 64), (2, 2, 16), (6, 2, 32)])
+@pytest.mark.parametrize("nt", [1, 3, 4, 5, 6, 7, 40])
+@pytest.mark.parametrize("nh,nkvh,dh", [(4, 1, 128), (5, 1, 64), (2, 2, 16), (6, 2, 32), (4, 2, 64)])
 def test_decode_attention_in_32_bits(nt, nh, nkvh, dh):
-    """Few sequences take a head per block and 512 threads, many the four-head form: both against 64 bits.  Scores of unit
+    """Few heads (up to 8, 16 or 24 by the size of a group) take a block each with 512 threads, more the one-, two- and four-head
+    forms: all against 64 bits.  Scores of unit
     normal values over sqrt(dh): 1e-5 covers the float sums of 700 keys."""
     from transformer_b200.csrc import lib
     g = torch.Generator().manual_seed(nt + dh)

@@ -227,11 +227,15 @@ static int decode_launch(const DecodeArgs& a, int nt, cudaStream_t s) {
     if (nt <= 0) return nt == 0 ? 0 : TB_ERR_ARG;
     const int group = a.nh / a.nkvh;
     int rc;
-    // 32 bits, a few short sequences (a slice holds two pages or more, so three sequences of 200 keys are six blocks of four
-    // heads): a head per block and four times the threads, so that 64 keys of 128 entries are in flight at once.
-    // Three sequences of 4 heads, 1 key head and 16 to 200 keys: 5.6 us (24.5 with four heads and 128 threads a block).
+    // 32 bits, a few heads: a head per block and four times the threads, so that 64 keys of 128 entries are in flight at once.
+    // Each of a group's heads then reads the cache by itself, so the line lies where that begins to cost with long contexts
+    // (a call and its merge, us, head per block and four heads of 128 threads; 100 / 2,000 / 8,000 keys): groups of four, 16
+    // heads 7.4 / 15.7 / 38.9 and 23.0 / 28.8 / 56.1, 24 heads 7.4 / 20.8 / 53.5 and 23.1 / 31.3 / 58.1, 32
+    // heads 7.6 / 25.7 / 64.5 and 23.1 / 32.4 / 59.2; groups of two, 16 heads 7.4 / 15.6 / 39.0 and 14.2 / 22.0 / 40.7; single heads, 8
+    // 7.4 / 10.8 / 24.2 and 10.0 / 17.9 / 36.7, 16 7.4 / 15.6 / 48.7 and 10.5 / 23.2 / 46.0.  A captured step keeps its shape for
+    // as long as the sequences grow, so their lengths cannot enter.
     bool few = false;
-    if constexpr (std::is_same<T, float>::value) few = (long long)nt * a.nkvh * ((group + 3) / 4) <= 37;
+    if constexpr (std::is_same<T, float>::value) few = (long long)nt * a.nh <= 8 * (group < 3 ? group : 3);
     if (few)
         rc = decode_launch_gc<T, 1, 4 * AD_THREADS>(a, nt, s);
     else if (group == 1)
