@@ -5,6 +5,8 @@
 #include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
 #include "router_pick.cuh"
 
+#include <type_traits>
+
 // x[i, :] = table[tokens[i], :]   (models/llama/cuda/src/infer.rs:98-104 copies row by row)
 template <typename T>
 __global__ void embed_kernel(const int* __restrict__ tokens, const T* __restrict__ table,
@@ -136,7 +138,11 @@ __device__ __forceinline__ void experts_sum(const T* __restrict__ wy, const int*
 // CH: pieces of 8 values a thread keeps (NORM_THREADS * 8 * CH >= d), POST: whether post_w is given.  What a width or a form does
 // not need costs registers, hence blocks on an SM, and code: 2,048 rows of 4,096 took 31 us (sums and experts' sums, mean)
 // with room for 8,192 values and the experts' rows loaded one after the other, and take 24.
-template <typename T, int NORM_THREADS, bool EARLY, bool TAIL, int CH, bool POST>
+// TAIL: 0 no router behind the norm; otherwise where its matrix comes from: TAIL_EARLY a warp's first 8 KB in registers before the
+// wait and the rest eight loads at a time, TAIL_SHORT from shared memory (`staged_at`) or four loads at a time.
+#define TAIL_EARLY 1
+#define TAIL_SHORT 2
+template <typename T, int NORM_THREADS, bool EARLY, int TAIL, int CH, bool POST>
 __global__ void __launch_bounds__(NORM_THREADS)
 add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const T* __restrict__ wy,
                        const int* __restrict__ pair_row, const float* __restrict__ topk_w, int k,
@@ -144,13 +150,23 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
                        int d, const void* warm, int warm_bytes, const RouterTail<T> tail,
                        const float* __restrict__ post_w, float post_eps) {
     // post_w: the delta is normed by itself first (delta / rms(delta) * post_w, with post_eps) and then added
-    constexpr int EPL = Vec16<T>::N;
+    constexpr int EPL = Vec16<T>::N, UN = 8;
     // TAIL: the row as T [d], the logits [E] (and scores), and, if `staged`, a row of the router's matrix per warp [warps][d]
     extern __shared__ __align__(16) unsigned char tail_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* const ys = reinterpret_cast<T*>(tail_smem);
     T* const my_w = TAIL ? reinterpret_cast<T*>(tail_smem + tail.staged_at) + (size_t)warp * d : nullptr;
-    if (TAIL) {
+    uint4 first[TAIL == TAIL_EARLY ? UN : 1];
+    if (TAIL == TAIL_EARLY) {
+        if (warp < tail.E) {
+#pragma unroll
+            for (int u = 0; u < UN; ++u) {
+                const int c = (lane + u * 32) * EPL;
+                first[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (c < d) first[u] = *reinterpret_cast<const uint4*>(tail.w + (size_t)warp * d + c);
+            }
+        }
+    } else if (TAIL == TAIL_SHORT) {
         if (tail.staged_at && warp < tail.E) {
 #pragma unroll 1
             for (int c = lane * EPL; c < d; c += 32 * EPL)
@@ -262,19 +278,44 @@ add_rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const
     if (!TAIL) return;
     __syncthreads();
     float* lg = reinterpret_cast<float*>(tail_smem + (size_t)d * sizeof(T));
-    if (tail.staged_at) cp_async_wait<0>();         // a lane reads what it copied itself
-    // A loop of a few instructions: the block runs once, and code that has to be fetched for it costs more than it saves (a step
-    // of one sequence, width 4,096, 16 experts: 9.0 us behind the kernel before with the row unrolled in registers, 7.7 so)
+    if (TAIL == TAIL_SHORT && tail.staged_at) cp_async_wait<0>();         // a lane reads what it copied itself
     for (int e = warp; e < tail.E; e += NORM_THREADS / 32) {
-        const T* we = tail.staged_at && e == warp ? my_w : tail.w + (size_t)e * d;
+        const T* we = TAIL == TAIL_SHORT && tail.staged_at && e == warp ? my_w : tail.w + (size_t)e * d;
         float acc = 0.f;
-#pragma unroll 4
-        for (int c = lane * EPL; c < d; c += 32 * EPL) {
-            float xf[EPL], wf[EPL];
-            Vec16<T>::unpack(*reinterpret_cast<const uint4*>(ys + c), xf);
-            Vec16<T>::unpack(*reinterpret_cast<const uint4*>(we + c), wf);
+        if (TAIL == TAIL_EARLY) {
+            for (int c0 = lane * EPL; c0 < d; c0 += 32 * EPL * UN) {
+                uint4 xv[UN], wv[UN];
+                const bool have = e == warp && c0 == lane * EPL;     // the batch read before the wait
 #pragma unroll
-            for (int q = 0; q < EPL; ++q) acc += xf[q] * wf[q];
+                for (int u = 0; u < UN; ++u) {
+                    const int c = c0 + u * 32 * EPL;
+                    xv[u] = wv[u] = make_uint4(0u, 0u, 0u, 0u);
+                    if (c < d) {
+                        xv[u] = *reinterpret_cast<const uint4*>(ys + c);
+                        wv[u] = have ? first[TAIL == TAIL_EARLY ? u : 0] : *reinterpret_cast<const uint4*>(we + c);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < UN; ++u) {
+                    float xf[EPL], wf[EPL];
+                    Vec16<T>::unpack(xv[u], xf);
+                    Vec16<T>::unpack(wv[u], wf);
+#pragma unroll
+                    for (int q = 0; q < EPL; ++q) acc += xf[q] * wf[q];
+                }
+            }
+        } else {
+            // A loop of a few instructions: the block runs once, and code that has to be fetched for it costs more than it
+            // saves (a step of one sequence, width 4,096, 16 experts: 9.0 us behind the kernel before with the row unrolled
+            // in registers, 7.7 so)
+#pragma unroll 4
+            for (int c = lane * EPL; c < d; c += 32 * EPL) {
+                float xf[EPL], wf[EPL];
+                Vec16<T>::unpack(*reinterpret_cast<const uint4*>(ys + c), xf);
+                Vec16<T>::unpack(*reinterpret_cast<const uint4*>(we + c), wf);
+#pragma unroll
+                for (int q = 0; q < EPL; ++q) acc += xf[q] * wf[q];
+            }
         }
         acc = warp_sum(acc);
         if (lane == 0) lg[e] = acc;
@@ -449,6 +490,7 @@ static int embed_launch(const int* tokens, const void* table, float* x, int nt, 
 }
 #define TAIL_SMEM (200 * 1024)
 #define TAIL_STAGED_ROWS 16     // more rows: the blocks find the router's matrix in L2
+#define TAIL_EARLY_ROWS 148     // more rows: the SMs take a second block, which the registers of the early read would not leave room for
 // The kernel, allowed that much shared memory.
 template <auto Kernel> static auto tail_kernel() {
     static std::once_flag raised;
@@ -481,10 +523,15 @@ static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const
             TB_LAUNCH(kernel, n_out, 512, tail.staged_at ? at + staged : smem, s, x, (const T*)delta, (const T*)wy, pair_row, topk_w, k,
                       rows, w, eps, (T*)y, d, nullptr, 0, tail, post_w, post_eps);
         };
-        if (post_w && d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, 1, true>>());
-        else if (post_w) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, true>>());
-        else if (d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, 1, false>>());
-        else go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, true, NORM_CHUNKS, false>>());
+        auto pick = [&](auto form) {
+            constexpr int F = decltype(form)::value;
+            if (post_w && d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, F, 1, true>>());
+            else if (post_w) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, F, NORM_CHUNKS, true>>());
+            else if (d <= 512 * 8) go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, F, 1, false>>());
+            else go(tail_kernel<add_rmsnorm_vec_kernel<T, 512, true, F, NORM_CHUNKS, false>>());
+        };
+        if (!tail.staged_at && n_out <= TAIL_EARLY_ROWS) pick(std::integral_constant<int, TAIL_EARLY>());
+        else pick(std::integral_constant<int, TAIL_SHORT>());
         return tb_last_error();
     }
     auto go = [&](auto kernel, int threads) {
@@ -492,18 +539,18 @@ static int add_rmsnorm_launch(float* x, const void* delta, const void* wy, const
                   warm_bytes, tail, post_w, post_eps);
     };
     if (d % 8 == 0 && n_out <= 256 && d <= 512 * 8 * NORM_CHUNKS && y) {
-        if (post_w && d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, false, 1, true>, 512);
-        else if (post_w) go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, true>, 512);
-        else if (d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, false, 1, false>, 512);
-        else go(add_rmsnorm_vec_kernel<T, 512, true, false, NORM_CHUNKS, false>, 512);
+        if (post_w && d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, 0, 1, true>, 512);
+        else if (post_w) go(add_rmsnorm_vec_kernel<T, 512, true, 0, NORM_CHUNKS, true>, 512);
+        else if (d <= 512 * 8) go(add_rmsnorm_vec_kernel<T, 512, true, 0, 1, false>, 512);
+        else go(add_rmsnorm_vec_kernel<T, 512, true, 0, NORM_CHUNKS, false>, 512);
         return tb_last_error();
     }
     if (d % 8 == 0 && d <= 256 * 8 * NORM_CHUNKS) {
-        if (post_w && d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, false, 1, true>, 256);
-        else if (post_w) go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, true>, 256);
-        else if (d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, false, 1, false>, 256);
-        else if (d <= 256 * 8 * 2) go(add_rmsnorm_vec_kernel<T, 256, false, false, 2, false>, 256);
-        else go(add_rmsnorm_vec_kernel<T, 256, false, false, NORM_CHUNKS, false>, 256);
+        if (post_w && d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, 0, 1, true>, 256);
+        else if (post_w) go(add_rmsnorm_vec_kernel<T, 256, false, 0, NORM_CHUNKS, true>, 256);
+        else if (d <= 256 * 8) go(add_rmsnorm_vec_kernel<T, 256, false, 0, 1, false>, 256);
+        else if (d <= 256 * 8 * 2) go(add_rmsnorm_vec_kernel<T, 256, false, 0, 2, false>, 256);
+        else go(add_rmsnorm_vec_kernel<T, 256, false, 0, NORM_CHUNKS, false>, 256);
         return tb_last_error();
     }
     if (post_w) return TB_ERR_UNSUPPORTED;      // the caller takes the kernel that keeps the row in shared memory
