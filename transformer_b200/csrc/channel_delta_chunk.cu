@@ -391,10 +391,8 @@ static int delta_chunk_go(const DeltaPrepArgs& p, int nt, int B, int max_chunks,
 template <int DIM, int LANES, int C>
 static int delta_chunk_scan_go(const DeltaChunkScanArgs& a, int B, cudaStream_t s) {
     constexpr size_t smem = (size_t)DC_STAGES * ((3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP + DC_TOK * DC_COLS) * sizeof(float);
-    static std::once_flag raised;
-    std::call_once(raised, [] {
-        tb_note_error(cudaFuncSetAttribute(delta_chunk_scan_kernel<DIM, LANES, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    });
+    static PerDevice raised;
+    tb_allow_smem(raised, (const void*)delta_chunk_scan_kernel<DIM, LANES, C>, smem);
     // the blocks run for the whole sequence and want an SM each (see tb_launch_plain)
     tb_launch_plain(delta_chunk_scan_kernel<DIM, LANES, C>, dim3(B, a.H, a.vdim / DC_COLS), dim3(128), smem, s, a);
     return tb_last_error();

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 #define TB_PAGE 64  // tokens in one cache page
 
 // argument errors returned by launchers (cudaError_t values are positive)
@@ -175,6 +177,18 @@ static inline void tb_note_error(cudaError_t e) {
         cudaGetLastError();   // the runtime's own copy would otherwise be blamed on a later, innocent call
         if (!tb_pending_error()) tb_pending_error() = (int)e;
     }
+}
+
+// Lets `kernel` have `bytes` of dynamic shared memory on the device that is current; `set` belongs to the kernel.
+static inline void tb_allow_smem(PerDevice& set, const void* kernel, size_t bytes) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return tb_note_error(e);
+    set.once(device, [&] {
+        const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        tb_note_error(rc);
+        return rc == cudaSuccess;
+    });
 }
 
 static inline void tb_state_carveout(const void* kernel, unsigned threads, size_t dyn_smem) {

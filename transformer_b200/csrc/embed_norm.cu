@@ -493,8 +493,8 @@ static int embed_launch(const int* tokens, const void* table, float* x, int nt, 
 #define TAIL_EARLY_ROWS 148     // more rows: the SMs take a second block, which the registers of the early read would not leave room for
 // The kernel, allowed that much shared memory.
 template <auto Kernel> static auto tail_kernel() {
-    static std::once_flag raised;
-    std::call_once(raised, [] { tb_note_error(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM)); });
+    static PerDevice raised;
+    tb_allow_smem(raised, (const void*)Kernel, TAIL_SMEM);
     return Kernel;
 }
 

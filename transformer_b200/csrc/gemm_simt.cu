@@ -450,11 +450,8 @@ static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
     const int tiles = (a.M + 63) / 64 + (a.group_offsets ? a.G : 0), cols = (a.N + 63) / 64;
     if (cols > 65535) return false;
     const size_t smem = (size_t)GT_STAGES * (dual ? 3 : 2) * 64 * GT_PITCH * sizeof(float);
-    static std::once_flag raised;
-    std::call_once(raised, [] {
-        tb_note_error(cudaFuncSetAttribute(gemm_tile_f32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        tb_note_error(cudaFuncSetAttribute(gemm_tile_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-    });
+    static PerDevice raised[2];
+    tb_allow_smem(raised[dual], dual ? (const void*)gemm_tile_f32_kernel<true> : (const void*)gemm_tile_f32_kernel<false>, smem);
     if (dual) TB_LAUNCH((gemm_tile_f32_kernel<true>), dim3(tiles, cols), 256, smem, s, a);
     else TB_LAUNCH((gemm_tile_f32_kernel<false>), dim3(tiles, cols), 256, smem, s, a);
     return true;

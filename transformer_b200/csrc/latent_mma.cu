@@ -581,10 +581,8 @@ static size_t latent_rows_smem(int DK) {
 
 template <int NT>
 static int latent_rows_go(const LatentMmaArgs& a, int tiles, cudaStream_t s) {
-    static std::once_flag raised;
-    std::call_once(raised, [] {
-        tb_note_error(cudaFuncSetAttribute(latent_rows_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    });
+    static PerDevice raised;
+    tb_allow_smem(raised, (const void*)latent_rows_kernel<NT>, 227 * 1024);
     dim3 grid((tiles + LR_TILES - 1) / LR_TILES, (a.H + a.heads_per_block - 1) / a.heads_per_block);
     TB_LAUNCH((latent_rows_kernel<NT>), grid, 256, latent_rows_smem(a.rank + a.rot), s, a, tiles);
     return tb_last_error();

@@ -376,11 +376,9 @@ int tb_mlstm_parallel_bf16(const void* qkv, const float* gates, const float* bia
     const MlstmParallelArgs p{MlstmArgs{qkv, gates, bias, state, out, seq_start, slots, ld, H, dim, vdim, cap, qscale}, work, max_chunks};
     const size_t smem_u = (size_t)2 * MC_L * 128 * sizeof(float);
     const size_t smem_r = (size_t)MC_L * ((dim > MP_COLS ? dim : MP_COLS) + dim + 4 + MP_C) * sizeof(float);      // 147 KB for dim 256
-    static std::once_flag raised;
-    std::call_once(raised, [] {
-        tb_note_error(cudaFuncSetAttribute(mlstm_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-        tb_note_error(cudaFuncSetAttribute(mlstm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    });
+    static PerDevice raised[2];
+    tb_allow_smem(raised[0], (const void*)mlstm_update_kernel, 80 * 1024);
+    tb_allow_smem(raised[1], (const void*)mlstm_rows_kernel, 160 * 1024);
     const int col_blocks = (vdim + MP_COLS - 1) / MP_COLS, row_blocks = (dim + MP_ROWS - 1) / MP_ROWS;
     TB_LAUNCH(mlstm_gates_kernel, dim3(B, H), MP_THREADS, 0, s, p);
     TB_LAUNCH(mlstm_update_kernel, dim3(max_chunks, H * row_blocks, col_blocks), MP_THREADS, smem_u, s, p, B);
