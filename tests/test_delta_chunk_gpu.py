@@ -29,6 +29,36 @@ def _plain(x, conv, a, beta, G, H, dim, vdim):
     return torch.stack(out), S
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("dim", [64, 128])
+def test_what_is_no_number_stays_behind_its_token(dim, bad):
+    """One value channel of one token is no number: the outputs of the tokens before it, those of its own chunk among them, and
+    of the other channels keep their bits, as token by token."""
+    from transformer_b200.csrc import lib
+    gen = torch.Generator().manual_seed(dim)
+    n, H, vdim, at, channel = 50, 2, 32, 21, 5
+    C = 2 * H * dim + H * vdim
+    x, a, bz = torch.randn(n, C, generator=gen), torch.randn(n, H * dim, generator=gen).cuda(), torch.randn(n, H, generator=gen).cuda()
+    conv, bias, A_log = torch.randn(C, 4, generator=gen).cuda(), torch.randn(H * dim, generator=gen).cuda(), torch.rand(H, generator=gen).cuda()
+    starts, slots = torch.tensor([0, n], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    chunks, outs = n // 16 + 1, []
+    for value in (0.5, bad):
+        z = x.clone()
+        z[at, 2 * H * dim + channel] = value
+        z, state = z.cuda(), torch.zeros(1, lib.delta_state_size(H, H, dim, vdim, 4)).cuda()
+        rec = torch.empty(H, chunks, lib.delta_chunk_record_size(dim, vdim, 4)).cuda()
+        o = torch.full((n, H, vdim), 7.0, device="cuda")
+        where = (lib.ptr(starts), lib.ptr(slots), n, 1, H, H, dim, vdim, 4, chunks)
+        lib.call("tb_delta_chunk_f32", lib.ptr(z), C, lib.ptr(conv), lib.ptr(state), lib.ptr(a), lib.ptr(bias), lib.ptr(A_log), lib.ptr(bz),
+                 lib.ptr(rec), *where, H * dim, H, 0)
+        lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where)
+        outs.append(o.cpu())
+    good, got = outs
+    assert bool(torch.isfinite(good).all()) and not bool(torch.isfinite(got[at:, 0, channel]).any())
+    got[at:, 0, channel] = good[at:, 0, channel]
+    assert torch.equal(good, got)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("G,H,dim,vdim,per_head,steep", [(2, 4, 64, 48, False, 0.0), (1, 1, 128, 128, True, 0.0),
                                                          (2, 2, 128, 16, False, 6.0), (1, 2, 64, 256, False, -12.0)])

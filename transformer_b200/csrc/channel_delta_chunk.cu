@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
                 F2 mine, bd;
                 mine.f = my_col ? make_float2(u[C - 2], u[C - 1]) : make_float2(u[0], u[1]);
                 bd.f = make_float2(bj[e4], bj[e4]);
-                o = fma2(bd, mine, o);
+                // B is zero for later tokens, but a later token's u may be no number, and that is not this one's affair
+                if (j <= my_tok) o = fma2(bd, mine, o);
 #pragma unroll
                 for (int r = 0; r < R4; ++r) {
                     Four kd;
