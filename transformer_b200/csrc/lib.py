@@ -56,7 +56,7 @@ _SIGNATURES: Dict[str, str] = {
     "tb_moe_identity_rows_f32": "pppppiiii", "tb_moe_identity_rows_bf16": "pppppiiii",
     "tb_mlstm_scan_f32": "pppppppiiiiiff", "tb_mlstm_scan_bf16": "pppppppiiiiiff",
     "tb_mlstm_chunk_f32": "pppppppiiiiiff", "tb_mlstm_chunk_bf16": "pppppppiiiiiff",
-    "tb_mlstm_parallel_bf16": "ppppppppiiiiiiiff",
+    "tb_mlstm_parallel_bf16": "pppppppppiiiiiiiiff",
     "tb_mlstm_out_f32": "ppippiiifii", "tb_mlstm_out_bf16": "ppippiiifii",
     "tb_latent_prep_f32": "pippfpppppippiiiii", "tb_latent_prep_bf16": "pippfpppppippiiiii",
     "tb_latent_attention_mma_bf16": "ppppppppppppiiiiiiiiiiifppi",
@@ -130,7 +130,7 @@ class TapeMap(ctypes.Structure):
 
 _NO_STREAM = {"tb_decay_scan_rect_record_size": "ii", "tb_split_delta_record_size": "i",
               "tb_decay_state_size": "iii", "tb_decay_record_size": "i",
-              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
+              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_gates": "", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
               "tb_attention_tc_tile_tokens": ""}
 
 _lock = threading.Lock()
@@ -426,8 +426,13 @@ def mlstm_state_size(dim: int, vdim: int) -> int:
 
 
 def mlstm_parallel_size(heads: int, dim: int, vdim: int, ld: int) -> int:
-    """Floats of scratch per (head, chunk) of the matrix memory's prompt kernels; 0: they do not take such heads."""
+    """Floats of scratch per (head, chunk of a portion) of the matrix memory's prompt kernels; 0: they do not take such heads."""
     return library().tb_mlstm_parallel_size(heads, dim, vdim, ld)
+
+
+def mlstm_parallel_gates() -> int:
+    """Floats of scratch per (head, chunk of the step) that those kernels want beside it."""
+    return library().tb_mlstm_parallel_gates()
 
 
 def mlstm_parallel_tokens() -> int:

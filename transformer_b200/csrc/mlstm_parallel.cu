@@ -7,6 +7,8 @@
 //   mlstm_update_kernel    a block = a chunk x a head x 128 rows x 128 columns: U = sum_j w_j k_j v_j^T (and n's alike)
 //   mlstm_state_kernel     a thread = four entries of S: walks the chunks, leaves the state before each where U was
 //   mlstm_rows_kernel      a block = a chunk x a head x 128 columns: scores, denominators, outputs
+// A state per chunk is a lot of memory (8 heads of 128 x 256: 1 MB), so the last three take a portion of the chunks at a time, as
+// many as the caller's scratch holds.
 // 154 us for the 2,039 tokens.  Every sum is taken in the order of mlstm_chunk_kernel: the results are the same bit for bit.  Float throughout; the
 // products are bound by multiply-adds on the CUDA cores with their operands in shared memory, 16 x 4 and 8 x 4 results a
 // thread so that a 16-byte read feeds 13 and 11 of them.
@@ -20,11 +22,13 @@
 
 struct MlstmParallelArgs {
     MlstmArgs a;
-    float* work;                // [H][max_chunks][mp_record]: gates | n's sum [dim] | U, then the state before [dim][vdim]
-    int max_chunks;
+    float* gates;               // [H][max_chunks][MP_GATES]
+    float* work;                // [H][portion][mp_record]: n's sum [dim] | U, then the state before [dim][vdim]
+    int max_chunks, portion;
+    int base;                   // the portion's first chunk
 };
 
-__host__ __device__ inline size_t mp_record(int dim, int vdim) { return MP_GATES + dim + (size_t)dim * vdim; }
+__host__ __device__ inline size_t mp_record(int dim, int vdim) { return dim + (size_t)dim * vdim; }
 
 // The sequence of chunk `chunk` of the step (counted over its sequences), or -1; `chunk` becomes its own number there.
 __device__ __forceinline__ int mp_find(const int* seq_start, int B, int& chunk, int& t0, int& n) {
@@ -54,14 +58,13 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_gates_kernel(const MlstmPara
     int first = 0;
     for (int i = 0; i < b; ++i) first += (a.seq_start[i + 1] - a.seq_start[i] + MC_L - 1) / MC_L;
     const int chunks = (len + MC_L - 1) / MC_L;
-    const size_t rec = mp_record(a.dim, a.vdim);
     float* n0 = a.state + ((size_t)a.slots[b] * a.H + h) * mp_state_size(a.dim, a.vdim) + (size_t)a.dim * a.vdim;
     const float bi = a.bias[h], bf = a.bias[a.H + h], cap = a.cap, inv_cap = 1.0f / a.cap;
     float m_prev = n0[a.dim];
     for (int base = 0; base < chunks; base += MP_THREADS) {
         const int here = min(MP_THREADS, chunks - base);
         for (int c = warp; c < here; c += MP_THREADS / 32) {
-            float* w = p.work + ((size_t)h * p.max_chunks + first + base + c) * rec;
+            float* w = p.gates + ((size_t)h * p.max_chunks + first + base + c) * MP_GATES;
             const int c0 = t0 + (base + c) * MC_L, nc = min(MC_L, len - (base + c) * MC_L);
             float fg[2], ig[2];
 #pragma unroll
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_gates_kernel(const MlstmPara
         __syncthreads();
         m_prev = mp_s[here];
         for (int c = warp; c < here; c += MP_THREADS / 32) {
-            float* w = p.work + ((size_t)h * p.max_chunks + first + base + c) * rec;
+            float* w = p.gates + ((size_t)h * p.max_chunks + first + base + c) * MP_GATES;
             const float mp = mp_s[c], bL = bL_s[c], mL = mp_s[c + 1];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {       // what this lane wrote above
@@ -141,10 +144,11 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_update_kernel(const MlstmPar
     __shared__ float w_s[MC_L];
     const int row_blocks = (a.dim + MP_ROWS - 1) / MP_ROWS;
     const int h = blockIdx.y / row_blocks, r0 = blockIdx.y % row_blocks * MP_ROWS, col0 = blockIdx.z * MP_COLS;
-    int chunk = blockIdx.x, t0, n;
+    int chunk = p.base + blockIdx.x, t0, n;
     if (mp_find(a.seq_start, B, chunk, t0, n) < 0) return;
-    float* w = p.work + ((size_t)h * p.max_chunks + blockIdx.x) * mp_record(a.dim, a.vdim);
-    if (threadIdx.x < MC_L) w_s[threadIdx.x] = w[4 * MC_L + threadIdx.x];
+    const float* gates = p.gates + ((size_t)h * p.max_chunks + p.base + blockIdx.x) * MP_GATES;
+    float* w = p.work + ((size_t)h * p.portion + blockIdx.x) * mp_record(a.dim, a.vdim);
+    if (threadIdx.x < MC_L) w_s[threadIdx.x] = gates[4 * MC_L + threadIdx.x];
     const int rows = min(MP_ROWS, a.dim - r0), cols = min(MP_COLS, a.vdim - col0);
     mp_load(a, t0, n, (size_t)(a.H + h) * a.dim + r0, rows, MP_ROWS, 1.f, false, k_s);
     mp_load(a, t0, n, (size_t)2 * a.H * a.dim + (size_t)h * a.vdim + col0, cols, MP_COLS, 1.f, false, v_s);
@@ -170,7 +174,7 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_update_kernel(const MlstmPar
                 }
             }
         }
-        float* U = w + MP_GATES + a.dim;
+        float* U = w + a.dim;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
             if (warp * 16 + i < rows)
@@ -180,11 +184,12 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_update_kernel(const MlstmPar
     if (blockIdx.z == 0 && threadIdx.x < rows) {
         float acc = 0.f;
         for (int j = 0; j < MC_L; ++j) acc += w_s[j] * k_s[j * MP_ROWS + threadIdx.x];
-        w[MP_GATES + r0 + threadIdx.x] = acc;
+        w[r0 + threadIdx.x] = acc;
     }
 }
 
-// Entries of (n, S) four at a time: n's sums lie right before U in a chunk's record.  Loads run four chunks ahead.
+// Entries of (n, S) four at a time: n's sums lie right before U in a chunk's record.  Loads run four chunks ahead.  A sequence that
+// goes on in the next portion leaves its state where that portion finds it: in the cache.
 __global__ void __launch_bounds__(MP_THREADS) mlstm_state_kernel(const MlstmParallelArgs p) {
     pdl_sync();
     const MlstmArgs& a = p.a;
@@ -194,10 +199,13 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_state_kernel(const MlstmPara
     if (len <= 0 || at >= dim + dim * vdim) return;
     int first = 0;
     for (int i = 0; i < b; ++i) first += (a.seq_start[i + 1] - a.seq_start[i] + MC_L - 1) / MC_L;
-    const int chunks = (len + MC_L - 1) / MC_L;
+    // its chunks in this portion, counted from the portion's first
+    const int lo = max(first, p.base) - p.base, chunks = min(first + (len + MC_L - 1) / MC_L, p.base + p.portion) - p.base - lo;
+    if (chunks <= 0) return;
     const size_t rec = mp_record(dim, vdim);
     float* S = a.state + ((size_t)a.slots[b] * a.H + h) * mp_state_size(dim, vdim);
-    float* w = p.work + ((size_t)h * p.max_chunks + first) * rec;
+    float* w = p.work + ((size_t)h * p.portion + lo) * rec;
+    const float* gates = p.gates + ((size_t)h * p.max_chunks + p.base + lo) * MP_GATES;
     const bool is_n = at < dim;                 // dim is a multiple of four
     float s[4];
 #pragma unroll
@@ -208,13 +216,13 @@ __global__ void __launch_bounds__(MP_THREADS) mlstm_state_kernel(const MlstmPara
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (c0 + i < chunks) {
-                u[i] = *reinterpret_cast<const float4*>(w + (c0 + i) * rec + MP_GATES + at);
-                G[i] = w[(c0 + i) * rec + 5 * MC_L];
+                u[i] = *reinterpret_cast<const float4*>(w + (c0 + i) * rec + at);
+                G[i] = gates[(c0 + i) * MP_GATES + 5 * MC_L];
             }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (c0 + i < chunks) {
-                *reinterpret_cast<float4*>(w + (c0 + i) * rec + MP_GATES + at) = make_float4(s[0], s[1], s[2], s[3]);
+                *reinterpret_cast<float4*>(w + (c0 + i) * rec + at) = make_float4(s[0], s[1], s[2], s[3]);
                 s[0] = G[i] * s[0] + u[i].x;
                 s[1] = G[i] * s[1] + u[i].y;
                 s[2] = G[i] * s[2] + u[i].z;
@@ -242,11 +250,12 @@ __global__ void __launch_bounds__(MP_THREADS, 2) mlstm_rows_kernel(const MlstmPa
     __shared__ float gate[5 * MC_L], den_s[MC_L];
     __shared__ float n_s[256];
     const int h = blockIdx.y, col0 = blockIdx.z * MP_COLS, tid = threadIdx.x;
-    int chunk = blockIdx.x, t0, n;
+    int chunk = p.base + blockIdx.x, t0, n;
     if (mp_find(a.seq_start, B, chunk, t0, n) < 0) return;
-    const float* w = p.work + ((size_t)h * p.max_chunks + blockIdx.x) * mp_record(dim, vdim);
-    for (int i = tid; i < 5 * MC_L; i += MP_THREADS) gate[i] = w[i];
-    if (tid < dim) n_s[tid] = w[MP_GATES + tid];
+    const float* gates = p.gates + ((size_t)h * p.max_chunks + p.base + blockIdx.x) * MP_GATES;
+    const float* w = p.work + ((size_t)h * p.portion + blockIdx.x) * mp_record(dim, vdim);
+    for (int i = tid; i < 5 * MC_L; i += MP_THREADS) gate[i] = gates[i];
+    if (tid < dim) n_s[tid] = w[tid];
     const float *b_s = gate, *ig_s = gate + MC_L, *m_s = gate + 2 * MC_L, *g_s = gate + 3 * MC_L;
     mp_load(a, t0, n, (size_t)h * dim, dim, dim, a.qscale, true, q_s);
     mp_load(a, t0, n, (size_t)(H + h) * dim, dim, kp, 1.f, false, k_s);
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(MP_THREADS, 2) mlstm_rows_kernel(const MlstmPa
     const int cols = min(MP_COLS, vdim - col0), lane = tid & 31, warp = tid >> 5, half = dim / 2;
     float* S_s = k_s;                   // [dim / 2][128]: fits 64 x (dim + 4)
     auto load_state = [&](int r0) {
-        const float* S = w + MP_GATES + dim + (size_t)r0 * vdim + col0;
+        const float* S = w + dim + (size_t)r0 * vdim + col0;
         for (int idx = tid; idx < half * (MP_COLS / 4); idx += MP_THREADS) {
             const int r = idx / (MP_COLS / 4), c = idx % (MP_COLS / 4) * 4;
             if (c < cols) *reinterpret_cast<float4*>(S_s + r * MP_COLS + c) = *reinterpret_cast<const float4*>(S + (size_t)r * vdim + c);
@@ -359,21 +368,25 @@ static bool mlstm_parallel_takes(int H, int dim, int vdim, int ld) {
 }
 
 extern "C" {
-// Floats of scratch per (head, chunk of 64 tokens), or 0 where these kernels do not take such heads and rows.
+// Floats of scratch per (head, chunk of 64 tokens of a portion), or 0 where these kernels do not take such heads and rows, and
+// per (head, chunk of the step).
 int tb_mlstm_parallel_size(int H, int dim, int vdim, int ld) {
     return mlstm_parallel_takes(H, dim, vdim, ld) ? (int)mp_record(dim, vdim) : 0;
 }
+int tb_mlstm_parallel_gates() { return MP_GATES; }
 int tb_mlstm_parallel_tokens() { return MC_L; }
 
-// As tb_mlstm_chunk_bf16; work [H][max_chunks][tb_mlstm_parallel_size], max_chunks >= nt / 64 + B.
+// As tb_mlstm_chunk_bf16; gate_work [H][max_chunks][tb_mlstm_parallel_gates], max_chunks >= nt / 64 + B; work
+// [H][portion][tb_mlstm_parallel_size].
 int tb_mlstm_parallel_bf16(const void* qkv, const float* gates, const float* bias, float* state, float* out, float* work,
-                           const int* seq_start, const int* slots, int nt, int B, int ld, int H, int dim, int vdim,
-                           int max_chunks, float cap, float qscale, cudaStream_t s) {
-    if (nt < 0 || B < 0 || H <= 0 || dim <= 0 || vdim <= 0 || max_chunks < 0 || !(cap > 0.f)) return TB_ERR_ARG;
+                           float* gate_work, const int* seq_start, const int* slots, int nt, int B, int ld, int H, int dim,
+                           int vdim, int max_chunks, int portion, float cap, float qscale, cudaStream_t s) {
+    if (nt < 0 || B < 0 || H <= 0 || dim <= 0 || vdim <= 0 || max_chunks < 0 || portion < 1 || !(cap > 0.f)) return TB_ERR_ARG;
     if (!mlstm_parallel_takes(H, dim, vdim, ld) || (((uintptr_t)qkv | (uintptr_t)work | (uintptr_t)out) & 15)) return TB_ERR_UNSUPPORTED;
     if (nt == 0 || B == 0) return 0;
     if (max_chunks < nt / MC_L + (B < nt ? B : nt)) return TB_ERR_ARG;
-    const MlstmParallelArgs p{MlstmArgs{qkv, gates, bias, state, out, seq_start, slots, ld, H, dim, vdim, cap, qscale}, work, max_chunks};
+    MlstmParallelArgs p{MlstmArgs{qkv, gates, bias, state, out, seq_start, slots, ld, H, dim, vdim, cap, qscale}, gate_work, work,
+                        max_chunks, portion, 0};
     const size_t smem_u = (size_t)2 * MC_L * 128 * sizeof(float);
     const size_t smem_r = (size_t)MC_L * ((dim > MP_COLS ? dim : MP_COLS) + dim + 4 + MP_C) * sizeof(float);      // 147 KB for dim 256
     static PerDevice raised[2];
@@ -381,9 +394,12 @@ int tb_mlstm_parallel_bf16(const void* qkv, const float* gates, const float* bia
     tb_allow_smem(raised[1], (const void*)mlstm_rows_kernel, 160 * 1024);
     const int col_blocks = (vdim + MP_COLS - 1) / MP_COLS, row_blocks = (dim + MP_ROWS - 1) / MP_ROWS;
     TB_LAUNCH(mlstm_gates_kernel, dim3(B, H), MP_THREADS, 0, s, p);
-    TB_LAUNCH(mlstm_update_kernel, dim3(max_chunks, H * row_blocks, col_blocks), MP_THREADS, smem_u, s, p, B);
-    TB_LAUNCH(mlstm_state_kernel, dim3(B, H, (dim + dim * vdim + 4 * MP_THREADS - 1) / (4 * MP_THREADS)), MP_THREADS, 0, s, p);
-    TB_LAUNCH(mlstm_rows_kernel, dim3(max_chunks, H, col_blocks), MP_THREADS, smem_r, s, p, B);
+    for (; p.base < max_chunks; p.base += portion) {
+        const int count = max_chunks - p.base < portion ? max_chunks - p.base : portion;
+        TB_LAUNCH(mlstm_update_kernel, dim3(count, H * row_blocks, col_blocks), MP_THREADS, smem_u, s, p, B);
+        TB_LAUNCH(mlstm_state_kernel, dim3(B, H, (dim + dim * vdim + 4 * MP_THREADS - 1) / (4 * MP_THREADS)), MP_THREADS, 0, s, p);
+        TB_LAUNCH(mlstm_rows_kernel, dim3(count, H, col_blocks), MP_THREADS, smem_r, s, p, B);
+    }
     return tb_last_error();
 }
 }

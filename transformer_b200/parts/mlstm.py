@@ -26,6 +26,9 @@ USE_CHUNKS = True      # prompts: the kernel that takes 64 tokens at a time
 # Tokens a sequence (on average) from which its chunks are done side by side: four launches against 22 us a chunk of 64 tokens
 # (8 heads of 128 x 256, us: 1 x 128 tokens 62 and 49, 1 x 192 67 and 71, 1 x 300 71 and 114, 1 x 2,039 154 and 699)
 PARALLEL_TOKENS = 192
+# ... and the most scratch that their states may take, one per chunk (8 heads of 128 x 256: 8 MB a chunk over the heads): steps of
+# more chunks are done in portions
+PARALLEL_BYTES = 256 << 20
 
 
 @MIXERS.register("mlstm")
@@ -74,10 +77,12 @@ class MatrixMemory(Mixer):
             per = lib.mlstm_parallel_size(H, self.dim, self.vdim, self.z_width)
             if per:
                 chunks = nt // lib.mlstm_parallel_tokens() + ctx.B
-                work = ctx.scratch("mlstm.work", (H, chunks, per), torch.float32)
+                portion = max(1, min(chunks, PARALLEL_BYTES // (4 * H * per)))
+                work = ctx.scratch("mlstm.work", (H, portion, per), torch.float32)
+                gate_work = ctx.scratch("mlstm.gate_work", (H, chunks, lib.mlstm_parallel_gates()), torch.float32)
         if work is not None:       # long prompts: the chunks of a sequence side by side
             lib.call("tb_mlstm_parallel_" + sfx, lib.ptr(z), lib.ptr(gates), lib.ptr(w["bif"]), lib.ptr(state), lib.ptr(o),
-                     lib.ptr(work), *where, nt, ctx.B, *sizes, chunks, self.cap, self.dim ** -0.5)
+                     lib.ptr(work), lib.ptr(gate_work), *where, nt, ctx.B, *sizes, chunks, portion, self.cap, self.dim ** -0.5)
         else:
             # short ones: 64 tokens of a sequence side by side; decoding: token by token, the state in registers
             kernel = "tb_mlstm_scan_" if ctx.decode or not USE_CHUNKS else "tb_mlstm_chunk_"
