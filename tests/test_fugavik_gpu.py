@@ -585,3 +585,48 @@ def test_squared_relu_in_the_products_epilogue():
         assert gemm_skinny(d_a, d_w, out, out_kind=3)
         torch.cuda.synchronize()
         assert float((out.cpu().double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+
+
+# ---- the delta rule 16 tokens at a time (steps of more than parts.channel_delta.CHUNK_MEAN tokens a sequence), in the model -----
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("cuts,most", [([330, 60, 70], 8192), ([60, 345, 40], 8192), ([460], 350), ([2, 321, 137], 8192)])
+def test_long_and_short_portions_share_the_state(cuts, most, dtype, folders):
+    """Portions above and below the line, in both orders and as pieces of one step, then six tokens decoded: the chunk form, the
+    token form and the decode step hand one state and one convolution's inputs to each other."""
+    cfg, tensors = FP.read_folder(folders["wide"])
+    tokens = _tokens(folders["wide"], 466, 31)
+    rows, routes = T.run_cuts(_load(folders["wide"], dtype, max_step_tokens=most), tokens, cuts)
+    T.check_request(cfg, tensors, tokens, rows, dtype, f"cuts {cuts}", routes)
+
+
+def test_unequal_sequences_in_one_step_of_chunks(folders, monkeypatch, dtype="float32"):
+    """Sequences of 1 to 130 tokens side by side in the chunk form (the line lowered), against the plain implementation (in
+    bfloat16 a token may choose another expert; the chunk form itself is held to 64 bits in test_delta_chunk_gpu.py)."""
+    from transformer_b200.parts import channel_delta
+    monkeypatch.setattr(channel_delta, "CHUNK_MEAN", 10)
+    cfg, tensors = FP.read_folder(folders["wide"])
+    engine = _load(folders["wide"], dtype)
+    lens = [17, 1, 130, 16, 50]
+    seqs = [_tokens(folders["wide"], n + 1, 50 + i) for i, n in enumerate(lens)]
+    slots = [engine.open() for _ in seqs]
+    first = engine.step(slots, [s[:-1] for s in seqs], [list(range(n)) for n in lens]).cpu().split(lens)
+    last = engine.step(slots, [s[-1:] for s in seqs]).cpu()
+    engine.check_kernels()
+    for i, seq in enumerate(seqs):
+        rows = dict(enumerate(first[i]))
+        rows[lens[i]] = last[i]
+        T.check_request(cfg, tensors, seq, rows, dtype, f"sequence {i}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_replayed_layers_of_chunks(dtype):
+    """Equal layers are recorded once and replayed with their own weights and state: the same bits as each run from Python."""
+    import transformer_b200 as tb
+    cfg = T.config(128, 128, [(T.delta(2, 1, 64, 64, 4), T.dense(96))] * 3)
+    prompt, got = random_prompts(128, [400], 3)[0], []
+    for tapes in (True, False):
+        engine = tb.random_model(cfg, seed=4, dtype=dtype, max_tokens=1024, std=0.1)
+        engine.use_tapes = tapes
+        slot = engine.open()
+        got.append(torch.cat([engine.step([slot], [prompt[:390]], [list(range(390))]), engine.step([slot], [prompt[390:]])]).clone())
+    assert torch.equal(*got)

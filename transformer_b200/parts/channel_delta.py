@@ -28,6 +28,15 @@ from .base import MIXERS, Mixer, ParamDecl, StateNeed
 from .linear import matmul_nt
 
 
+# A step of more tokens than this a sequence, on average, takes 16 tokens at a time (csrc/channel_delta_chunk.cu), where that
+# kernel takes the heads.  It is the faster form from some 20 tokens a sequence on (16 heads of 128, both kernels, us: 16 x 8
+# tokens 65 there and 63 token by token, 1 x 64 32 and 46, 8 x 70 91 and 145, 1 x 320 a tenth of a millisecond apart, 1 x 2,048
+# 294 and 812); the line is kept where it is because the forms round differently (both in float: 1e-5 of the largest value
+# from the 64-bit recurrence) and a request's short prompts keep the bits they had.  The average is the step's: which form a
+# prompt takes, and so its last bits, depends on the sequences that share its step and on where a step is cut.
+CHUNK_MEAN = 320
+
+
 @MIXERS.register("channel_delta")
 class ChannelDelta(Mixer):
     """params: width, heads, kv_heads, dim, vdim, taps, decay_rank, gate_rank, eps; optional: decay ("channel" |
@@ -115,12 +124,9 @@ class ChannelDelta(Mixer):
         o = ctx.scratch("delta.o", (nt, self.hv), torch.float32)
         where = (lib.ptr(ctx.seq_start), lib.ptr(ctx.slots), nt, ctx.B, self.G, H, self.dim, self.vdim, self.taps)
         per_head = 1 if self.decay == "head" else 0
-        # long prompts: 16 tokens at a time (csrc/channel_delta_chunk.cu).  It is the faster form from some 20 tokens a
-        # sequence on (16 heads of 128, both kernels: 16 x 8 tokens 65 us here and 63 token by token, 1 x 64 32 and 46,
-        # 8 x 70 91 and 145), but its sums round differently, so it begins where the gain is worth that: at 320 tokens
-        # the two differ by a tenth of a millisecond a layer, at 2,048 by half a millisecond
+        # long prompts: 16 tokens at a time (csrc/channel_delta_chunk.cu)
         per_chunk = lib.delta_chunk_record_size(self.dim, self.vdim, self.taps)
-        if per_chunk and nt > 320 * ctx.B and self.z_width % 2 == 0:
+        if per_chunk and nt > CHUNK_MEAN * ctx.B and self.z_width % 2 == 0:
             chunks = nt // lib.delta_chunk_tokens() + ctx.B
             rec = ctx.scratch("delta.rec", (H, chunks, per_chunk), torch.float32)
             lib.call("tb_delta_chunk_" + sfx, lib.ptr(z), self.z_width, lib.ptr(w["conv"]), lib.ptr(state), lib.ptr(a),
