@@ -1,6 +1,6 @@
 """Latent attention with 64 rows a block against the kernel with 16: the same sums in the same order, so the same bits.
 
-The launcher takes the first from some hundred query tiles on; called with fewer at a time it is the second.  Sequences that
+Sequences that
 share a block, tiles that do not fill the last one, windows that begin and end inside a page, heads that do not fill a tile, ranks and rotated parts
 with an odd number of k-steps."""
 import pytest
@@ -9,8 +9,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("H,rank,rot,window", [(16, 512, 64, 1 << 30), (8, 256, 32, 100), (20, 128, 16, 64), (3, 256, 0, 200),
-                                               (16, 512, 48, 70), (16, 128, 64, 1 << 30)])
+@pytest.mark.parametrize("H,rank,rot,window", [(16, 512, 64, 1 << 30), (8, 256, 32, 100), (20, 256, 16, 64), (3, 256, 0, 200),
+                                               (16, 512, 48, 70), (16, 256, 64, 1 << 30)])
 def test_same_bits(H, rank, rot, window):
     from transformer_b200.csrc import lib
     g = torch.Generator().manual_seed(rank + rot)
@@ -35,18 +35,19 @@ def test_same_bits(H, rank, rot, window):
         at += n
     seq, t0, nq, pos = I(seq), I(t0), I(nq), I(pos)
 
-    def run(step):
+    def run(name, step):
         out = torch.full((nt, H, rank), 7.0, dtype=torch.bfloat16, device="cuda")
+        partial, splits = ((), ()) if name == "rows" else ((0,), (1,))
         for i in range(0, len(t0), step):
             n = min(step, len(t0) - i)
-            assert lib.try_call("tb_latent_attention_mma_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(out), 0, lib.ptr(cache),
+            assert lib.try_call(f"tb_latent_attention_{name}_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(out), *partial, lib.ptr(cache),
                                 lib.ptr(seq[i:]), lib.ptr(t0[i:]), lib.ptr(nq[i:]), lib.ptr(pos), lib.ptr(table), lib.ptr(cos),
-                                lib.ptr(sin), n, nt, max_pages, H * q_head, q_head, H, rank, rot, rot, window, 1,
+                                lib.ptr(sin), n, nt, max_pages, H * q_head, q_head, H, rank, rot, rot, window, *splits,
                                 (16 + rot) ** -0.5, lib.ptr(sinks), lib.ptr(gate), H)
         torch.cuda.synchronize()
         return out
 
-    want = run(150)
+    want = run("mma", len(t0))
     assert bool(torch.isfinite(want).all()) and float(want.abs().mean()) > 1e-3
-    for step in (len(t0), len(t0) - 1, len(t0) - 3):
-        assert torch.equal(run(step), want)
+    for step in (len(t0), len(t0) - 1, len(t0) - 3, 5):
+        assert torch.equal(run("rows", step), want)

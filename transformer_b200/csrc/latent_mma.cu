@@ -659,14 +659,6 @@ int tb_latent_attention_mma_bf16(const void* qa, const void* q, void* out, float
                         2 * LM_ROWS * 4 + LM_ROWS * 4;
     if (smem > 120 * 1024) return TB_ERR_UNSUPPORTED;
     int rc;
-    // The rows kernel (its shared memory must fit an SM) for prompts of so many 16-row tiles that its quarter as many blocks
-    // still pay (us, here and with 16 rows a block).  Rank 512 + 64, 16 heads: 300 tiles 52 and 44, 450 66 and 71, 600 85 and
-    // 101, 1,100 148 and 252, 2,039 439 and 720; rank 256 + 32, 8 heads: 450 78 and 63, 600 101 and 93, 800 129 and 139,
-    // 1,020 161 and 205
-    const int all_tiles = tiles * ((H + hc - 1) / hc);
-    if (splits == 1 && all_tiles >= (rank == 512 ? 400 : 700) && (rank == 128 || rank == 256 || rank == 512) && latent_rows_smem(DK) <= 227 * 1024)
-        return rank == 512 ? latent_rows_go<8>(a, tiles, s) : rank == 256 ? latent_rows_go<4>(a, tiles, s)
-                                                                          : latent_rows_go<2>(a, tiles, s);
     if (rank % 64 == 0) {               // eight warps: rank / 8 columns of the output each
         const int nt8 = rank / 8 / 8;
         if (nt8 <= 2) rc = latent_mma_go<2, 8>(a, tiles, smem, s);
@@ -684,7 +676,28 @@ int tb_latent_attention_mma_bf16(const void* qa, const void* q, void* out, float
               (const __nv_bfloat16*)gate, ldg, H);
     return tb_last_error();
 }
+// The same without slices, 64 rows a block (latent_rows_kernel): the same bits, faster or slower by what the step brings (see
+// parts/latent_attention.py).  TB_ERR_UNSUPPORTED for sizes it does not take.
+int tb_latent_attention_rows_bf16(const void* qa, const void* q, void* out, const void* cache, const int* tile_seq,
+                                  const int* tile_t0, const int* tile_nq, const int* tok_pos, const int* page_table,
+                                  const float* cosT, const float* sinT, int tiles, int nt, int max_pages, int ldq, int q_head,
+                                  int H, int rank, int rot, int rdims, int window, float scale, const float* sinks,
+                                  const void* gate, int ldg, cudaStream_t s) {
+    if (tiles < 0 || nt < 0 || H <= 0 || rank <= 0 || rot < 0 || window <= 0 || rdims < 0 || rdims > rot || rdims % 2)
+        return TB_ERR_ARG;
+    if ((rank != 256 && rank != 512) || (rank + rot) % 16 || latent_rows_smem(rank + rot) > 227 * 1024 ||
+        ((((uintptr_t)cache) | ((uintptr_t)qa)) & 15))
+        return TB_ERR_UNSUPPORTED;
+    if (tiles == 0) return 0;
+    const int hc = H < LM_ROWS ? H : LM_ROWS;
+    const LatentMmaArgs a{(const __nv_bfloat16*)qa, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, nullptr,
+                          (const __nv_bfloat16*)cache, tile_seq, tile_t0, tile_nq, tok_pos, page_table, cosT, sinT, max_pages,
+                          ldq, q_head, q_head - rot, H, rank, rot, rdims, window, hc, LM_ROWS / hc, 1, scale, sinks,
+                          (const __nv_bfloat16*)gate, ldg};
+    return rank == 512 ? latent_rows_go<8>(a, tiles, s) : latent_rows_go<4>(a, tiles, s);
+}
 }
 
 #include "tape.h"
 TB_TAPE_REGISTER(tb_latent_attention_mma_bf16)
+TB_TAPE_REGISTER(tb_latent_attention_rows_bf16)

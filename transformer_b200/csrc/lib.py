@@ -60,6 +60,7 @@ _SIGNATURES: Dict[str, str] = {
     "tb_mlstm_out_f32": "ppippiiifii", "tb_mlstm_out_bf16": "ppippiiifii",
     "tb_latent_prep_f32": "pippfpppppippiiiii", "tb_latent_prep_bf16": "pippfpppppippiiiii",
     "tb_latent_attention_mma_bf16": "ppppppppppppiiiiiiiiiiifppi",
+    "tb_latent_attention_rows_bf16": "pppppppppppiiiiiiiiiifppi",
     "tb_latent_attention_f32": "pppppppppppiiiiiiiiiifppi", "tb_latent_attention_bf16": "pppppppppppiiiiiiiiiifppi",
     "tb_embed_bigram_f32": "pppppppppiifiii", "tb_embed_bigram_bf16": "pppppppppiifiii",
     "tb_scale_f32": "plf",

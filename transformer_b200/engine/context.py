@@ -154,6 +154,7 @@ class StepContext:
         self._offsets = offsets
         self._views: Dict[str, torch.Tensor] = {}       # made once per step: every layer asks for the same ones
         self._scratch: Dict[tuple, torch.Tensor] = {}
+        self.plans: Dict[tuple, object] = {}            # what parts have worked out on the host for this step
         self.run_index = -1     # which entry of the run order is executing
 
     def _view(self, name: str) -> torch.Tensor:

@@ -33,6 +33,35 @@ from .spec import PartSpec
 
 USE_TENSOR_CORES = True    # bfloat16: the mma.sync kernel before the general one
 
+# 64 rows of one sequence that share a page (csrc/latent_mma.cu, latent_rows_kernel) against 16: for ranks of 256 and 512,
+# (blocks of 16 rows from which it is looked at, the cost of 64 rows in that of 16, the part of a block that a sequence leaves empty,
+# keys' worth of a block's start and end).  With T tiles of 16 rows that see K keys each on average, 64 rows a block cost about
+# cost * (T / 4 + part) * (K + edge), 16 rows T * K; over the step's sequences the smaller sum wins.  Chosen so that of 71 and 63 steps
+# measured no one is slower (us, 64 rows a block and 16; rank 512 + 64, 16 heads): one prompt of 2,039 tokens 439 and 722, 4 of 300 88
+# and 106, 8 of 128 behind 500 cached 163 and 227, a window of 256 415 and 478, of 128 327 and 335; not taken: 16 prompts of 100 85 and
+# 82, 200 of 6 77 and 54, 420 sequences of one token behind 2,000 cached 778 and 356.  Rank 256 + 32, 8 heads: 2,039 tokens 159 and 203; not
+# taken: 8 of 200 48 and 34, a window of 512 of 4,096 tokens 209 and 180.  Rank 128 gained 10 % at best and lost up to a factor of four.
+SHARED_ROWS = {512: (400, 2.1, 0.5, 96), 256: (700, 3.0, 0.75, 256)}
+
+
+def keys_seen(n: int, before: int, window: int) -> int:
+    """Keys that the n tokens behind ``before`` cached ones see together: min(window, position + 1) each."""
+    growing = max(0, min(n, window - before))
+    return growing * before + growing * (growing + 1) // 2 + (n - growing) * window
+
+
+def rows_pay(lens, before, window: int, tile: int, rank: int, blocks: int) -> bool:
+    """Whether a step of such sequences (new tokens, cached ones) is faster with 64 rows a block."""
+    if rank not in SHARED_ROWS or blocks < SHARED_ROWS[rank][0]:
+        return False
+    _, cost, part, edge = SHARED_ROWS[rank]
+    shared = alone = 0.0
+    for n, b in zip(lens, before):
+        tiles, keys = -(-n // tile), keys_seen(n, b, window) / n
+        shared += cost * (tiles / 4 + part) * (keys + edge)
+        alone += tiles * keys
+    return shared < alone
+
 
 @MIXERS.register("latent_attention")
 class LatentAttention(Mixer):
@@ -169,7 +198,16 @@ class LatentAttention(Mixer):
             splits = int(max(1, min(16, (min(self.window, ctx.engine.spec.max_context) + 63) // 64 + 1,
                                     (2 * ctx.engine.sm_count) // max(1, blocks))))
             partial = ctx.scratch("latent.partial", (nt, H, splits, self.rank + 2), torch.float32) if splits > 1 else None
-            done = lib.try_call("tb_latent_attention_mma_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(ol), lib.ptr(partial),
+            plan = ("latent", self.window, self.tile, self.rank, blocks)
+            if splits == 1 and not ctx.decode and plan not in ctx.plans:
+                ctx.plans[plan] = rows_pay(ctx.h_lens, ctx.h_pos0, *plan[1:])
+            if splits == 1 and ctx.plans.get(plan):
+                done = lib.try_call("tb_latent_attention_rows_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(ol), lib.ptr(cache.kv),
+                                    lib.ptr(tiles.seq), lib.ptr(tiles.t0), lib.ptr(tiles.nq), lib.ptr(ctx.tok_pos),
+                                    lib.ptr(table), lib.ptr(cos), lib.ptr(sin), tiles.count, nt, ctx.max_pages, ldq,
+                                    self.q_head, H, self.rank, self.rot, self.rdims, self.window, self.scale,
+                                    lib.ptr(sinks), lib.ptr(gate), wa)
+            done = done or lib.try_call("tb_latent_attention_mma_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(ol), lib.ptr(partial),
                                 lib.ptr(cache.kv), lib.ptr(tiles.seq), lib.ptr(tiles.t0), lib.ptr(tiles.nq),
                                 lib.ptr(ctx.tok_pos), lib.ptr(table), lib.ptr(cos), lib.ptr(sin), tiles.count, nt,
                                 ctx.max_pages, ldq, self.q_head, H, self.rank, self.rot, self.rdims,
