@@ -49,9 +49,10 @@ struct SkinnyArgs {
     const int* row_group;   // [M] group of every row, rows in any order (instead of group_offsets and x_rows), or null
     int x_div;              // with row_group: row m reads X[m / x_div] and writes Y[m]
     int w_constant;         // W is a weight: nothing the kernel before this one may have written
-    // With row_group and at most half as many rows as groups: a block column per ROW (the first of its group does the group's)
-    // instead of one per group, most of which would be launched to find no row (a step of one sequence, 4 of 16 experts:
-    // 2,106 to 2,039 us in 32 layers).
+    // With row_group, 16 groups or more and at most a quarter as many rows, up to 16: a block column per ROW (the first of its group
+    // does the group's) instead of one per group, most of which would be launched to find no row.  A step of one sequence, 4 of 16
+    // experts: 2,106 to 2,039 us in 32 layers; alone, 128 pairs of 704 x 2,048: 1 row 13.5 to 4.4 us, 16 rows 25.4 to 20.0.  A block
+    // looks at the rows before its own one by one, so with more rows it turns: 32 rows 35.4 to 37.8, 64 51 to 69.
     int by_row;
     GluRule glu;            // DUAL: how the (gate, up) pair becomes one value
 };
@@ -276,10 +277,13 @@ static int skinny_launch_shape(const SkinnyArgs& a, cudaStream_t s) {
     // long rows: all 8 warps of a block share 16 columns and split K;
     // short rows (an expert's down projection): 2 warps on K
     //
-    // How many k-steps a thread loads before it multiplies (the order of the sums does not depend on it): where the blocks of
-    // a dense product fit the SMs at once, all of a warp's, so that a block that has waited for the kernel before it has
-    // nothing left to wait for but its activations.  A step of one sequence through a layer of width 1,024, us behind the
-    // kernel before: q-k-v and output products 5.3 to 3.1, gate/up pair 5.6 to 4.3, down product (K 2,816) 4.3 to 4.1.
+    // How many k-steps a thread loads before it multiplies (the order of the sums does not depend on it).  Up to 8 rows against one
+    // matrix whose blocks fit the SMs at once take more of them, so that a block that has waited for the kernel before it has
+    // little left to wait for but its activations: all of a warp's for K <= 1,024 (4, 8 or 16 steps by what K has) and in 2,048 < K
+    // <= 3,072 (12), 16 at a time in between and 8 at a time above; a pair's warp, which loads two rows each, up to 8 (K <= 512: all).
+    // A step of one sequence through a layer of width 1,024, us behind the kernel before: q-k-v and output products 5.3 to 3.1,
+    // gate/up pair 5.6 to 4.3, down product (K 2,816) 4.3 to 4.1; by themselves, one row x 2,048 columns, K 512 2.5 to 2.3, 688 3.3 to
+    // 2.5, 1,024 5.2 to 2.9.  More steps than K has cost: K 256 1.9 us with 4, 2.4 with 16.
     // Where blocks queue for the SMs registers are worth more: an expert's down product (K 688, four experts) 8.4 us with
     // 4 steps ahead, 10.0 with all 11.
     const unsigned blocks = (unsigned)((a.N + SK_COLS - 1) / SK_COLS);
@@ -302,12 +306,14 @@ static int skinny_launch_shape(const SkinnyArgs& a, cudaStream_t s) {
         // step at batch 8 took 2.4 % longer; 4 or 1 warps on K, or 8 loads ahead, are slower too).  Tried on the
         // gate/up pair as well (8 gate and 8 up rows per tile, half the bytes per block): no gain.
         constexpr int WK = 2, WN = 1, UNR = NT >= 4 ? 2 : 4;
+        const int steps = (a.K + WK * 32 - 1) / (WK * 32);
         dim3 grid(blocks, a.by_row ? a.M : a.G);
         if constexpr (NT == 1 && DUAL) {
-            if (few) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
+            if (few && steps > 4) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
             else TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
         } else if constexpr (NT == 1) {
-            if (few) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 16>), grid, WK * WN * 32, 0, s, a);
+            if (few && steps > 8) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 16>), grid, WK * WN * 32, 0, s, a);
+            else if (few && steps > 4) TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, 8>), grid, WK * WN * 32, 0, s, a);
             else TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
         } else
             TB_LAUNCH((gemm_skinny_kernel<NT, DUAL, TY, WK, WN, UNR>), grid, WK * WN * 32, 0, s, a);
@@ -341,7 +347,7 @@ static int skinny_entry(const void* X, const int* x_rows, const void* W, void* Y
     if (((uintptr_t)X | (uintptr_t)W) & 15) return TB_ERR_UNSUPPORTED;
     if (M == 0) return 0;
     SkinnyArgs a{(const __nv_bfloat16*)X, x_rows, (const __nv_bfloat16*)W, Y, group_offsets, w_group_stride,
-                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, row_group && 2 * M <= G, glu};
+                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, row_group && G >= 16 && 4 * M <= G && M <= 16, glu};
     int rows = (max_group_rows > 0 && max_group_rows < M) ? max_group_rows : M;
     if (G > 1) {
         // A pass takes 8, 16 or 32 rows of a group and a thread's registers are sized by the pass (with 16 rows the
