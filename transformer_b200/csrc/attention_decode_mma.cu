@@ -437,7 +437,7 @@ attention_decode_mma_kernel(const __grid_constant__ CUtensorMap mk, const __grid
     __syncthreads();
     if (!last_slice) return;
     __threadfence();
-    // Every thread asks for two channels of up to eight slices, then every slice's maximum and sum go to factors in shared memory
+    // The sums in the order of attention_merge_kernel, to the bit.  Every thread asks for two channels of up to eight slices, then every slice's maximum and sum go to factors in shared memory
     // (the ring's), all loads at once.  (A loop over the slices per channel, each load waiting for the
     // one before, was a large part of a step of one sequence; the sums keep their order.)
     float* f_m = sm_o;                                      // [nheads][slices] maxima

@@ -37,7 +37,7 @@ __host__ __device__ inline int cd_vpitch(int vdim) { return (vdim + 31) / 32 * 3
 // tokens), a warp per token for the two unit norms and k . q, then all threads write the group's records: q, k,
 // decays, betas, and the values.  Four tokens a block for prompts, one for steps of few tokens (more blocks).
 #define CD_PT 4
-#define CD_PREP_FEW 384     // threads of a block with one token
+#define CD_PREP_FEW 384     // threads of a block with one token: a channel each up to so many channels a key head (3 heads of 128)
 template <typename T>
 __global__ void __launch_bounds__(CD_PREP_FEW) delta_prep_kernel(const DeltaPrepArgs p, int nt, int pt) {
     pdl_sync();
@@ -250,7 +250,7 @@ static int delta_prep_launch(const DeltaPrepArgs& p, int nt, int B, cudaStream_t
     }
     const int pt = nt >= 256 ? CD_PT : 1;
     dim3 pgrid((nt + pt - 1) / pt, p.G);
-    // a few tokens: a thread per channel (heads of 128), so that a block waits for its inputs once and not three times
+    // a few tokens: more threads, so that a block waits for its inputs once (up to CD_PREP_FEW channels) and not three times
     TB_LAUNCH((delta_prep_kernel<T>), pgrid, pt == 1 ? CD_PREP_FEW : 32 * CD_PT, smem, s, p, nt, pt);
     int rc = tb_last_error();
     if (rc || p.update_state || p.taps == 1) return rc;

@@ -433,7 +433,8 @@ static int mlstm_chunk_launch(const MlstmArgs& a, int B, cudaStream_t s) {
 }
 
 // y[t, h, :] = o[t, h, :] / sqrt(mean_h(o^2) + eps) * w[h, :] * sigmoid(g[t, h, :])     one warp per (token, head)
-// NV > 0: heads of 32 NV entries, everything a lane needs asked for at once (3,451 tokens of 16 heads of 128: 28 to 16 us); 0: any size.
+// NV > 0: heads of 32 NV entries, everything a lane needs asked for at once (3,451 tokens of 16 heads of 128: 28 to 16 us); made for 128
+// and 256, the sizes whose rows are worth it (shorter ones are one or two loads a lane anyway).  0: any size.
 template <typename T, int NV>
 __global__ void __launch_bounds__(128)
 mlstm_out_kernel(const float* __restrict__ o, const T* __restrict__ g, int ldg, const float* __restrict__ w,

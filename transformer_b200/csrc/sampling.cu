@@ -129,7 +129,8 @@ __device__ Cut select_cut(const float* __restrict__ row, int V, float inv_t, flo
 // ---- a small top_k ---------------------------------------------------------------------------------------------
 // The top_k-th largest of the threads' maxima is a lower bound of the top_k-th largest z, so a second pass over the row
 // collects a few more than top_k candidates; these are sorted (key descending, id ascending), and the rest happens in
-// shared memory, its sums in a fixed order.  The radix selects read the row thirteen times, with most of its values in a
+// shared memory, its sums in a fixed order.  A row of so many ties that the candidates don't fit pays for the attempt (three rows of
+// 32,000 with four values: 163 to 179 us).  The radix selects read the row thirteen times, with most of its values in a
 // few bins of the first pass: 145 us for three rows of 32,000 with top_k 40 and top_p 0.9.  Here 17 us.
 #define SAMP_FEW 256            // largest top_k
 #define SAMP_CANDIDATES 1024    // more values than this at or above the bound (ties): the radix selects

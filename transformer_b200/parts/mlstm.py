@@ -26,7 +26,7 @@ USE_CHUNKS = True      # prompts: the kernel that takes 64 tokens at a time
 # Tokens a sequence (on average) from which its chunks are done side by side: four launches against 22 us a chunk of 64 tokens
 # (8 heads of 128 x 256, us: 1 x 128 tokens 62 and 49, 1 x 192 67 and 71, 1 x 300 71 and 114, 1 x 2,039 154 and 699)
 PARALLEL_TOKENS = 192
-# ... and the most scratch that their states may take, one per chunk (8 heads of 128 x 256: 8 MB a chunk over the heads): steps of
+# ... and the most scratch that their states may take, one per chunk (8 heads of 128 x 256: 1 MB a chunk over the heads): steps of
 # more chunks are done in portions
 PARALLEL_BYTES = 256 << 20
 
