@@ -621,6 +621,21 @@ def test_attention_decode_on_tensor_cores(nh, nkvh, dh):
     assert _run_attention(lib, c48, torch.bfloat16, 1, decode=True, ring=True) is None, "a head of 48 is refused"
 
 
+@pytest.mark.parametrize("nh,nkvh,dh", [(16, 4, 128), (20, 1, 64), (8, 2, 256)])
+def test_slices_merged_in_the_kernel_have_the_merge_kernels_bits(nh, nkvh, dh):
+    """Grouped heads and contexts of up to 3,000 keys: a slice goes round the ring of pages several times, then the block that ends
+    last merges its head group's slices.  Against partial results that a kernel of its own merges, bit for bit."""
+    lib = _lib()
+    c = attention_case([1] * 5, [2999, 1850, 511, 64, 3], nh, nkvh, dh, torch.bfloat16, 1, seed=5 * nh + dh)
+    done = torch.zeros(5 * nh, dtype=torch.int32, device="cuda")
+    for splits in (2, 4, 16, 32):
+        want = _run_attention(lib, c, torch.bfloat16, splits, decode=True, ring=True, done=None)
+        assert float((want - c["ref"]).abs().max()) <= _tol(torch.bfloat16, 4.0)
+        for _ in range(3):
+            assert torch.equal(_run_attention(lib, c, torch.bfloat16, splits, decode=True, ring=True, done=done), want)
+        assert int(done.abs().sum()) == 0
+
+
 @pytest.mark.parametrize("pairing", ["adjacent", "half"])
 @pytest.mark.parametrize("nh,nkvh,dh", [(4, 4, 64), (8, 2, 128), (12, 2, 64), (40, 2, 128), (3, 1, 128), (6, 2, 192),
                                         (4, 1, 256)])
