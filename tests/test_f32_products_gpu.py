@@ -1,5 +1,6 @@
-"""The 32-bit products at the edges of their kernels: passes of 4, 8 and 16 rows, one and several warps on K, tiles of
-64 x 64 with remainders, groups that are empty or hold a remainder, gathered rows, and rows the 16-byte kernels refuse.
+"""The 32-bit products at the edges of their kernels: passes of 4, 8 and 16 rows, four and eight warps on K, tiles of
+64 x 64 with remainders, groups that are empty or hold a remainder, gathered rows, rows the 16-byte kernels refuse, and rows
+below 512 entries, which the general kernel takes.
 
 The bound is that of any order of summation in float: |error| <= (K + 8) 2^-24 sum |a b| for a product."""
 import pytest

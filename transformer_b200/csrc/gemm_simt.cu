@@ -13,8 +13,9 @@
 //    stores silu(gate) * up  (swiglu, compute.rs:324-326), in float, rounded once.
 //  Any M, N, K >= 1; edges are predicated.
 //
-// Three kernels: gemm_simt_kernel takes anything; for float with 16-byte rows, gemm_rows_f32_kernel streams the weights
-// past a few rows (decoding), and gemm_tile_f32_kernel multiplies tiles fed by cp.async (prompts).
+// Three kernels: gemm_simt_kernel takes anything; for float with 16-byte rows of GF_K entries or more, gemm_rows_f32_kernel
+// streams the weights past a few rows (decoding), and gemm_tile_f32_kernel multiplies tiles fed by cp.async (prompts).  The three
+// take a sum in different orders, so the last bits of a row depend on how many rows (of its group, on average) the call has.
 #include "attention_prefill.cuh"        // cp_async16, cp_async_commit, cp_async_wait
 #include "memory_common.cuh"            // fma2
 
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const GemmArgs a) {
 // and 7.1 us; a decode step of three sequences (width 1,024, 8 layers, 8 experts of 512) 4.6 and 0.58 ms.
 // SLICED (many rows, no pair): the rows of a crowded group are dealt to several blocks, 16 passes each.  2,048 rows for 128 experts
 // (512 -> 1,024) that all went to one: 442 us by the blocks of that expert alone (the general kernel: 390), 217 so; evenly
-// spread 223 and 216.  A pair has twice the work a row and stays ahead of the general kernel without (424 and 714 us; dealt out, its
+// spread 223 and 212.  A pair has twice the work a row and stays ahead of the general kernel without (424 and 714 us; dealt out, its
 // registers run out and an even spread costs 7 % more).
 #define GR_PASSES 16
 template <int MT, int CT, bool DUAL, bool SLICED>
@@ -296,7 +297,8 @@ __global__ void __launch_bounds__(256) gemm_rows_f32_kernel(const GemmArgs a, in
 
 template <int MT, int CT, bool DUAL>
 static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
-    // as many warps on K as it has pieces of 128 entries, up to eight; with fewer than four, more columns a block
+    // as many warps on K as it has pieces of 128 entries, up to eight; with fewer than four (K below GF_K, which the launcher keeps
+    // away), more columns a block
     const int wk = a.K >= 1024 ? 8 : a.K >= 512 ? 4 : a.K >= 256 ? 2 : 1;
     const int warps = wk == 8 ? 8 : 4, cols = (DUAL ? CT / 2 : CT) * (warps / wk);
     // Without offsets all rows belong to matrix 0, whatever G is: a block for every g would write the same places.
@@ -310,12 +312,12 @@ static void gemm_rows_f32_go(const GemmArgs& a, cudaStream_t s) {
 // 64 x 64 outputs a block, 32 x 32 a warp, 8 x 4 a thread; K in steps of 32 through a ring of three stages filled by
 // cp.async.  Four warps take the first 16 entries of a step and four the others, and their sums are joined at the end:
 // a prompt of a few hundred tokens has fewer tiles than the GPU has SMs, and one warp a scheduler does not hide the
-// latencies of its own loads (254 rows x 1,536 x 1,024: 85 us with four warps a block, 61 with eight; an expert's pair
-// for 254 tokens 110 and 73; 2,048 x 4,096 x 4,096, where tiles abound, 1,510 and 1,674).  Tiles lie in shared memory as in memory (K innermost, rows 36 floats apart: the eight
+// latencies of its own loads.  Tiles lie in shared memory as in memory (K innermost, rows 36 floats apart: the eight
 // rows that a quarter of a warp reads start in different banks), so a thread's operands are 16-byte loads of four
-// entries of K: 12 of them feed 128 multiply-adds, two an instruction (one each: 44, 23 and 74 us behind the kernel before for the
-// q-k-v, output and gate/up products of such a prompt, 33, 17 and 65 with two).  Bound by multiply-add issue; the general kernel reads
-// one float at a time (8 loads for 16 multiply-adds) and waits for global memory in every step: 148, 274 and 3,236 us for these three.
+// entries of K: 12 of them feed 128 multiply-adds, two an instruction.  Bound by multiply-add issue.  The general kernel reads one float
+// at a time (8 loads for 16 multiply-adds) and waits for global memory in every step.  us, here and there:
+// 254 rows x 1,536 x 1,024 38 and 84, a pair of 2,816 125 and 258, pairs of 8 experts (1,024 -> 512, 508 rows) 64 and 182, 2,048 x 4,096 x
+// 4,096 1,956 and 3,240.
 #define GT_BK 32
 #define GT_PITCH (GT_BK + 4)
 #define GT_STAGES 3
@@ -433,9 +435,10 @@ __global__ void __launch_bounds__(256) gemm_tile_f32_kernel(const GemmArgs a) {
 // taken 4, 8 or 16 at a time by what most groups hold, as gemm_skinny does; above, tiles.  Measured at the border: 16
 // rows x 1,536 x 1,024 7.1 us here, 17 rows 39 us in tiles; a pair of 8 experts (1,024 -> 512) 25 us for groups of 15 rows
 // here, 73 for groups of 25 in tiles (one tile a group, mostly empty, and the general kernel's 200 and 219).
-// Rows shorter than GF_K stay with the general kernel, whose walk over K is short then (calls from Python one after the other: 254
-// rows x 1,024 x 252 22.6 us, x 256 in tiles 12.8; 3 rows x 512 x 128 13 us with either): models that small have tokens whose
-// logits another order of the sums moves by several times their mean error, and little to win.
+// Rows shorter than GF_K stay with the general kernel, not because it is faster (calls from Python one after the other: 254 rows x
+// 1,024 x 252 22.6 us, x 256 in tiles 12.8; 3 rows x 512 x 128 13 us with either) but because its walk over K is short there and models
+// that small keep the results they had: a tiny model of the tests has a token whose logits another order of the sums moves by 1.1e-4
+// where the mean error is 6e-6 in either order.
 #define GF_K 512
 static bool gemm_f32_launch(const GemmArgs& a, bool dual, cudaStream_t s) {
     if (a.K < GF_K || a.K % 4 || a.lda % 4 || a.ldb % 4 || a.b_group_stride % 4 || (((uintptr_t)a.A | (uintptr_t)a.B) & 15)) return false;
