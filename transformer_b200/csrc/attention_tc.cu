@@ -31,18 +31,30 @@
 #define AT_BN 64
 #define AT_STAGES 2
 #define AT_THREADS 192
+#define AT_BARS (4 * AT_STAGES + 7)
+
+// What a kernel does beside plain causal attention.
+#define AT_PLAIN 0
+#define AT_WINDOW 1       // window, kept first tokens, chunks, sinks, gates (attention_window.cu)
+#define AT_CAPPED 2       // the same with capped scores
 
 struct AtArgs {
-    __nv_bfloat16* out;       // [nt, nh * dh]
+    __nv_bfloat16* out;       // [nt, ldo]
     const int* tile_seq;
     const int* tile_t0;
     const int* tile_nq;
     const int* tok_pos;
     const int* page_table;
     int* error;
-    int tiles, max_pages, nh, nkvh;
+    int tiles, max_pages, nh, nkvh, ldo;
     float scale_log2e;
     unsigned v_lbo, v_sbo;    // descriptor strides of the MN-major V operand, in bytes
+    // all but AT_PLAIN
+    const float* sinks;           // [nh] or null
+    const __nv_bfloat16* gate;    // [nt, gate_stride] or null
+    int gate_stride, gate_per_head, window, keep_first, chunk;
+    float out_scale;
+    float cap_l2, pre_cap;        // AT_CAPPED: cap * log2 e and 2 log2 e * scale / cap
 };
 
 // Shared-memory descriptor with explicit strides (K-major operands use umma_desc of tc_common.cuh).
@@ -113,13 +125,15 @@ __device__ __forceinline__ void tmem_st32_words(uint32_t taddr, const uint32_t (
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-template <int DH>
-__global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
-                                                                 const __grid_constant__ CUtensorMap map_k,
-                                                                 const __grid_constant__ CUtensorMap map_v,
-                                                                 const AtArgs a) {
+// KB: 64-wide column boxes of a head; FORM: see AT_PLAIN.
+template <int KB, int FORM>
+__global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                    const __grid_constant__ CUtensorMap map_k,
+                                                                    const __grid_constant__ CUtensorMap map_v,
+                                                                    const AtArgs a) {
     pdl_sync();
-    constexpr int KB = DH / 64;                          // 64-wide column boxes of a row of dh values
+    constexpr bool CAPPED = FORM == AT_CAPPED, PLAIN = FORM == AT_PLAIN;
+    constexpr int DH = KB * 64;
     constexpr uint32_t Q_BYTES = AT_BM * DH * 2, KV_BYTES = AT_BN * DH * 2;
     constexpr uint32_t STAGE_BYTES = 2 * KV_BYTES;
     constexpr uint32_t TMEM_COLS = 256;                  // S twice (2 x 64 columns) and O (dh columns)
@@ -129,8 +143,8 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     const uint32_t smem_base = smem_u32(smem_raw);
     const uint32_t sq = smem_base, skv = sq + Q_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Q_BYTES + AT_STAGES * STAGE_BYTES);   // 4 * stages + 7
-    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 4 * AT_STAGES + 7);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Q_BYTES + AT_STAGES * STAGE_BYTES);
+    uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + AT_BARS);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (smem_base & 1023u) {                              // never expected; refuse rather than compute garbage
         if (threadIdx.x == 0) atomicCAS(a.error, 0, 19);
@@ -143,8 +157,17 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
     const int h = blockIdx.x, g = h / (a.nh / a.nkvh);
     const int b = a.tile_seq[tile], t0 = a.tile_t0[tile], nq = a.tile_nq[tile];
     const int pos_first = a.tok_pos[t0], pos_last = pos_first + nq - 1;
-    const int n_tiles = pos_last / AT_BN + 1;
     const int* pt = a.page_table + (size_t)b * a.max_pages;
+    // the pages to visit: those of the kept first tokens that lie before the window's, then the window's
+    int first = 0, win_p0 = 0;
+    if constexpr (!PLAIN) {
+        int win_lo = a.window > pos_first ? 0 : pos_first - a.window + 1;
+        if (a.chunk > 0) win_lo = max(win_lo, pos_first / a.chunk * a.chunk);     // nothing before the first row's chunk
+        win_p0 = win_lo / AT_BN;
+        first = min((min(a.keep_first, pos_last + 1) + AT_BN - 1) / AT_BN, win_p0);
+    }
+    const int n_tiles = first + pos_last / AT_BN + 1 - win_p0;
+    auto page_of = [&](int j) { return PLAIN || j >= first ? win_p0 + j - first : j; };
 
     const uint32_t bar0 = smem_u32(bars);
     // K and V have barriers of their own: a K slot is free as soon as the scores that read it are done,
@@ -195,7 +218,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             int issued = 0;
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int s = j % AT_STAGES;
-                const int row = (pt[j] * a.nkvh + g) * TB_PAGE;
+                const int row = (pt[page_of(j)] * a.nkvh + g) * TB_PAGE;
                 const uint32_t sk = skv + s * STAGE_BYTES, sv = sk + KV_BYTES;
                 if (j >= AT_STAGES) ok = mbar_wait(k_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11);
                 if (!ok) break;
@@ -275,6 +298,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         float m_used = -INFINITY, l_run = 0.f;
         bool ok = true;
+        const float scale = CAPPED ? 1.0f : a.scale_log2e;
         for (int j = 0; j < n_tiles && ok; ++j) {
             ok = mbar_wait(s_full(j & 1), (j >> 1) & 1, a.error, 15);
             tc_fence_after();
@@ -295,11 +319,36 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             // handled with as few instructions as will do: the maximum on the raw scores (the scale is
             // positive), the mask only on tiles that reach past the row's own position, and
             // p = 2^(s * scale - m) as one fused multiply-add and one ex2.approx each.
-            const int key0 = j * AT_BN;
-            if (key0 + AT_BN - 1 > pos_first) {             // uniform over the block: a tile on or past the diagonal
+            const int key0 = page_of(j) * AT_BN;
+            if constexpr (CAPPED) {
+                // score * log2 e, capped: cap tanh(y) = cap - 2 cap / (1 + e^{2y}), y = s * scale / cap
 #pragma unroll
-                for (int i = 0; i < AT_BN; ++i)
-                    if (key0 + i > pos_r) s[i] = -INFINITY;
+                for (int i = 0; i < AT_BN; ++i) {
+                    float e;
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(s[i] * a.pre_cap));
+                    s[i] = a.cap_l2 - __fdividef(2.0f * a.cap_l2, 1.0f + e);
+                }
+            }
+            if constexpr (PLAIN) {
+                if (key0 + AT_BN - 1 > pos_first) {             // uniform over the block: a tile on or past the diagonal
+#pragma unroll
+                    for (int i = 0; i < AT_BN; ++i)
+                        if (key0 + i > pos_r) s[i] = -INFINITY;
+                }
+            } else {
+                // every key visible to every row: not later than the first row's token, inside the last row's window
+                // or among the kept, in the last row's chunk (uniform over the block)
+                const bool open = key0 + AT_BN - 1 <= pos_first &&
+                                  (pos_last - key0 < a.window || key0 + AT_BN - 1 < a.keep_first) &&
+                                  (a.chunk <= 0 || key0 / a.chunk == pos_last / a.chunk);
+                if (!open) {
+                    const int near = pos_r - a.window, from = a.chunk > 0 ? pos_r / a.chunk * a.chunk : 0;
+#pragma unroll
+                    for (int i = 0; i < AT_BN; ++i) {
+                        const int key = key0 + i;
+                        if (key > pos_r || key < from || !(key > near || key < a.keep_first)) s[i] = -INFINITY;
+                    }
+                }
             }
             // two chains of three-input maxima: 32 instructions for the 64 scores
             float mx = -INFINITY, mx1 = -INFINITY;
@@ -308,7 +357,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
                 asm("max.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(s[i]), "f"(s[i + 1]));
                 asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(s[i + 2]), "f"(s[i + 3]));
             }
-            mx = fmaxf(mx, mx1) * a.scale_log2e;
+            mx = fmaxf(mx, mx1) * scale;
             // raise the maximum only when it has grown by more than 8; then O must be rescaled
             const bool raise = mx > m_used + 8.0f;          // also true for the first visible keys (m_used = -inf)
             const float m_new = raise ? mx : m_used;
@@ -319,7 +368,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             // only the stores below come after it
             uint32_t pk[AT_BN / 2];
             // two scores at a time through the packed forms of multiply-add and add (half the instructions)
-            const uint64_t sc2 = pack_f32x2(a.scale_log2e, a.scale_log2e), nm2 = pack_f32x2(neg_m, neg_m);
+            const uint64_t sc2 = pack_f32x2(scale, scale), nm2 = pack_f32x2(neg_m, neg_m);
             uint64_t psum_a = 0ull, psum_b = 0ull;              // two pairs of +0.0f
 #pragma unroll
             for (int i = 0; i < AT_BN; i += 4) {
@@ -378,8 +427,22 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
             tc_fence_after();
         }
         if (ok) {
-            const float inv = 1.0f / l_run;
-            __nv_bfloat16* dst = a.out + ((size_t)(t0 + row) * a.nh + h) * DH;
+            float inv = 1.0f / l_run;
+            const int t = t0 + row;
+            const __nv_bfloat16* gt = nullptr;
+            if constexpr (!PLAIN) {
+                if (a.sinks) {      // the larger of the sink and the reference stays the reference
+                    const float sk = a.sinks[h] * 1.4426950408889634f;
+                    inv = sk > m_used ? exp2f(m_used - sk) / (l_run * exp2f(m_used - sk) + 1.f) : 1.0f / (l_run + exp2f(sk - m_used));
+                }
+                inv *= a.out_scale;
+                if (a.gate && row < nq) {
+                    const __nv_bfloat16* gr = a.gate + (size_t)t * a.gate_stride;
+                    if (a.gate_per_head) inv = __fdividef(inv, 1.0f + __expf(-__bfloat162float(gr[h])));
+                    else gt = gr + (size_t)h * DH;
+                }
+            }
+            __nv_bfloat16* dst = a.out + (size_t)t * a.ldo + (size_t)h * DH;
 #pragma unroll
             for (int c0 = 0; c0 < DH; c0 += 32) {
                 float o[32];
@@ -390,6 +453,14 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
                         float f8[8];
 #pragma unroll
                         for (int e = 0; e < 8; ++e) f8[e] = o[i + e] * inv;
+                        if constexpr (!PLAIN) {
+                            if (gt) {
+                                float g8[8];
+                                load8(gt + c0 + i, g8);
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) f8[e] = __fdividef(f8[e], 1.0f + __expf(-g8[e]));
+                            }
+                        }
                         store8(dst + c0 + i, f8);
                     }
                 }
@@ -401,19 +472,48 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tc_kernel(const __grid_c
     if (warp == 1) tmem_dealloc(tmem_slot, TMEM_COLS);
 }
 
-template <int DH>
+template <int KB, int FORM>
 static int attention_tc_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AtArgs& a,
                                cudaStream_t s) {
-    const size_t smem = (size_t)AT_BM * DH * 2 + (size_t)AT_STAGES * 2 * AT_BN * DH * 2 + 160;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    const size_t smem = (size_t)AT_BM * KB * 128 + (size_t)AT_STAGES * 2 * AT_BN * KB * 128 + (AT_BARS + 1) * 8;
+    static PerDevice raised;
+    tb_allow_smem(raised, (const void*)attention_tc_kernel<KB, FORM>, smem);
     dim3 grid(a.nh, a.tiles);
-    TB_LAUNCH((attention_tc_kernel<DH>), grid, AT_THREADS, smem, s, mq, mk, mv, a);
+    TB_LAUNCH((attention_tc_kernel<KB, FORM>), grid, AT_THREADS, smem, s, mq, mk, mv, a);
     return tb_last_error();
+}
+
+// What the forms' arguments have in common: checked, in `a` and in the maps.
+static int at_paged(const void* q, void* out, const void* kc, const void* vc, const int* tile_seq, const int* tile_t0,
+                    const int* tile_nq, const int* tok_pos, const int* page_table, int tiles, int nt, int max_pages,
+                    int q_stride, int nh, int nkvh, int dh, int cache_pages, AtArgs& a, CUtensorMap& mq, CUtensorMap& mk,
+                    CUtensorMap& mv) {
+    if (nh <= 0 || nkvh <= 0 || nh % nkvh || tiles < 0 || nt < 0 || cache_pages <= 0) return TB_ERR_ARG;
+    if (dh != 64 && dh != 128) return TB_ERR_UNSUPPORTED;
+    if (q_stride % 8 || (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kc | (uintptr_t)vc) & 15)) return TB_ERR_UNSUPPORTED;
+    if (tiles == 0) return 0;
+    int rc = make_map(&mq, q, nt, nh * dh, q_stride, AT_BM);
+    if (rc) return rc;
+    const long long rows = (long long)cache_pages * nkvh * TB_PAGE;
+    rc = make_map(&mk, kc, rows, dh, dh, AT_BN);
+    if (rc) return rc;
+    rc = make_map(&mv, vc, rows, dh, dh, AT_BN);
+    if (rc) return rc;
+    a.out = (__nv_bfloat16*)out;
+    a.tile_seq = tile_seq;
+    a.tile_t0 = tile_t0;
+    a.tile_nq = tile_nq;
+    a.tok_pos = tok_pos;
+    a.page_table = page_table;
+    a.error = tc_error_ptr();
+    if (!a.error) return tb_last_error();
+    a.tiles = tiles;
+    a.max_pages = max_pages;
+    a.nh = nh;
+    a.nkvh = nkvh;
+    a.v_lbo = AT_BN * 128;
+    a.v_sbo = 1024;
+    return 0;
 }
 
 extern "C" {
@@ -426,26 +526,51 @@ int tb_attention_tc_bf16(const void* q, void* out, const void* kc, const void* v
                          const int* tile_t0, const int* tile_nq, const int* tok_pos, const int* page_table, int tiles,
                          int nt, int max_pages, int q_stride, int nh, int nkvh, int dh, int cache_pages, float scale,
                          cudaStream_t s) {
-    if (nh <= 0 || nkvh <= 0 || nh % nkvh || tiles < 0 || nt < 0 || cache_pages <= 0) return TB_ERR_ARG;
-    if (dh != 64 && dh != 128) return TB_ERR_UNSUPPORTED;
-    if (q_stride % 8 || (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kc | (uintptr_t)vc) & 15)) return TB_ERR_UNSUPPORTED;
-    if (tiles == 0) return 0;
+    AtArgs a = {};
+    a.ldo = nh * dh;
+    a.scale_log2e = scale * 1.4426950408889634f;
     CUtensorMap mq, mk, mv;
-    int rc = make_map(&mq, q, nt, nh * dh, q_stride, AT_BM);
-    if (rc) return rc;
-    const long long rows = (long long)cache_pages * nkvh * TB_PAGE;
-    rc = make_map(&mk, kc, rows, dh, dh, AT_BN);
-    if (rc) return rc;
-    rc = make_map(&mv, vc, rows, dh, dh, AT_BN);
-    if (rc) return rc;
-    int* err_ptr = tc_error_ptr();
-    if (!err_ptr) return tb_last_error();
-    AtArgs a{(__nv_bfloat16*)out, tile_seq, tile_t0, tile_nq, tok_pos, page_table, err_ptr, tiles, max_pages, nh, nkvh,
-             scale * 1.4426950408889634f, (unsigned)(AT_BN * 128), 1024u};
-    return dh == 64 ? attention_tc_launch<64>(mq, mk, mv, a, s) : attention_tc_launch<128>(mq, mk, mv, a, s);
+    const int rc = at_paged(q, out, kc, vc, tile_seq, tile_t0, tile_nq, tok_pos, page_table, tiles, nt, max_pages, q_stride,
+                            nh, nkvh, dh, cache_pages, a, mq, mk, mv);
+    if (rc || tiles == 0) return rc;
+    return dh == 64 ? attention_tc_launch<1, AT_PLAIN>(mq, mk, mv, a, s) : attention_tc_launch<2, AT_PLAIN>(mq, mk, mv, a, s);
+}
+
+// The same with what the windowed attention (attention_window.cu) adds: a window, kept first tokens, chunks, capped scores, sinks
+// [nh], a gate [nt, gate_stride] (a number per output entry, or per head) and a multiplier of the output, whose rows are ldo apart.
+int tb_attention_tc_window_bf16(const void* q, void* out, const void* kc, const void* vc, const void* gate, const int* tile_seq,
+                                const int* tile_t0, const int* tile_nq, const int* tok_pos, const int* page_table, int tiles,
+                                int nt, int max_pages, int q_stride, int gate_stride, int nh, int nkvh, int dh, int cache_pages,
+                                int window, int keep_first, float scale, float softcap, int chunk, const float* sinks,
+                                int gate_per_head, float out_scale, int ldo, cudaStream_t s) {
+    if (window <= 0 || keep_first < 0 || chunk < 0 || ldo < nh * dh) return TB_ERR_ARG;
+    if (!(scale > 0.f) || !(softcap >= 0.f) || ldo % 8) return TB_ERR_UNSUPPORTED;
+    if (gate && !gate_per_head && (gate_stride % 8 || ((uintptr_t)gate & 15))) return TB_ERR_UNSUPPORTED;
+    const float log2e = 1.4426950408889634f;
+    AtArgs a = {};
+    a.ldo = ldo;
+    a.scale_log2e = scale * log2e;
+    a.sinks = sinks;
+    a.gate = (const __nv_bfloat16*)gate;
+    a.gate_stride = gate_stride;
+    a.gate_per_head = gate_per_head;
+    a.window = window;
+    a.keep_first = keep_first;
+    a.chunk = chunk;
+    a.out_scale = out_scale;
+    a.cap_l2 = softcap * log2e;
+    a.pre_cap = softcap > 0.f ? scale / softcap * 2.0f * log2e : 0.f;
+    CUtensorMap mq, mk, mv;
+    const int rc = at_paged(q, out, kc, vc, tile_seq, tile_t0, tile_nq, tok_pos, page_table, tiles, nt, max_pages, q_stride,
+                            nh, nkvh, dh, cache_pages, a, mq, mk, mv);
+    if (rc || tiles == 0) return rc;
+    if (softcap > 0.f)
+        return dh == 64 ? attention_tc_launch<1, AT_CAPPED>(mq, mk, mv, a, s) : attention_tc_launch<2, AT_CAPPED>(mq, mk, mv, a, s);
+    return dh == 64 ? attention_tc_launch<1, AT_WINDOW>(mq, mk, mv, a, s) : attention_tc_launch<2, AT_WINDOW>(mq, mk, mv, a, s);
 }
 }
 
 // replayable from C++ (tape.h)
 #include "tape.h"
 TB_TAPE_REGISTER(tb_attention_tc_bf16)
+TB_TAPE_REGISTER(tb_attention_tc_window_bf16)

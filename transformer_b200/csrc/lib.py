@@ -33,6 +33,7 @@ _SIGNATURES: Dict[str, str] = {
     "tb_attention_decode_f32": "ppppppppiiiiiiif", "tb_attention_decode_bf16": "ppppppppiiiiiiif",
     "tb_attention_prefill_bf16": "pppppppppiiiiiif",
     "tb_attention_tc_bf16": "pppppppppiiiiiiiif",
+    "tb_attention_tc_window_bf16": "ppppppppppiiiiiiiiiiiffipifi",
     "tb_gemm_tc_bf16": "ppppiiiiiiii", "tb_gather_rows_bf16": "pppii",
     "tb_attention_decode_mma_bf16": "pppppppppiiiiiiiif",
     "tb_attention_decode_rope_bf16": "pppppppppppiiiiiiiiiif",

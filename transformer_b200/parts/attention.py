@@ -193,7 +193,9 @@ class Attention(Mixer):
         self.window_tile = lib.attention_window_mma_tile_tokens(self.nh, self.nkvh) \
             if (self.extended and dtype == torch.bfloat16) else 0
         if self.extended:
-            self.prompt_tile = self.tc_tile = 0
+            self.prompt_tile = 0
+            if self.dv != self.dh or self.value_rotation or self.distance_bias is not None or not self.window_tile:
+                self.tc_tile = 0
         self.tile_sizes = [t for t in (self.general_tile, self.prompt_tile, self.tc_tile, self.window_tile) if t]
 
     @property
@@ -478,6 +480,21 @@ class Attention(Mixer):
                             ctx.max_pages, self.qkv_width, self.nh, self.nkvh, self.dh, splits, self.scale)
 
 
+def window_tcgen05_pays(ctx, m) -> bool:
+    """Whether a step's windowed attention is faster with 128 tokens of a head a block on the tcgen05 tensor cores than with the
+    mma.sync kernel's 64 rows of a head group, which can cut the keys into slices as well.  From 256 tokens a sequence on,
+    on average, if no sequence goes on behind more cached tokens than it brings or the blocks fill the SMs.  us, mma.sync and
+    tcgen05, 16 heads of 128 over 4 key heads, window 2,048, capped scores: 300 tokens 26 and 19, 2 x 600 42 and 28, 2,048 110
+    and 63 (uncapped 103 and 44), 4 x 400 behind 1,500 108 and 84; not taken: 8 x 129 20 and 23, 64 behind 2,000 33 and 60,
+    64 x 3 behind 500 26 and 95.  Heads of 64 from 80 blocks on: 8 heads, 2 x 600 25 and 23, 1,000 28 and 32."""
+    key = ("window_tc", m.tc_tile, m.nh, m.dh)
+    if key not in ctx.plans:
+        blocks = ctx.tiles(m.tc_tile).count * m.nh
+        fills = blocks >= ctx.engine.sm_count or all(b <= n for b, n in zip(ctx.h_pos0, ctx.h_lens))
+        ctx.plans[key] = ctx.nt >= 256 * ctx.B and fills and (m.dh != 64 or blocks >= 80)
+    return ctx.plans[key]
+
+
 def run_window_attention(ctx, m, z, o, gate, cache, table, nt, window, q_stride=None, sinks=None, ocos=None,
                          osin=None, heads=None, dist_bias=None) -> None:
     """The windowed attention of the step's rotated queries ``z`` over the cache, into ``o`` (gate applied).
@@ -493,7 +510,16 @@ def run_window_attention(ctx, m, z, o, gate, cache, table, nt, window, q_stride=
     q_stride = m.qkv_width if q_stride is None else q_stride
     g_stride = m.qkv_width if gate is None else gate.stride(0)
     if m.window_tile and USE_WINDOW_MMA:
-        # bfloat16: the tensor-core kernel, for prompts and decoding alike.  Slices of the visited pages so that a few
+        if m.tc_tile and USE_TCGEN05 and not ctx.decode and ocos is None and dist_bias is None and window_tcgen05_pays(ctx, m):
+            # prompts: S and O in tensor memory, K and V pages by TMA
+            tiles = ctx.tiles(m.tc_tile)
+            per_head, mult, ldo = heads or (0, 1.0, o.stride(0))
+            if lib.try_call("tb_attention_tc_window_bf16", lib.ptr(z), lib.ptr(o), lib.ptr(cache.k), lib.ptr(cache.v), lib.ptr(gate),
+                            lib.ptr(tiles.seq), lib.ptr(tiles.t0), lib.ptr(tiles.nq), lib.ptr(ctx.tok_pos), lib.ptr(table),
+                            tiles.count, nt, ctx.max_pages, q_stride, g_stride, m.nh, m.nkvh, m.dh, cache.k.shape[0], window,
+                            m.keep_first, m.scale, m.softcap, m.chunk, lib.ptr(sinks), per_head, mult, ldo):
+                return
+        # bfloat16: the mma.sync kernel, for prompts and decoding alike.  Slices of the visited pages so that a few
         # sequences still fill the GPU: a function of the batch's shape alone (a captured graph keeps it)
         tiles = ctx.tiles(m.window_tile)
         reach = min(window, ctx.engine.spec.max_context) if not m.chunk else min(window, m.chunk)
