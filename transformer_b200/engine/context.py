@@ -113,7 +113,7 @@ class StepContext:
         # ---- pack everything into one int32 array -------------------------------------------
         seq_start = np.zeros(B + 1, dtype=np.int32)
         np.cumsum(lens, out=seq_start[1:])
-        tok_ids = np.fromiter((t for ts in tokens for t in ts), dtype=np.int32, count=nt)
+        tok_ids = np.concatenate([np.asarray(t, dtype=np.int32) for t in tokens]) if nt else np.zeros(0, np.int32)
         tok_seq = np.repeat(np.arange(B, dtype=np.int32), lens)
         tok_pos = np.concatenate([np.arange(p, p + n, dtype=np.int32) for p, n in zip(pos0, lens)]) if nt else \
             np.zeros(0, np.int32)
@@ -126,16 +126,14 @@ class StepContext:
             "want_rows": np.asarray(want_rows, dtype=np.int32), "page_table": table.reshape(-1),
         }
         self._tile_counts = {}
+        n_tokens = np.asarray(lens, dtype=np.int64)
         for tq in tile_sizes:
-            ts, t0, nq = [], [], []
-            for b in range(B):
-                for off in range(0, lens[b], tq):
-                    ts.append(b)
-                    t0.append(int(seq_start[b]) + off)
-                    nq.append(min(tq, lens[b] - off))
-            parts[f"tile_seq.{tq}"] = np.asarray(ts, dtype=np.int32)
-            parts[f"tile_t0.{tq}"] = np.asarray(t0, dtype=np.int32)
-            parts[f"tile_nq.{tq}"] = np.asarray(nq, dtype=np.int32)
+            counts = (n_tokens + tq - 1) // tq
+            ts = np.repeat(np.arange(B, dtype=np.int32), counts)
+            off = (np.arange(len(ts)) - np.repeat(np.cumsum(counts) - counts, counts)) * tq
+            parts[f"tile_seq.{tq}"] = ts
+            parts[f"tile_t0.{tq}"] = (seq_start[ts] + off).astype(np.int32)
+            parts[f"tile_nq.{tq}"] = np.minimum(tq, n_tokens[ts] - off).astype(np.int32)
             self._tile_counts[tq] = len(ts)
         offsets, total = {}, 0
         for k, v in parts.items():

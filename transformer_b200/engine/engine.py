@@ -15,6 +15,7 @@ from __future__ import annotations
 import gc
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..cache.paged import Cache
@@ -34,6 +35,28 @@ FUSE_DEPTH_ROWS = 1024
 
 class StepError(ValueError):
     pass
+
+
+def whole_numbers(values, below: int, wrong) -> np.ndarray:
+    """The values as int64, each of them in [0, below): ``wrong(value)`` makes the error of the first that is not.  A list of
+    ints is looked at as a whole; anything else value by value."""
+    if len(values) > 8:
+        try:
+            a = np.asarray(values)
+        except Exception:           # what it is then said of value by value
+            a = None
+        if a is not None and a.ndim == 1 and a.dtype.kind in "iu" and len(a) == len(values):
+            bad = (a < 0) | (a >= below)
+            if bad.any():
+                raise wrong(values[int(bad.argmax())])
+            return a.astype(np.int64)
+    out = np.empty(len(values), dtype=np.int64)
+    for i, v in enumerate(values):
+        n = int(v)
+        if not 0 <= n < below:
+            raise wrong(v)
+        out[i] = n
+    return out
 
 
 def _pending_signature(pending):
@@ -224,18 +247,17 @@ class Engine:
         if len(set(slots)) != B:
             raise StepError("a slot appears twice in one step")
         V = self.spec.vocab
+        ids, wanted = [], []
         for b in range(B):
             n = len(tokens[b])
             if n == 0:
                 raise StepError(f"sequence {b} of the step brings no token")
-            for t in tokens[b]:
-                if not (0 <= int(t) < V):
-                    raise StepError(f"token {t} lies outside the vocabulary of {V}")
-            for w in want[b]:
-                if not (0 <= int(w) < n):
-                    raise StepError(f"wanted place {w} lies outside the {n} tokens of sequence {b}")
+            ids.append(whole_numbers(tokens[b], V, lambda t: StepError(f"token {t} lies outside the vocabulary of {V}")))
+            wanted.append(whole_numbers(want[b], n, lambda w: StepError(
+                f"wanted place {w} lies outside the {n} tokens of sequence {b}")))
+        tokens, want = ids, wanted
         n_total = sum(len(t) for t in tokens)
-        one_each = n_total == B and all(list(w) == [0] for w in want)
+        one_each = n_total == B and all(len(w) == 1 for w in want)
         if device_tokens is not None and not one_each:
             raise StepError("device_tokens serve steps of one token per sequence that want its logits")
         # room for everything first: a step either runs whole or not at all
@@ -251,10 +273,8 @@ class Engine:
             if one_each and (device_tokens is not None or self._graphs_on(B)):
                 return self._run_decode(slots, tokens, pos0, device_tokens)
             if n_total <= self.max_step_tokens:
-                rows, base = [], 0
-                for b in range(B):
-                    rows.extend(base + int(w) for w in want[b])
-                    base += len(tokens[b])
+                base = np.cumsum([0] + [len(t) for t in tokens])
+                rows = np.concatenate([w + at for w, at in zip(want, base)]) if B else []
                 return self._run(slots, tokens, pos0, rows)
             return self._run_in_pieces(slots, tokens, pos0, want)
         except BaseException:
