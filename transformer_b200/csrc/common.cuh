@@ -132,7 +132,15 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&f)[8]) {
 struct GluRule {
     int kind;
     float alpha, limit;
+    // Not null: the pair has biases, gate's [N] then up's [N], and is silu(g + b) * (u + b'), both products rounded to bfloat16 first,
+    // as a pass over the stored products would have them; `fill` columns behind the results are then a one and zeros.
+    const float* bias = nullptr;
+    int fill = 0;
 };
+__device__ __forceinline__ float glu_apply_biased(float g, float u, float bg, float bu) {
+    const float a = __bfloat162float(__float2bfloat16_rn(g)) + bg;
+    return a / (1.0f + expf(-a)) * (__bfloat162float(__float2bfloat16_rn(u)) + bu);
+}
 __device__ __forceinline__ float gelu_tanh_2y(float g) { return 1.5957691216057308f * (g + 0.044715f * g * g * g); }
 __device__ __forceinline__ float glu_apply(float g, float u, const GluRule r) {
     if (r.kind == 0) return g / (1.0f + expf(-g)) * u;

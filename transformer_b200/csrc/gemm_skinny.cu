@@ -262,13 +262,18 @@ __global__ void __launch_bounds__(WK * WN * 32) gemm_skinny_kernel(const SkinnyA
                 if (DUAL) v2 += red[w_n][w][NMAT - 1][r][c];
             }
             if (DUAL) {
-                v = glu_apply(v, v2, a.glu);
+                v = a.glu.bias ? glu_apply_biased(v, v2, a.glu.bias[nb0 + cc], a.glu.bias[a.N + nb0 + cc]) : glu_apply(v, v2, a.glu);
             } else if (a.glu.kind == TB_ACT_RELU2) {
                 v = fmaxf(v, 0.f);
                 v *= v;
             }
             stf(static_cast<TY*>(a.Y) + (size_t)(listed ? list[chunk + r] : chunk + r) * a.ldy + nb0 + cc, v);
         }
+        if (DUAL && a.glu.fill && blockIdx.x == gridDim.x - 1)
+            for (int idx = threadIdx.x; idx < rows * a.glu.fill; idx += blockDim.x) {
+                const int r = idx / a.glu.fill, e = idx - r * a.glu.fill;
+                stf(static_cast<TY*>(a.Y) + (size_t)(chunk + r) * a.ldy + a.N + e, e == 0 ? 1.f : 0.f);
+            }
     }
 }
 
@@ -379,9 +384,16 @@ int tb_gemm_skinny_glu_bf16(const void* X, const int* x_rows, const void* W, voi
     return skinny_entry(X, x_rows, W, Y, group_offsets, w_group_stride, ldx, ldw, ldy, M, N, K, G, 2, max_group_rows,
                         row_group, x_div, w_constant, GluRule{kind, alpha, limit}, s);
 }
+// The pair with biases (see GluRule), one dense weight.
+int tb_gemm_skinny_bias_glu_bf16(const void* X, const void* W, const float* bias, void* Y, int ldx, int ldw, int ldy, int M, int N,
+                                 int K, int fill, cudaStream_t s) {
+    if (!bias || fill < 0 || ldy < N + fill) return TB_ERR_ARG;
+    return skinny_entry(X, nullptr, W, Y, nullptr, 0, ldx, ldw, ldy, M, N, K, 1, 2, 0, nullptr, 1, 1, GluRule{0, 0.f, 0.f, bias, fill}, s);
+}
 }
 
 // replayable from C++ (tape.h)
 #include "tape.h"
 TB_TAPE_REGISTER(tb_gemm_skinny_bf16)
 TB_TAPE_REGISTER(tb_gemm_skinny_glu_bf16)
+TB_TAPE_REGISTER(tb_gemm_skinny_bias_glu_bf16)

@@ -295,8 +295,18 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     // (2 ulp; the result is rounded to bfloat16 next).  The exact forms cost some hundred clocks
                     // per value with only these four warps on the SM to hide them: measured, the epilogue of a tile
                     // took 7 to 18 us, as long as streaming half of the tile's weights.
+                    if (a.glu.bias) {
+                        const float* bg = a.glu.bias + n0 + c0;
+                        const int last = a.N - 1 - n0 - c0;           // columns past the last are computed and not stored
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = glu_apply_fast(v[i], u[i], a.glu);
+                        for (int i = 0; i < 32; ++i) {
+                            const float* b = bg + min(i, last);
+                            v[i] = glu_apply_biased(v[i], u[i], __ldg(b), __ldg(b + a.N));
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = glu_apply_fast(v[i], u[i], a.glu);
+                    }
                 }
                 if (wide) {
                     // A lane holds 32 columns of ONE row: stored from here, every instruction of the warp would touch
@@ -369,6 +379,10 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                             if (i < c_end) dst[i] = __float2bfloat16_rn(v[i]);
                     }
                 }
+            }
+            if (a.glu.fill && piece == 0 && n0 + n_out >= a.N && m < tl.row_end) {
+                __nv_bfloat16* pad = static_cast<__nv_bfloat16*>(a.C) + (size_t)m * a.ldc + a.N;
+                for (int e = 0; e < a.glu.fill; ++e) pad[e] = __float2bfloat16_rn(e == 0 ? 1.f : 0.f);
             }
             // this warp has read its lanes of the accumulator: tell the leader's MMA thread
             tc_fence_before();
@@ -586,6 +600,13 @@ int tb_gemm_tc_glu_bf16(const void* A, const void* B, void* C, const int* group_
     return gemm_tc_entry(A, B, C, group_offsets, lda, ldb, ldc, M, N, K, G, 2, GluRule{kind, alpha, limit}, s);
 }
 
+// The (gate, up) pair with biases: C[m, n] = silu(g + bias[n]) (u + bias[N + n]), then `fill` columns of a one and zeros.
+int tb_gemm_tc_bias_glu_bf16(const void* A, const void* B, const float* bias, void* C, int lda, int ldb, int ldc, int M, int N, int K,
+                             int fill, cudaStream_t s) {
+    if (!bias || fill < 0 || ldc < N + fill) return TB_ERR_ARG;
+    return gemm_tc_entry(A, B, C, nullptr, lda, ldb, ldc, M, N, K, 1, 2, GluRule{0, 0.f, 0.f, bias, fill}, s);
+}
+
 // Nonzero if any tensor-core product gave up on a wait since the last call (1 producer, 2 MMA,
 // 3 epilogue, 4 drain, 5 accumulator hand-back); reading it synchronises the device and clears it.
 int tb_gemm_tc_status() {
@@ -616,4 +637,5 @@ int tb_gather_rows_bf16(const void* x, const int* rows, void* out, int M, int d,
 #include "tape.h"
 TB_TAPE_REGISTER(tb_gemm_tc_bf16)
 TB_TAPE_REGISTER(tb_gemm_tc_glu_bf16)
+TB_TAPE_REGISTER(tb_gemm_tc_bias_glu_bf16)
 TB_TAPE_REGISTER(tb_gather_rows_bf16)

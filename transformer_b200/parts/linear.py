@@ -128,6 +128,18 @@ def matmul_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w_is_weigh
         torch.mm(a, w.t(), out=out)
 
 
+def bias_glu_matmul(a, w, bias, h) -> bool:
+    """h[:, :n] = silu(gate + bias[:n]) * (up + bias[n:]), (gate, up) = a @ w.T with w [2 n, K]; a one and zeros in what columns h has
+    behind.  The bits of the product stored in bfloat16 and a pass over it.  False (and nothing done) where no kernel takes it."""
+    if a.dtype != torch.bfloat16:
+        return False
+    M, K, n = a.shape[0], a.shape[-1], w.shape[0] // 2
+    assert a.stride(-1) == 1 and w.is_contiguous() and h.stride(-1) == 1
+    name = "tb_gemm_skinny_bias_glu_bf16" if M <= SKINNY_MAX_ROWS else "tb_gemm_tc_bias_glu_bf16"
+    return lib.try_call(name, lib.ptr(a), lib.ptr(w), lib.ptr(bias), lib.ptr(h), a.stride(0), w.stride(0), h.stride(0), M, n, K,
+                        h.shape[1] - n)
+
+
 def stack_products(weights):
     """Weights [n_i, width] of products with the same rows as ONE weight, and where each one's columns begin in the
     product: at multiples of eight (rows of zeros between them), so that each part of a row is aligned like a row."""
