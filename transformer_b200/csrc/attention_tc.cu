@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
     const uint32_t sq = smem_base, skv = sq + Q_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Q_BYTES + AT_STAGES * STAGE_BYTES);
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + AT_BARS);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_number(), lane = threadIdx.x & 31;
     if (smem_base & 1023u) {                              // never expected; refuse rather than compute garbage
         if (threadIdx.x == 0) atomicCAS(a.error, 0, 19);
         return;
@@ -210,44 +210,50 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_expect_tx(q_full, Q_BYTES);
 #pragma unroll
             for (int kb = 0; kb < KB; ++kb) tma_load_2d(sq + kb * (AT_BM * 128), &map_q, q_full, h * DH + kb * 64, t0);
-            bool ok = true;
-            int issued = 0;
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int s = j % AT_STAGES;
-                const int row = (pt[page_of(j)] * a.nkvh + g) * TB_PAGE;
-                const uint32_t sk = skv + s * STAGE_BYTES, sv = sk + KV_BYTES;
-                if (j >= AT_STAGES) ok = mbar_wait(k_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11);
-                if (!ok) break;
+        }
+        __syncwarp();
+        bool ok = true;
+        int k_issued = 0, v_issued = 0;
+        for (int j = 0; j < n_tiles; ++j) {
+            const int s = j % AT_STAGES;
+            const int row = (pt[page_of(j)] * a.nkvh + g) * TB_PAGE;
+            const uint32_t sk = skv + s * STAGE_BYTES, sv = sk + KV_BYTES;
+            if (j >= AT_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(k_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11));
+            if (!ok) break;
+            if (elect_one()) {
                 mbar_expect_tx(k_full(s), KV_BYTES);
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) tma_load_2d(sk + kb * (AT_BN * 128), &map_k, k_full(s), kb * 64, row);
-                if (j >= AT_STAGES) ok = mbar_wait(v_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11);
-                if (!ok) break;
+            }
+            __syncwarp();
+            k_issued = j + 1;
+            if (j >= AT_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(v_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11));
+            if (!ok) break;
+            if (elect_one()) {
                 mbar_expect_tx(v_full(s), KV_BYTES);
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) tma_load_2d(sv + kb * (AT_BN * 128), &map_v, v_full(s), kb * 64, row);
-                issued = j + 1;
             }
-            if (*(volatile int*)a.error != 0) {
-                mbar_wait(q_full, 0, a.error, 14);
-                for (int j = max(0, issued - AT_STAGES); j < issued; ++j) {
-                    mbar_wait(k_full(j % AT_STAGES), (j / AT_STAGES) & 1, a.error, 14);
-                    mbar_wait(v_full(j % AT_STAGES), (j / AT_STAGES) & 1, a.error, 14);
-                }
-            }
+            __syncwarp();
+            v_issued = j + 1;
+        }
+        if (*(volatile int*)a.error != 0) {
+            mbar_wait(q_full, 0, a.error, 14);
+            for (int j = max(0, k_issued - AT_STAGES); j < k_issued; ++j) mbar_wait(k_full(j % AT_STAGES), (j / AT_STAGES) & 1, a.error, 14);
+            for (int j = max(0, v_issued - AT_STAGES); j < v_issued; ++j) mbar_wait(v_full(j % AT_STAGES), (j / AT_STAGES) & 1, a.error, 14);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc_s = umma_idesc(AT_BM, AT_BN);                       // both operands K-major
-            const uint32_t idesc_o = umma_idesc(AT_BM, DH) | (1u << 16);             // B (= V) is MN-major
-            // S = Q K^T of tile j into S buffer j & 1: K = dh in steps of 16; step k lives in column box k / 4,
-            // 32 bytes * (k % 4) along the row
-            auto issue_s = [&](int j) {
+        const uint32_t idesc_s = umma_idesc(AT_BM, AT_BN);                       // both operands K-major
+        const uint32_t idesc_o = umma_idesc(AT_BM, DH) | (1u << 16);             // B (= V) is MN-major
+        // S = Q K^T of tile j into S buffer j & 1: K = dh in steps of 16; step k lives in column box k / 4,
+        // 32 bytes * (k % 4) along the row
+        auto issue_s = [&](int j) {
+            if (elect_one()) {
                 const uint32_t sk = skv + (j % AT_STAGES) * STAGE_BYTES;
 #pragma unroll
                 for (int k = 0; k < DH / 16; ++k) {
@@ -257,26 +263,31 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                 }
                 umma_commit(s_full(j & 1));
                 umma_commit(k_empty(j % AT_STAGES));          // K of tile j is free once these scores are done
-            };
-            bool ok = mbar_wait(q_full, 0, a.error, 12);
-            if (ok) ok = mbar_wait(k_full(0), 0, a.error, 12);
-            if (ok) {
-                tc_fence_after();
-                issue_s(0);
             }
-            for (int j = 0; j < n_tiles && ok; ++j) {
-                const int s = j % AT_STAGES;
-                // the scores of the NEXT tile are computed while the softmax warps work on this one
-                if (j + 1 < n_tiles) {
-                    ok = mbar_wait(k_full((j + 1) % AT_STAGES), ((j + 1) / AT_STAGES) & 1, a.error, 12);
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_s(j + 1);
-                }
-                ok = mbar_wait(p_ready(j & 1), (j >> 1) & 1, a.error, 13);   // P is in tensor memory, where S of tile j was
-                if (ok) ok = mbar_wait(v_full(s), (j / AT_STAGES) & 1, a.error, 12);
+            __syncwarp();
+        };
+        bool ok = mbar_wait(q_full, 0, a.error, 12);
+        if (ok) ok = mbar_wait(k_full(0), 0, a.error, 12);
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            tc_fence_after();
+            issue_s(0);
+        }
+        for (int j = 0; j < n_tiles && ok; ++j) {
+            const int s = j % AT_STAGES;
+            // the scores of the NEXT tile are computed while the softmax warps work on this one
+            if (j + 1 < n_tiles) {
+                ok = __all_sync(0xffffffffu, mbar_wait(k_full((j + 1) % AT_STAGES), ((j + 1) / AT_STAGES) & 1, a.error, 12));
                 if (!ok) break;
                 tc_fence_after();
+                issue_s(j + 1);
+            }
+            ok = mbar_wait(p_ready(j & 1), (j >> 1) & 1, a.error, 13);   // P is in tensor memory, where S of tile j was
+            if (ok) ok = mbar_wait(v_full(s), (j / AT_STAGES) & 1, a.error, 12);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
                 const uint32_t sv = skv + s * STAGE_BYTES + KV_BYTES;
                 // O += P V: K = 64 keys in steps of 16 (16 keys = two 8-row groups = 2048 bytes along V's rows;
                 // 32 bytes along P's rows); N = dh spans KB column boxes of V
@@ -289,6 +300,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                 umma_commit(v_empty(s));
                 umma_commit(o_done(j & 1));
             }
+            __syncwarp();
         }
     } else {
         // ---------------- softmax / correction / epilogue: thread = query row ----------------

@@ -8,6 +8,17 @@
 #define TC_SPIN_LIMIT (1u << 22)
 
 // ---- small PTX wrappers ----------------------------------------------------------------------
+// One lane of a whole warp, the same at every call.  The instructions that one thread issues (tcgen05.mma, TMA copies) take
+// their descriptors from the warp's uniform registers; with a branch on the lane's number around a whole loop the compiler cannot always
+// use those, and an instruction then comes with a loop of its own (196 clocks a tcgen05.mma of any size, measured, against 48 to 128).  So
+// the loops and waits are the whole warp's, and only what has to come from one lane stands behind this.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
+// The warp's number in its block, known to be the same for all of its lanes.
+__device__ __forceinline__ int warp_number() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
