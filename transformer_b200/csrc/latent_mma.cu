@@ -14,47 +14,13 @@
 // With more than one slice a block leaves (maximum, sum, unnormalized output) and latent_merge_kernel joins them.
 //
 // Sizes: rank a multiple of 32 up to 512, rank + rot a multiple of 16; anything else goes to the general kernel.
-#include "common.cuh"
+#include "latent_common.cuh"
 
 // warps per block: 4 (any rank that is a multiple of 32), or 8 when the rank is a multiple of 64: twice the warps
 // on an SM to hide the latencies of a k-step's chain of ldmatrix and mma (with four, no unit was busy for more than
 // a third of the time and an SM held eight warps)
 #define LM_ROWS 16
 #define LM_KEYS TB_PAGE     // keys per tile = one page
-
-struct LatentMmaArgs {
-    const __nv_bfloat16* qa;     // [nt, H, rank]
-    const __nv_bfloat16* q;      // [nt, ldq]; head h's rotated part at h * q_head + q_plain
-    __nv_bfloat16* out;          // [nt, H, rank]
-    float* partial;              // [nt, H, splits, rank + 2] when splits > 1
-    const __nv_bfloat16* cache;  // [pages, TB_PAGE, rank + rot]
-    const int* tile_seq;
-    const int* tile_t0;
-    const int* tile_nq;
-    const int* tok_pos;
-    const int* page_table;
-    const float* cosT;
-    const float* sinT;
-    int max_pages, ldq, q_head, q_plain, H, rank, rot, rdims, window, heads_per_block, tokens_per_block, splits;
-    float scale;
-    const float* sinks;          // [H] or null: a number per head that joins the softmax's denominator once
-    const __nv_bfloat16* gate;   // [nt, ldg] or null: head h's output is multiplied by sigmoid(gate[t, h])
-    int ldg;
-};
-
-// What a sink and a gate make of a row's (maximum, sum): the factor for its unnormalized output.
-__device__ __forceinline__ float lm_finish(float m, float l, const float* sinks, const __nv_bfloat16* gate, int ldg,
-                                           int t, int h) {
-    float f = 1.f;
-    if (sinks) {
-        const float sk = sinks[h], m2 = fmaxf(m, sk);
-        f = m > -INFINITY ? __expf(m - m2) : 0.f;
-        l = l * f + __expf(sk - m2);
-    }
-    f = l > 0.f ? f / l : 0.f;
-    if (gate) f *= 1.0f / (1.0f + __expf(-__bfloat162float(gate[(size_t)t * ldg + h])));
-    return f;
-}
 
 __device__ __forceinline__ void lm_ldmatrix_x4(unsigned (&r)[4], const void* p) {
     const unsigned addr = (unsigned)__cvta_generic_to_shared(p);
@@ -96,16 +62,7 @@ __device__ __forceinline__ void lm_load_queries(const LatentMmaArgs& a, __nv_bfl
         float v = 0.f;
         if (ti < n_tok && h < a.H) {
             const int t = t0 + ti;
-            const __nv_bfloat16* qr = a.q + (size_t)t * a.ldq + (size_t)h * a.q_head + a.q_plain;
-            const int half = a.rdims / 2, pos = a.tok_pos[t];
-            v = __bfloat162float(qr[r]);
-            if (r < half) {
-                const float co = a.cosT[(size_t)pos * half + r], si = a.sinT[(size_t)pos * half + r];
-                v = v * co - __bfloat162float(qr[r + half]) * si;
-            } else if (r < a.rdims) {
-                const float co = a.cosT[(size_t)pos * half + r - half], si = a.sinT[(size_t)pos * half + r - half];
-                v = v * co + __bfloat162float(qr[r - half]) * si;
-            }
+            v = lm_turned(a, a.q + (size_t)t * a.ldq + (size_t)h * a.q_head + a.q_plain, r, a.tok_pos[t]);
         }
         q_s[row * pitch + a.rank + r] = __float2bfloat16_rn(v);
     }

@@ -61,6 +61,7 @@ _SIGNATURES: Dict[str, str] = {
     "tb_mlstm_out_f32": "ppippiiifii", "tb_mlstm_out_bf16": "ppippiiifii",
     "tb_latent_prep_f32": "pippfpppppippiiiii", "tb_latent_prep_bf16": "pippfpppppippiiiii",
     "tb_latent_attention_mma_bf16": "ppppppppppppiiiiiiiiiiifppi",
+    "tb_latent_attention_tc_bf16": "pppppppppppiiiiiiiiiiifppi",
     "tb_latent_attention_rows_bf16": "pppppppppppiiiiiiiiiifppi",
     "tb_latent_attention_f32": "pppppppppppiiiiiiiiiifppi", "tb_latent_attention_bf16": "pppppppppppiiiiiiiiiifppi",
     "tb_embed_bigram_f32": "pppppppppiifiii", "tb_embed_bigram_bf16": "pppppppppiifiii",
@@ -133,7 +134,7 @@ class TapeMap(ctypes.Structure):
 
 _NO_STREAM = {"tb_decay_scan_rect_record_size": "ii", "tb_split_delta_record_size": "i",
               "tb_decay_state_size": "iii", "tb_decay_record_size": "i",
-              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_gates": "", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
+              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_gates": "", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_latent_tc_tile_tokens": "iii", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
               "tb_attention_tc_tile_tokens": ""}
 
 _lock = threading.Lock()
@@ -494,6 +495,11 @@ def attention_window_mma_tile_tokens(nh: int, nkvh: int) -> int:
 
 def latent_attention_tile_tokens(heads: int) -> int:
     return library().tb_latent_attention_tile_tokens(heads)
+
+
+def latent_tc_tile_tokens(heads: int, rank: int, rot: int) -> int:
+    """Query tokens per tile of the tcgen05 latent attention (0: it does not take such heads and latents)."""
+    return library().tb_latent_tc_tile_tokens(heads, rank, rot)
 
 
 def attention_prefill_tile_tokens() -> int:

@@ -63,6 +63,18 @@ def rows_pay(lens, before, window: int, tile: int, rank: int, blocks: int) -> bo
     return shared < alone
 
 
+def tc_pays(ctx, m) -> bool:
+    """Whether a step without slices is faster on the tcgen05 tensor cores (latent_tc.cu) than with 16 or 64 rows a block: from a third
+    of the tiles' rows in use on.  us, the faster of those two and tcgen05 (rank 512 + 64, 16 heads): one prompt of 2,039
+    tokens 440 and 208, 4 of 300 88 and 43, 16 of 100 82 and 42, 40 of 16 behind 1,000 244 and 115, 200 of 6 (0.75 in use) 54 and
+    34; not taken: 420 of 2 behind 2,000 (0.25) 574 and 615.  Rank 256 + 32, 8 heads: 2,039 tokens 159 and 76, 200 of 6 (0.38) 17 and 16;
+    not taken: 420 of 2 behind 300 (0.12) 35 and 47."""
+    key = ("latent_tc", m.tc_tile)
+    if key not in ctx.plans:
+        ctx.plans[key] = 3 * ctx.nt >= ctx.tiles(m.tc_tile).count * m.tc_tile
+    return ctx.plans[key]
+
+
 @MIXERS.register("latent_attention")
 class LatentAttention(Mixer):
     """params: width, heads, dim, rot_dim, vdim, kv_rank, q_rank, window, scale, eps, own_latent, position (a
@@ -99,7 +111,9 @@ class LatentAttention(Mixer):
             raise ValueError(f"the latent attention kernel takes latents of up to 512 entries, got {self.rank}")
         self.q_head = self.dim + self.rot
         self.tile = lib.latent_attention_tile_tokens(self.H)
-        self.tile_sizes = [self.tile]
+        # bfloat16 prompts: the tcgen05 kernel's tiles, where it takes the heads and the latent
+        self.tc_tile = lib.latent_tc_tile_tokens(self.H, self.rank, self.rot) if dtype == torch.bfloat16 else 0
+        self.tile_sizes = [t for t in (self.tile, self.tc_tile) if t]
 
     @property
     def graph_safe(self) -> bool:
@@ -198,10 +212,17 @@ class LatentAttention(Mixer):
             splits = int(max(1, min(16, (min(self.window, ctx.engine.spec.max_context) + 63) // 64 + 1,
                                     (2 * ctx.engine.sm_count) // max(1, blocks))))
             partial = ctx.scratch("latent.partial", (nt, H, splits, self.rank + 2), torch.float32) if splits > 1 else None
+            if splits == 1 and self.tc_tile and not ctx.decode and tc_pays(ctx, self):
+                wide = ctx.tiles(self.tc_tile)
+                done = lib.try_call("tb_latent_attention_tc_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(ol), lib.ptr(cache.kv),
+                                    lib.ptr(wide.seq), lib.ptr(wide.t0), lib.ptr(wide.nq), lib.ptr(ctx.tok_pos), lib.ptr(table),
+                                    lib.ptr(cos), lib.ptr(sin), wide.count, nt, ctx.max_pages, ldq, self.q_head, H, self.rank,
+                                    self.rot, self.rdims, cache.kv.shape[0], self.window, self.scale, lib.ptr(sinks),
+                                    lib.ptr(gate), wa)
             plan = ("latent", self.window, self.tile, self.rank, blocks)
-            if splits == 1 and not ctx.decode and plan not in ctx.plans:
+            if splits == 1 and not done and not ctx.decode and plan not in ctx.plans:
                 ctx.plans[plan] = rows_pay(ctx.h_lens, ctx.h_pos0, *plan[1:])
-            if splits == 1 and ctx.plans.get(plan):
+            if splits == 1 and not done and ctx.plans.get(plan):
                 done = lib.try_call("tb_latent_attention_rows_bf16", lib.ptr(qa), lib.ptr(q), lib.ptr(ol), lib.ptr(cache.kv),
                                     lib.ptr(tiles.seq), lib.ptr(tiles.t0), lib.ptr(tiles.nq), lib.ptr(ctx.tok_pos),
                                     lib.ptr(table), lib.ptr(cos), lib.ptr(sin), tiles.count, nt, ctx.max_pages, ldq,
