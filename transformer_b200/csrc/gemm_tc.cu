@@ -55,6 +55,9 @@
 #define TC_MAX_STAGES 6
 #define TC_A_BYTES (TC_BM * TC_BK * 2)
 #define TC_BHALF_BYTES (TC_BN / 2 * TC_BK * 2)     // half of the B tile: all that a block of a pair stages
+#define TC_EPI_BF16 0                              // bfloat16, the (gate, up) pair among it
+#define TC_EPI_BIASED 1                            // the pair with biases
+#define TC_EPI_FLOAT 2
 #define TC_STRIP_BYTES (32 * 128)                  // an epilogue warp's strip: 32 rows x 64 bfloat16, on their way out
 
 template <int CTAS> struct TcShape {
@@ -70,7 +73,6 @@ struct TcArgs {
     int ldc, M, N, K, G;
     int b_group_rows;   // rows of B per group in the stacked view (N, or 2N when dual)
     int dual;
-    int out_float;
     int tiles_m;        // row tiles (with groups: an upper bound; tiles past the last group are skipped)
     int n_tile;         // rows of B in a tile: a multiple of 16 up to TC_BN (fewer when that fills the SMs better)
     GluRule glu;        // dual: how the (gate, up) pair becomes one value
@@ -128,14 +130,16 @@ __device__ __forceinline__ TcTile tc_tile(const TcArgs& a, const int* offsets, i
     return r;
 }
 
-template <int CTAS>
+// EPI: what the epilogue makes of the accumulator (TC_EPI_*).  Kernels of their own: with all of it in one the products that stream
+// weights for a few rows took 2 to 6 % longer (256 rows of 16 experts, (gate, up) of 688 x 4,096: 51.2 and 54.3 us).
+template <int CTAS, int EPI>
 __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                             const __grid_constant__ CUtensorMap map_b,
                                                             const TcArgs a) {
     pdl_sync();
     extern __shared__ uint8_t smem_raw[];
     constexpr int TC_STAGES = TcShape<CTAS>::STAGES, TC_STAGE_BYTES = TcShape<CTAS>::STAGE_BYTES;
-    constexpr bool PAIR = CTAS == 2;
+    constexpr bool PAIR = CTAS == 2, BIASED = EPI == TC_EPI_BIASED, FLOAT = EPI == TC_EPI_FLOAT;
     __shared__ __align__(8) uint64_t bars[2 * TC_MAX_STAGES + 4];
     __shared__ uint32_t tmem_slot;
     __shared__ int group_rows[TC_SHARED_GROUPS + 1];
@@ -268,8 +272,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         const int row = quad * 32 + lane;
         // results whose rows start on 16-byte boundaries leave through this warp's strip of shared memory
         uint8_t* strip = smem_raw + (smem_base - smem_u32(smem_raw)) + TC_STAGES * TC_STAGE_BYTES + (warp - 2) * TC_STRIP_BYTES;
-        const bool wide = !a.out_float && a.N % 8 == 0 && a.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
-        const bool wide_float = a.out_float && a.N % 4 == 0 && a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
+        const bool wide = !FLOAT && a.N % 8 == 0 && a.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
+        const bool wide_float = FLOAT && a.N % 4 == 0 && a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0;
         bool ok = true;
         int lt = 0;
         for (int t = pair; t < total && ok; t += pairs) {
@@ -288,14 +292,14 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 if (((c0 >> 6) & 1) != piece) continue;
                 float v[32];
                 tmem_ld32(trow + c0, v);               // warp-collective: every lane takes part
-                if (a.dual) {
+                if (!FLOAT && a.dual) {
                     float u[32];
                     tmem_ld32(trow + a.n_tile / 2 + c0, u);
                     // silu(g) * u = g * u / (1 + e^-g) in float, with the hardware's exponential and division
                     // (2 ulp; the result is rounded to bfloat16 next).  The exact forms cost some hundred clocks
                     // per value with only these four warps on the SM to hide them: measured, the epilogue of a tile
                     // took 7 to 18 us, as long as streaming half of the tile's weights.
-                    if (a.glu.bias) {
+                    if constexpr (BIASED) {
                         const float* bg = a.glu.bias + n0 + c0;
                         const int last = a.N - 1 - n0 - c0;           // columns past the last are computed and not stored
 #pragma unroll
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                         for (int i = 0; i < 32; ++i) v[i] = glu_apply_fast(v[i], u[i], a.glu);
                     }
                 }
-                if (wide) {
+                if (!FLOAT && wide) {
                     // A lane holds 32 columns of ONE row: stored from here, every instruction of the warp would touch
                     // 32 lines of memory.  So the warp passes two such chunks through its strip of shared memory
                     // (32 rows x 128 bytes; the 16-byte pieces of a row are XOR-swizzled by the row, so that neither
@@ -346,7 +350,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     }
                     continue;
                 }
-                if (wide_float) {
+                if (FLOAT && wide_float) {
                     // the same for floats: a chunk's 32 columns are a whole line.  (Logits of 1,000 rows, K 2,048, N 32,000: 290 us
                     // row by row, 150 so.)
 #pragma unroll
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 }
                 const int c_end = min(n_out - c0, a.N - n0 - c0);   // columns of this chunk that exist (may be <= 0)
                 if (m < tl.row_end && c_end > 0) {
-                    if (a.out_float) {
+                    if constexpr (FLOAT) {
                         float* dst = static_cast<float*>(a.C) + (size_t)m * a.ldc + n0 + c0;
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
@@ -380,7 +384,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     }
                 }
             }
-            if (a.glu.fill && piece == 0 && n0 + n_out >= a.N && m < tl.row_end) {
+            if (BIASED && a.glu.fill && piece == 0 && n0 + n_out >= a.N && m < tl.row_end) {
                 __nv_bfloat16* pad = static_cast<__nv_bfloat16*>(a.C) + (size_t)m * a.ldc + a.N;
                 for (int e = 0; e < a.glu.fill; ++e) pad[e] = __float2bfloat16_rn(e == 0 ? 1.f : 0.f);
             }
@@ -472,12 +476,12 @@ int* tc_error_ptr() {
     return p;
 }
 
-template <int CTAS>
+template <int CTAS, int EPI>
 static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, TcArgs a, cudaStream_t s) {
     const size_t smem = (size_t)TcShape<CTAS>::STAGES * TcShape<CTAS>::STAGE_BYTES + TC_EPI_WARPS * TC_STRIP_BYTES + 1024;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<CTAS, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -505,7 +509,7 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, TcArgs a, cud
             int n = 0;
             cfg.gridDim = dim3(sms > 1 ? sms / 2 * 2 : 2);
             cfg.numAttrs = 2;
-            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<CTAS>, &cfg);
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_kernel<CTAS, EPI>, &cfg);
             if (e != cudaSuccess) {
                 cudaGetLastError();
                 max_units = 0;                 // asked again at the next launch
@@ -522,8 +526,8 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, TcArgs a, cud
     const int units = total < max_units ? total : max_units;
     cfg.gridDim = dim3(CTAS * units);
     cfg.numAttrs = CTAS == 2 ? 2 : 1;
-    tb_state_carveout((const void*)gemm_tc_kernel<CTAS>, TC_THREADS, smem);
-    cudaLaunchKernelEx(&cfg, gemm_tc_kernel<CTAS>, ma, mb, a);
+    tb_state_carveout((const void*)gemm_tc_kernel<CTAS, EPI>, TC_THREADS, smem);
+    cudaLaunchKernelEx(&cfg, gemm_tc_kernel<CTAS, EPI>, ma, mb, a);
     return tb_last_error();
 }
 
@@ -582,9 +586,14 @@ static int gemm_tc_entry(const void* A, const void* B, void* C, const int* group
     // and what counts is how few bytes its start needs.  With K = 4,096 both forms measure the same, and with wide
     // experts (K or N of 14,336) the single blocks are 4..20 % faster (1.41 against 1.18 PFLOP/s at 2,048 rows).
     const bool pair = (long long)M >= 1024ll * G && K < 2048;
-    TcArgs a{C, group_offsets, err_ptr, ldc, M, N, K, G, rows_b, dual, out_kind == 1, 0, n_tile, glu};
-    rc = pair ? tc_launch<2>(ma, mb, a, s) : tc_launch<1>(ma, mb, a, s);
-    if (pair && rc == TB_ERR_UNSUPPORTED) rc = tc_launch<1>(ma, mb, a, s);
+    TcArgs a{C, group_offsets, err_ptr, ldc, M, N, K, G, rows_b, dual, 0, n_tile, glu};
+    if (glu.bias) return tc_launch<1, TC_EPI_BIASED>(ma, mb, a, s);
+    if (out_kind == 1) {
+        rc = pair ? tc_launch<2, TC_EPI_FLOAT>(ma, mb, a, s) : TB_ERR_UNSUPPORTED;
+        return rc == TB_ERR_UNSUPPORTED ? tc_launch<1, TC_EPI_FLOAT>(ma, mb, a, s) : rc;
+    }
+    rc = pair ? tc_launch<2, TC_EPI_BF16>(ma, mb, a, s) : TB_ERR_UNSUPPORTED;
+    if (rc == TB_ERR_UNSUPPORTED) rc = tc_launch<1, TC_EPI_BF16>(ma, mb, a, s);
     return rc;
 }
 
