@@ -55,6 +55,10 @@ struct SkinnyArgs {
     // looks at the rows before its own one by one, so with more rows it turns: 32 rows 35.4 to 37.8, 64 51 to 69.
     int by_row;
     GluRule glu;            // DUAL: how the (gate, up) pair becomes one value
+    // One weight matrix with short rows (K < 2,048): what a thread's registers do not take before the wait is asked into L2.  Steps of one
+    // sequence of width 1,024, 8 layers, vocabulary 32,000: 1,042 to 1,018 us for four.  Longer rows lose: K 4,096, 32 layers of one
+    // sequence +3 % (the kernel before still reads from memory).
+    int ahead;
 };
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
@@ -131,6 +135,14 @@ __global__ void __launch_bounds__(WK * WN * 32) gemm_skinny_kernel(const SkinnyA
                 ua[u] = live ? ld16w(u0 + k) : zero4;
                 ub[u] = live ? ld16w(u1 + k) : zero4;
             }
+        }
+    }
+    if (a.ahead && warp == 0) {
+        // the rest of the block's weights comes into L2 meanwhile
+        constexpr int R = SK_COLS * WN * NMAT, K0 = UNR * WK * 32;
+        for (int r = lane; r < R && K0 < a.K; r += 32) {
+            const int c = min((int)blockIdx.x * WN * SK_COLS + r % (SK_COLS * WN), a.N - 1) + (r >= SK_COLS * WN ? a.N : 0);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(Wg + (size_t)c * a.ldw + K0), "r"((a.K - K0) * 2) : "memory");
         }
     }
     pdl_sync();
@@ -352,7 +364,8 @@ static int skinny_entry(const void* X, const int* x_rows, const void* W, void* Y
     if (((uintptr_t)X | (uintptr_t)W) & 15) return TB_ERR_UNSUPPORTED;
     if (M == 0) return 0;
     SkinnyArgs a{(const __nv_bfloat16*)X, x_rows, (const __nv_bfloat16*)W, Y, group_offsets, w_group_stride,
-                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, row_group && G >= 16 && 4 * M <= G && M <= 16, glu};
+                 ldx, ldw, ldy, M, N, K, G, row_group, x_div, w_constant, row_group && G >= 16 && 4 * M <= G && M <= 16, glu,
+                 G == 1 && !row_group && !group_offsets && w_constant && K < 2048};
     int rows = (max_group_rows > 0 && max_group_rows < M) ? max_group_rows : M;
     if (G > 1) {
         // A pass takes 8, 16 or 32 rows of a group and a thread's registers are sized by the pass (with 16 rows the
