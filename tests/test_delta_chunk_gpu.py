@@ -110,3 +110,35 @@ def test_chunks(dtype, G, H, dim, vdim, per_head, steep):
         row = state[int(slots[i])].cpu().double()
         assert float((row[:H * dim * vdim].view(H, dim, vdim) - S).abs().max()) <= 1e-5 * (float(S.abs().max()) + 1.0)
         assert torch.equal(row[H * dim * vdim:].view(3, C), x[i][-3:].double())
+
+
+@pytest.mark.parametrize("H,vdim,copies", [(4, 128, 5), (3, 32, 25), (3, 48, 17), (1, 256, 9), (1, 256, 10)])
+def test_scan_of_many_columns(H, vdim, copies):
+    """More blocks of 16 columns than SMs, where the scan takes 32 columns a block (not with 48), and just fewer (9 x 256): lengths
+    around a chunk's edges and an empty sequence.  The bound is that of `test_chunks`."""
+    from transformer_b200.csrc import lib
+    gen, dim = torch.Generator().manual_seed(vdim + copies), 128
+    lens = [(1, 15, 0, 16, 33, 50, 17)[i % 7] for i in range(copies)]
+    B, nt, C = copies, sum(lens), 2 * H * dim + H * vdim
+    x, a, bz = torch.randn(nt, C, generator=gen), torch.randn(nt, H * dim, generator=gen) * 3, torch.randn(nt, H, generator=gen) * 2
+    conv, bias, A_log = torch.randn(C, 4, generator=gen) * 0.6, torch.randn(H * dim, generator=gen) - 1, torch.rand(H, generator=gen) * 3 - 2.5
+    state, slots = torch.zeros(B, lib.delta_state_size(H, H, dim, vdim, 4)).cuda(), torch.arange(B).flip(0).int().cuda()
+    d = [t.cuda() for t in (x, conv, a, bias, A_log, bz, torch.tensor([0] + lens).cumsum(0).int())]
+    chunks = nt // 16 + B
+    rec = torch.full((H, chunks, lib.delta_chunk_record_size(dim, vdim, 4)), float("nan"), device="cuda")
+    o = torch.full((nt, H, vdim), float("nan"), device="cuda")
+    where = (lib.ptr(d[6]), lib.ptr(slots), nt, B, H, H, dim, vdim, 4, chunks)
+    lib.call("tb_delta_chunk_f32", lib.ptr(d[0]), C, lib.ptr(d[1]), lib.ptr(state), *(lib.ptr(t) for t in d[2:6]), lib.ptr(rec), *where,
+             H * dim, H, 0)
+    lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where)
+    got = o.cpu().double().split(lens)
+    assert not lib.library().tb_gemm_tc_status()
+    for i, (xi, ai, bi) in enumerate(zip(x.split(lens), a.split(lens), bz.split(lens))):
+        if not lens[i]:
+            continue
+        decay = torch.exp(-torch.exp(A_log.double())[None, :, None] *
+                          torch.nn.functional.softplus(ai.double() + bias.double()).view(lens[i], H, dim))
+        want, S = _plain(xi.double(), conv.double(), decay, torch.sigmoid(bi.double()), H, H, dim, vdim)
+        assert float((got[i] - want).abs().max()) <= 1e-5 * (float(want.abs().max()) + 1.0)
+        row = state[B - 1 - i].cpu().double()[:H * dim * vdim].view(H, dim, vdim)
+        assert float((row - S).abs().max()) <= 1e-5 * (float(S.abs().max()) + 1.0)

@@ -11,13 +11,14 @@
 //
 //   delta_chunk_kernel        a block = a chunk x a head: convolution, silu, unit norms, decays, A and B, the two
 //                             solutions, one record for the scan
-//   delta_chunk_scan_kernel   a block = a sequence x a head x 16 columns of S
+//   delta_chunk_scan_kernel   a block = a sequence x a head x 16 or 32 columns of S
 // Measured with 16 heads of 128 x 128 (both kernels; before: records and scan token by token): one prompt of 2,048 tokens
-// 294 us (812), two of 1,500 358 (837), eight of 1,024 848 (1,770).  The first kernel is bound by instruction issue
-// and shared-memory reads in equal parts (47 % and 43 % of their rates, 34 KB and 64 registers a thread leave four blocks
-// an SM); the scan of few sequences by the chain of a chunk (1.5 us; one block an SM, a third of the issue slots), that of
-// many by shared-memory reads: four columns of four rows a thread use a record's entry four times, 504 us for eight
-// prompts where two columns of eight rows took 611.
+// 329 us (812), two of 1,500 353 (837), eight of 1,024 777 (1,770).  The first kernel is bound by instruction issue
+// and shared-memory reads in equal parts (34 KB and 64 registers a thread leave four blocks an SM); a warp leaves out the
+// tokens before its first key (136 to 128 us for two prompts of 1,500 tokens).  The scan of few sequences is bound by the
+// chain of a chunk (1.8 us; one block an SM), that of many by what goes through shared memory: a piece of a record that a
+// lane loads serves its four columns, and 16 lanes to a column instead of 32 halve the exchange of the sums: eight
+// prompts 451 us (569 with 32 lanes), four of 600 142 (191), two of 1,500 226 (234).  Eight lanes to a column: 481 and 163.
 #include "channel_delta.cuh"
 #include "memory_common.cuh"            // fma2, mul2
 #include "tc_common.cuh"                // bulk copies, barriers with bounded waits
@@ -27,6 +28,7 @@
 #define DC_BP 20            // pitch of B's rows: the 16 lanes that read a row each start in different banks
 #define DC_COLS 16          // columns of the state per scan block
 #define DC_STAGES 3
+#define DC_SMS 148          // of a B200
 
 // A record of one (head, chunk):  W | G q | G_last / G_j k, [16][dim] each | G_last [dim] | B [16][DC_BP], then
 // U0 as [vdim / 16][16 tokens][16 columns], so that a scan block's share is one piece.
@@ -130,13 +132,14 @@ __global__ void __launch_bounds__(256, 4) delta_chunk_kernel(const DeltaPrepArgs
     // the 16 ends with row i
     {
         constexpr int R4 = DIM / 64;
-        const int j = tid >> 4, part = tid & 15;
+        const int j = tid >> 4, part = tid & 15, first = __shfl_sync(0xffffffffu, j, 0);     // no key of the warp is there earlier
         float kt[R4 * 4], s[2 * DC_TOK];
 #pragma unroll
         for (int e = 0; e < R4 * 4; ++e) kt[e] = 0.f;
 #pragma unroll
         for (int i = 0; i < DC_TOK; ++i) {
             float sa = 0.f, sb = 0.f;
+            if (i >= first)
 #pragma unroll
             for (int r = 0; r < R4; ++r) {
                 const int c = i * DIM + r * 64 + part * 4;
@@ -214,20 +217,22 @@ struct DeltaChunkScanArgs {
 
 // 128 threads: LANES lanes share C columns and split the rows (DIM / LANES each, in registers, pieces of four
 // interleaved).  Per chunk: the sums over S for W and G q (16 tokens x C columns each), scattered so that every lane ends
-// with one token's two columns; u through shared memory to all lanes of the columns; the update.  The records come by
-// bulk copy, two chunks ahead, with bounded waits.
+// with one token's sums for C or, of 32 lanes, C / 2 columns; u through shared memory to all lanes of the columns; the
+// update.  A lane takes the tokens in an order of its own (place t holds token t ^ its number), so the half that it gives
+// away is at the same places in every lane and nothing is selected.  The records come by bulk copy, two chunks ahead,
+// with bounded waits.
 template <int DIM, int LANES, int C>
 __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkScanArgs a) {
     pdl_sync();
-    constexpr int R4 = DIM / (4 * LANES), NV = DC_TOK * C;
-    static_assert(NV == 2 * LANES && 128 / LANES * C == DC_COLS && R4 * 4 * LANES == DIM, "a lane ends with two sums");
-    constexpr int MAIN = (3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP, STAGE = MAIN + DC_TOK * DC_COLS;
+    constexpr int R4 = DIM / (4 * LANES), CB = LANES / DC_TOK, OUT = C / CB, COLS = 128 / LANES * C;
+    static_assert((CB == 1 || CB == 2) && OUT % 2 == 0 && COLS % DC_COLS == 0 && R4 * 4 * LANES == DIM, "a lane ends with a token's sums");
+    constexpr int MAIN = (3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP, STAGE = MAIN + DC_TOK * COLS;
     extern __shared__ __align__(16) float dc_sm[];          // [DC_STAGES][STAGE]
-    __shared__ __align__(16) float us[DC_COLS / C][DC_TOK][C];
+    __shared__ __align__(16) float us[COLS / C][DC_TOK][C];
     __shared__ __align__(8) unsigned long long bars[DC_STAGES];
     const int b = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
-    const int part = tid & (LANES - 1), group = tid / LANES, col = blockIdx.z * DC_COLS + group * C;
-    const int my_tok = part * 2 / C, my_col = part * 2 % C;     // whose two sums this lane ends with
+    const int part = tid & (LANES - 1), group = tid / LANES, col = blockIdx.z * COLS + group * C;
+    const int my_tok = part / CB, my_col = part % CB * OUT;     // whose sums this lane ends with
     const int H = a.H, vdim = a.vdim;
     const int t0 = a.seq_start[b], n_tok = a.seq_start[b + 1] - t0;
     if (n_tok <= 0) return;
@@ -261,19 +266,20 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
         const float* from = rec + (size_t)ch * rec_floats;
         mbar_expect_tx(bar, STAGE * sizeof(float));
         bulk_load(to, from, MAIN * sizeof(float), bar);
-        bulk_load(to + MAIN * sizeof(float), from + MAIN + (size_t)blockIdx.z * (DC_TOK * DC_COLS),
-                  DC_TOK * DC_COLS * sizeof(float), bar);
+        bulk_load(to + MAIN * sizeof(float), from + MAIN + (size_t)blockIdx.z * (DC_TOK * COLS), DC_TOK * COLS * sizeof(float), bar);
     };
     union Four { float4 f; F2 p[2]; };
-    // this lane's part of the sums over S for 16 rows of a record, then the lane's two sums
-    auto sums = [&](const float* rows, float (&sum)[NV]) {
+    // this lane's part of the sums over S for 16 rows of a record, then the lane's own sums
+    auto sums = [&](const float* rows, float (&mine)[OUT]) {
+        F2 sum[DC_TOK][C / 2];
 #pragma unroll
         for (int t = 0; t < DC_TOK; ++t) {
+            const float* row = rows + (t ^ my_tok) * DIM + part * 4;
             F2 acc[C];
 #pragma unroll
             for (int r = 0; r < R4; ++r) {
                 Four w;
-                w.f = *reinterpret_cast<const float4*>(rows + t * DIM + r * (4 * LANES) + part * 4);
+                w.f = *reinterpret_cast<const float4*>(row + r * (4 * LANES));
 #pragma unroll
                 for (int c = 0; c < C; ++c)
 #pragma unroll
@@ -281,18 +287,31 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
                         acc[c] = r == 0 && e == 0 ? mul2(w.p[e], s[c][r * 2 + e]) : fma2(w.p[e], s[c][r * 2 + e], acc[c]);
             }
 #pragma unroll
-            for (int c = 0; c < C; ++c) sum[t * C + c] = acc[c].f.x + acc[c].f.y;
+            for (int c = 0; c < C; c += 2) sum[t][c / 2].f = make_float2(acc[c].f.x + acc[c].f.y, acc[c + 1].f.x + acc[c + 1].f.y);
         }
-    };
-    auto scatter = [&](float (&sum)[NV]) {
 #pragma unroll
-        for (int half = LANES / 2; half > 0; half >>= 1) {
-            const bool up = part & half;
+        for (int half = DC_TOK / 2; half > 0; half >>= 1)
 #pragma unroll
-            for (int i = 0; i < 2 * half; ++i) {
-                const float keep = up ? sum[i + 2 * half] : sum[i], give = up ? sum[i] : sum[i + 2 * half];
-                sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+            for (int t = 0; t < half; ++t)
+#pragma unroll
+                for (int c = 0; c < C / 2; ++c) {
+                    F2 in;
+                    in.f.x = __shfl_xor_sync(0xffffffffu, sum[t + half][c].f.x, half * CB);
+                    in.f.y = __shfl_xor_sync(0xffffffffu, sum[t + half][c].f.y, half * CB);
+                    sum[t][c] = add2(sum[t][c], in);
+                }
+#pragma unroll
+        for (int c = 0; c < OUT / 2; ++c) {
+            F2 keep = sum[0][c];
+            if (CB == 2) {
+                const F2 give = my_col ? keep : sum[0][c + OUT / 2];
+                F2 in;
+                in.f.x = __shfl_xor_sync(0xffffffffu, give.f.x, 1);
+                in.f.y = __shfl_xor_sync(0xffffffffu, give.f.y, 1);
+                keep = add2(my_col ? sum[0][c + OUT / 2] : keep, in);
             }
+            mine[2 * c] = keep.f.x;
+            mine[2 * c + 1] = keep.f.y;
         }
     };
     int issued = 0;
@@ -308,16 +327,17 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
         if (issued < chunks) issue(issued++);
         const float* W = dc_sm + (size_t)(ch % DC_STAGES) * STAGE;
         const float* G = W + 3 * DC_TOK * DIM;
-        float su[NV], so[NV];                               // [token][column]
+        float su[OUT], o[OUT];
         sums(W, su);
-        scatter(su);
-        const float2 u0 = *reinterpret_cast<const float2*>(W + MAIN + my_tok * DC_COLS + group * C + my_col);
-        *reinterpret_cast<float2*>(&us[group][my_tok][my_col]) = make_float2(u0.x - su[0], u0.y - su[1]);
-        sums(W + DC_TOK * DIM, so);
+        const int lc = group * C + my_col;
+        const float* u0 = W + MAIN + lc / DC_COLS * (DC_TOK * DC_COLS) + my_tok * DC_COLS + lc % DC_COLS;
+#pragma unroll
+        for (int c = 0; c < OUT; c += 2) {
+            const float2 x = *reinterpret_cast<const float2*>(u0 + c);
+            *reinterpret_cast<float2*>(&us[group][my_tok][my_col + c]) = make_float2(x.x - su[c], x.y - su[c + 1]);
+        }
+        sums(W + DC_TOK * DIM, o);
         __syncwarp();           // the lanes of a group of columns are lanes of one warp
-        scatter(so);
-        F2 o;
-        o.f = make_float2(so[0], so[1]);
 #pragma unroll
         for (int r = 0; r < R4; ++r) {
             Four gl;
@@ -335,33 +355,35 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
             for (int e4 = 0; e4 < 4; ++e4) {
                 const int j = j4 * 4 + e4;
                 float u[C];
-#pragma unroll
-                for (int c = 0; c < C; c += 2) {
-                    const float2 x = *reinterpret_cast<const float2*>(&us[group][j][c]);
-                    u[c] = x.x;
-                    u[c + 1] = x.y;
+                if constexpr (C == 4) {
+                    *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(us[group][j]);
+                } else {
+                    *reinterpret_cast<float2*>(u) = *reinterpret_cast<const float2*>(us[group][j]);
                 }
-                F2 mine, bd;
-                mine.f = my_col ? make_float2(u[C - 2], u[C - 1]) : make_float2(u[0], u[1]);
-                bd.f = make_float2(bj[e4], bj[e4]);
                 // B is zero for later tokens, but a later token's u may be no number, and that is not this one's affair
-                if (j <= my_tok) o = fma2(bd, mine, o);
+                if (j <= my_tok)
+#pragma unroll
+                    for (int c = 0; c < OUT; ++c) o[c] = __fmaf_rn(bj[e4], CB == 2 && my_col ? u[C - OUT + c] : u[c], o[c]);
 #pragma unroll
                 for (int r = 0; r < R4; ++r) {
                     Four kd;
                     kd.f = *reinterpret_cast<const float4*>(W + (2 * DC_TOK + j) * DIM + r * (4 * LANES) + part * 4);
 #pragma unroll
-                    for (int c = 0; c < C; ++c) {
-                        F2 ub;
-                        ub.f = make_float2(u[c], u[c]);
+                    for (int c = 0; c < C; ++c)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) s[c][r * 2 + e] = fma2(kd.p[e], ub, s[c][r * 2 + e]);
-                    }
+                        for (int e = 0; e < 2; ++e) {
+                            F2 ub;
+                            ub.f = make_float2(u[c], u[c]);
+                            s[c][r * 2 + e] = fma2(kd.p[e], ub, s[c][r * 2 + e]);
+                        }
                 }
             }
         }
         const int t = ch * DC_TOK + my_tok;
-        if (t < n_tok) *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + t) * H + h) * vdim + col + my_col) = o.f;
+        if (t < n_tok)
+#pragma unroll
+            for (int c = 0; c < OUT; c += 2)
+                *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + t) * H + h) * vdim + col + my_col + c) = make_float2(o[c], o[c + 1]);
     }
 #pragma unroll
     for (int i = 0; i < R4 * 2; ++i) {
@@ -391,11 +413,12 @@ static int delta_chunk_go(const DeltaPrepArgs& p, int nt, int B, int max_chunks,
 
 template <int DIM, int LANES, int C>
 static int delta_chunk_scan_go(const DeltaChunkScanArgs& a, int B, cudaStream_t s) {
-    constexpr size_t smem = (size_t)DC_STAGES * ((3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP + DC_TOK * DC_COLS) * sizeof(float);
+    constexpr int COLS = 128 / LANES * C;
+    constexpr size_t smem = (size_t)DC_STAGES * ((3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP + DC_TOK * COLS) * sizeof(float);
     static PerDevice raised;
     tb_allow_smem(raised, (const void*)delta_chunk_scan_kernel<DIM, LANES, C>, smem);
     // the blocks run for the whole sequence and want an SM each (see tb_launch_plain)
-    tb_launch_plain(delta_chunk_scan_kernel<DIM, LANES, C>, dim3(B, a.H, a.vdim / DC_COLS), dim3(128), smem, s, a);
+    tb_launch_plain(delta_chunk_scan_kernel<DIM, LANES, C>, dim3(B, a.H, a.vdim / COLS), dim3(128), smem, s, a);
     return tb_last_error();
 }
 
@@ -439,7 +462,10 @@ int tb_delta_chunk_scan(const float* rec, float* state, float* out, const int* s
     if (per % 2) return TB_ERR_ARG;
     DeltaChunkScanArgs a{rec, state, tc_error_ptr(), out, seq_start, slots, per, max_chunks, H, vdim};
     if (!a.error) return tb_last_error();
-    return dim == 64 ? delta_chunk_scan_go<64, 16, 2>(a, B, s) : delta_chunk_scan_go<128, 32, 4>(a, B, s);
+    if (dim == 64) return delta_chunk_scan_go<64, 16, 2>(a, B, s);
+    // More than one block an SM: blocks of 32 columns.  Fewer leave SMs without one (one prompt of 2,048 tokens: 304 us, 237 so).
+    if (vdim % 32 == 0 && (long long)B * H * (vdim / DC_COLS) > DC_SMS) return delta_chunk_scan_go<128, 16, 4>(a, B, s);
+    return delta_chunk_scan_go<128, 32, 4>(a, B, s);
 }
 }
 

@@ -55,6 +55,11 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.u) : "l"(a.u), "l"(b.u), "l"(c.u));
     return d;
 }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
+    return d;
+}
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
     F2 d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
