@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(WK * WN * 32) gemm_skinny_kernel(const SkinnyA
             }
         }
     }
-    if (a.ahead && warp == 0) {
-        // the rest of the block's weights comes into L2 meanwhile
+    if (WK < 8 && a.ahead && warp == 0) {
+        // the rest of the block's weights comes into L2 meanwhile (WK < 8: the shapes for K < 2,048)
         constexpr int R = SK_COLS * WN * NMAT, K0 = UNR * WK * 32;
         for (int r = lane; r < R && K0 < a.K; r += 32) {
             const int c = min((int)blockIdx.x * WN * SK_COLS + r % (SK_COLS * WN), a.N - 1) + (r >= SK_COLS * WN ? a.N : 0);

@@ -8,11 +8,8 @@
 //     one tcgen05.mma issued by the leader reads both blocks' operands and writes rows 0..127 of the product
 //     into the leader's tensor memory and rows 128..255 into the other's.  Per block and k-block that is 32 KB
 //     from L2 for 128 x 256 x 64 of product instead of 48 KB, and six ring stages fit instead of four.
-//     Measured when it went in: 1.61 against 1.53 PFLOP/s on 8192 x 4096 x 4096 and +7 % on experts with 2,048 rows
-//     each; with few rows per group the 256-row tiles are mostly padding and there are half as many work items
-//     (decoding at batch 64: -7 %).  Since the tiles of a group are numbered with its row tiles innermost (tc_tile)
-//     the single blocks share their B tiles through L2 just as well, and the launcher takes pairs only from 1,024
-//     rows per group on and for a short K (see tb_gemm_tc_bf16);
+//     With few rows per group the 256-row tiles are mostly padding and there are half as many work items (decoding at
+//     batch 64: -7 %); the launcher goes by the rounds either form takes (see gemm_tc_entry, with the measurements);
 //   * operands are staged by TMA (cp.async.bulk.tensor, 128-byte swizzle) into a ring of TC_STAGES stages;
 //     with pairs, both blocks' copies are counted on the LEADER's barrier of the stage;
 //   * tcgen05.commit (with pairs: multicast to both blocks) hands a finished stage back to the TMA warps and, after
@@ -160,7 +157,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         offsets = group_rows;        // visible to all after the block-wide barrier below
     }
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = PAIR ? warp_number() : (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0;  // 0 leads the pair
     const int pair = blockIdx.x / CTAS, pairs = gridDim.x / CTAS;     // this unit of work and how many there are
     const int n_out = a.dual ? a.n_tile / 2 : a.n_tile; // output columns of a tile
@@ -197,9 +194,12 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
 
+    // Pairs: these two loops are the whole warp's, and one elected lane issues (see elect_one).  As one thread's loops they cost the down
+    // product of 16 experts at 2,048 rows each 163 us for 156; single blocks are 1 to 2 % faster with a thread's loops.
+    auto agreed = [&](bool ok) { return PAIR ? (bool)__all_sync(0xffffffffu, ok) : ok; };
     if (warp == 0) {
         // ---------------- TMA producer (both blocks; bytes are counted on the leader's barrier) ----------------
-        if (lane == 0) {
+        if (PAIR || lane == 0) {
             bool ok = true;
             int it = 0;                       // k-blocks handed to the ring so far, over all tiles
             int s = 0;                        // its stage, and the parity of the stage's last use:
@@ -210,15 +210,18 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 const int a_row = tl.row0 + (int)rank * TC_BM;
                 const int b_row = tl.g * a.b_group_rows + tl.n0 + (int)rank * (a.dual ? a.N : a.n_tile / 2);
                 for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
-                    if (it >= TC_STAGES) ok = mbar_wait(empty_bar(s), used, a.error, 1);
+                    if (it >= TC_STAGES) ok = agreed(mbar_wait(empty_bar(s), used, a.error, 1));
                     if (!ok) break;
                     const uint32_t sa = smem_base + s * TC_STAGE_BYTES, sb = sa + TC_A_BYTES;
-                    if (rank == 0) mbar_expect_tx(full_bar(s), CTAS * stage_tx);
                     if (PAIR) {
                         const uint32_t counted = mapa_shared(full_bar(s), 0);
-                        tma_load_2d_pair(sa, &map_a, counted, kb * TC_BK, a_row);
-                        tma_load_2d_pair(sb, &map_b, counted, kb * TC_BK, b_row);
+                        if (elect_one()) {
+                            if (rank == 0) mbar_expect_tx(full_bar(s), CTAS * stage_tx);
+                            tma_load_2d_pair(sa, &map_a, counted, kb * TC_BK, a_row);
+                            tma_load_2d_pair(sb, &map_b, counted, kb * TC_BK, b_row);
+                        }
                     } else {
+                        mbar_expect_tx(full_bar(s), CTAS * stage_tx);
                         tma_load_2d(sa, &map_a, full_bar(s), kb * TC_BK, a_row);
                         tma_load_2d(sb, &map_b, full_bar(s), kb * TC_BK, b_row);
                         tma_load_2d(sb + half_bytes, &map_b, full_bar(s), kb * TC_BK,
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: the leader's one thread, for the pair ----------------
-        if (lane == 0 && rank == 0) {
+        if ((PAIR || lane == 0) && rank == 0) {
             const uint32_t idesc = umma_idesc(TcShape<CTAS>::ROWS, a.n_tile);
             bool ok = true;
             int lt = 0;                       // tiles done by this unit
@@ -248,31 +251,33 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 const TcTile tl = tc_tile(a, offsets, t, tiles_n, n_out, TcShape<CTAS>::ROWS);
                 if (!tl.valid) continue;
                 const int buf = lt & 1;
-                if (lt >= 2) ok = mbar_wait(acc_empty(buf), ((lt >> 1) - 1) & 1, a.error, 5);   // drained two tiles ago
+                if (lt >= 2) ok = agreed(mbar_wait(acc_empty(buf), ((lt >> 1) - 1) & 1, a.error, 5));   // drained two tiles ago
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + buf * TC_BN;
                 for (int kb = 0; kb < nkb && ok; ++kb) {
-                    ok = mbar_wait(full_bar(s), use, a.error, 2);
+                    ok = agreed(mbar_wait(full_bar(s), use, a.error, 2));
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t sa = smem_base + s * TC_STAGE_BYTES, sb = sa + TC_A_BYTES;
                     const uint64_t da = umma_desc(sa), db = umma_desc(sb);
+                    if (!PAIR || elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)   // 16 bfloat16 = 32 bytes further along K: +2 in units of 16 bytes
-                        if (PAIR) umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                        else umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-                    // the stage is free (in both blocks) once these MMAs have read it
-                    if (PAIR) umma_commit_pair(empty_bar(s), 3);
-                    else umma_commit(empty_bar(s));
+                        for (int k = 0; k < TC_BK / 16; ++k)   // 16 bfloat16 = 32 bytes further along K: +2 in units of 16 bytes
+                            if (PAIR) umma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                            else umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+                        // the stage is free (in both blocks) once these MMAs have read it
+                        if (PAIR) umma_commit_pair(empty_bar(s), 3);
+                        else umma_commit(empty_bar(s));
+                    }
                     if (++s == TC_STAGES) {
                         s = 0;
                         use ^= 1;
                     }
                 }
                 // the accumulator is complete (or abandoned), in both blocks
-                if (PAIR) umma_commit_pair(acc_full(buf), 3);
-                else umma_commit(acc_full(buf));
+                if (!PAIR) umma_commit(acc_full(buf));
+                else if (elect_one()) umma_commit_pair(acc_full(buf), 3);
                 ++lt;
             }
         }
@@ -542,6 +547,17 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, TcArgs a, cud
     return tb_last_error();
 }
 
+static int tc_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (sms < 2) sms = 2;
+    }
+    return sms;
+}
+
 // C[m] = A[m] . B[g(m)]^T.  A [M, K] (rows sorted by group), B [G, rows_b, K] with rows_b = N (or 2N when
 // out_kind == 2: gate rows then up rows).  out_kind: 0 bfloat16, 1 float, 2 swiglu (bfloat16).
 // Refuses (TB_ERR_UNSUPPORTED) what TMA cannot address: K or a pitch that is no multiple of 8,
@@ -556,24 +572,31 @@ static int gemm_tc_entry(const void* A, const void* B, void* C, const int* group
     const int rows_b = dual ? 2 * N : N;
     // Rows of B per tile: as many column tiles as the full width would need, but of equal widths (N = 688 with
     // swiglu: six tiles of 120 gate and 120 up rows instead of five of 128 and one of 48 padded to 128).
+    const int sms = tc_sms(), out_max = dual ? TC_BN / 2 : TC_BN, tiles_n = (N + out_max - 1) / out_max;
+    // Pairs of blocks, where their rounds over the SMs are not too many more than the single blocks' (a round of theirs takes 7/8 of the
+    // time: B is staged once for 256 rows), counting half a tile of padding a group.  What one round holds starts 2 us earlier in single
+    // blocks, and with a short K that start counts up to 512 rows a group.  Single blocks / pairs, us:
+    //   (gate, up) 5,632 wide, K 2,048: 520 rows 39.8 / 34.8, 1,000 51 / 45, 2,048 78 / 68, 3,451 124 / 109; 300 rows 28.7 / 33.7 (1 round, 2)
+    //   logits of 32,000 tokens, K 2,048: 200 rows 62 / 46, 500 100 / 72, 1,000 174 / 118; 64 rows 41 / 44
+    //   16 experts, (gate, up) 688 wide, K 4,096: 200 rows each 74 / 66, 384 96 / 84, 512 96 / 104 (3 rounds, 4), 1,024 166 / 148
+    //   their down product (4,096 wide, K 688): 512 rows each 64 / 59, 1,024 104 / 92, 2,048 197 / 163; 2,048 wide, K 704: 384 31 / 33
+    bool pair = false;
+    if (M > TC_BM * (long long)G && (K >= 1024 || M >= 512ll * G)) {
+        const long long pad = group_offsets ? G : 0;
+        const long long single = (((long long)M + TC_BM - 1) / TC_BM + pad / 2) * tiles_n, twos = (((long long)M + 2 * TC_BM - 1) / (2 * TC_BM) + pad / 2) * tiles_n;
+        const long long rounds = (single + sms - 1) / sms, pair_rounds = (twos + sms / 2 - 1) / (sms / 2);
+        pair = rounds >= 2 && 7 * pair_rounds <= 8 * rounds;
+    }
     int n_tile;
     {
-        const int out_max = dual ? TC_BN / 2 : TC_BN, unit = dual ? 8 : 16;
-        const int tiles = (N + out_max - 1) / out_max;
-        const int out = ((N + tiles - 1) / tiles + unit - 1) / unit * unit;
+        const int unit = (pair ? 32 : 16) >> dual;      // a pair's B tile is a multiple of 32 rows
+        const int out = ((N + tiles_n - 1) / tiles_n + unit - 1) / unit * unit;
         n_tile = dual ? 2 * out : out;
     }
     // With about one row tile per group (decoding with many sequences: the product streams
     // the experts' weights once and has G x column tiles to spread over the SMs) narrower tiles can fill a round
     // of SMs where the full width leaves a third of them idle; costs in rows loaded per k-block and round.
     if (group_offsets && (long long)M <= (long long)TC_BM * G) {
-        static int sms = 0;
-        if (!sms) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (sms <= 0) sms = 1;
-        }
         long long best = -1;
         for (int nt = TC_BN; nt >= 64; nt -= 16) {
             const int out = dual ? nt / 2 : nt;
@@ -592,16 +615,15 @@ static int gemm_tc_entry(const void* A, const void* B, void* C, const int* group
     if (rc) return rc;
     int* err_ptr = tc_error_ptr();
     if (!err_ptr) return tb_last_error();
-    // Pairs of blocks pay from about a thousand rows per group on, and only with a short K (the experts' down
-    // product of narrow experts, K = 688: -9 % at 2,048 rows per group), where a tile is over after a few k-blocks
-    // and what counts is how few bytes its start needs.  With K = 4,096 both forms measure the same, and with wide
-    // experts (K or N of 14,336) the single blocks are 4..20 % faster (1.41 against 1.18 PFLOP/s at 2,048 rows).
-    const bool pair = (long long)M >= 1024ll * G && K < 2048;
     TcArgs a{C, group_offsets, err_ptr, ldc, M, N, K, G, rows_b, dual, 0, n_tile, glu,
              // at most a tile of rows a group, on average: 8 of them (a prompt of 131 tokens through 8 layers of 16 experts 1,268 us
              // without, 1,246 with 4 or 8, 1,253 with 16, 1,288 with 64)
              (long long)M <= (long long)TC_BM * G ? 8 : 0};
-    if (glu.bias) return tc_launch<1, TC_EPI_BIASED>(ma, mb, a, s);
+    if (glu.bias) {
+        rc = pair ? tc_launch<2, TC_EPI_BIASED>(ma, mb, a, s) : TB_ERR_UNSUPPORTED;
+        if (rc == TB_ERR_UNSUPPORTED) rc = tc_launch<1, TC_EPI_BIASED>(ma, mb, a, s);
+        return rc;
+    }
     if (out_kind == 1) {
         rc = pair ? tc_launch<2, TC_EPI_FLOAT>(ma, mb, a, s) : TB_ERR_UNSUPPORTED;
         return rc == TB_ERR_UNSUPPORTED ? tc_launch<1, TC_EPI_FLOAT>(ma, mb, a, s) : rc;
