@@ -8,7 +8,7 @@
 //
 //   warp 0   TMA: the Q tile once, then K and V of each page into a two-stage ring (the cache of a
 //            layer is one 2-D tensor [pages * nkvh * 64, dh], so a page of a head is a box of rows)
-//   warp 1   one thread issues  S = Q K^T  (128 x 64, accumulator S in TMEM) and  O += P V
+//   warp 1   issues  S = Q K^T  (128 x 64, accumulator S in TMEM) and  O += P V
 //            (128 x dh, accumulator O in TMEM; P from TMEM, V is the MN-major B operand, straight as cached)
 //   warps 2-5  128 threads = the 128 query rows: read their row of S from TMEM, mask, running
 //            maximum and sum, P = exp2(s - m) rounded to bfloat16 and written back into tensor memory
@@ -19,7 +19,10 @@
 // The running maximum is only raised when it grows by more than 8 (in the exponent's log2 units):
 // then the row of O in TMEM is rescaled; otherwise P is simply computed against the older maximum
 // (it stays below 2^8, exact enough in bfloat16 and float), so the costly read-modify-write of O is
-// rare.  Every wait on an mbarrier is bounded (see gemm_tc.cu); a wait that runs out sets the error
+// rare.  Windows, kept first tokens, chunks, sinks, gates and capped scores are forms of the one kernel (AT_WINDOW, AT_CAPPED; rule and
+// measurements in parts/attention.py).  Warps 0 and 1 run their loops whole and one elected lane issues (see elect_one): 2,048
+// tokens of 32 heads of 128 40.9 us where one thread's loops took 45.5, 8 x 1,024 101 (111), 600 behind 1,000 of 8 heads over 2
+// 20 (26).  Bound by the softmax warps' chain a tile.  Every wait on an mbarrier is bounded (see gemm_tc.cu); a wait that runs out sets the error
 // word that tb_gemm_tc_status() reports.
 //
 // Head sizes 64 and 128.
