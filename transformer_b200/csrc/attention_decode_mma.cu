@@ -289,7 +289,7 @@ attention_decode_mma_kernel(const __grid_constant__ CUtensorMap mk, const __grid
         const int vrow = 16 * warp + (mi & 1) * 8 + lr, vch = mi >> 1;     // V: matrices (channels lo/hi) x (keys lo/hi)
         for (int i = 0; i < np && ok; ++i) {
             const int s = i % S;
-            ok = mbar_wait(full_bar(s), (i / S) & 1, a.error, 26);
+            ok = mbar_wait_warp(full_bar(s), (i / S) & 1, a.error, 26);
             if (!ok) break;
             const uint32_t sk = smem_base + s * STAGE_BYTES, sv = sk + PAGE_BYTES;
             if (patcher && i == np - 1) {

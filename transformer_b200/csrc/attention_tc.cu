@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             const int s = j % AT_STAGES;
             const int row = (pt[page_of(j)] * a.nkvh + g) * TB_PAGE;
             const uint32_t sk = skv + s * STAGE_BYTES, sv = sk + KV_BYTES;
-            if (j >= AT_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(k_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11));
+            if (j >= AT_STAGES) ok = mbar_wait_warp(k_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11);
             if (!ok) break;
             if (elect_one()) {
                 mbar_expect_tx(k_full(s), KV_BYTES);
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             }
             __syncwarp();
             k_issued = j + 1;
-            if (j >= AT_STAGES) ok = __all_sync(0xffffffffu, mbar_wait(v_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11));
+            if (j >= AT_STAGES) ok = mbar_wait_warp(v_empty(s), ((j / AT_STAGES) - 1) & 1, a.error, 11);
             if (!ok) break;
             if (elect_one()) {
                 mbar_expect_tx(v_full(s), KV_BYTES);
@@ -269,9 +269,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             }
             __syncwarp();
         };
-        bool ok = mbar_wait(q_full, 0, a.error, 12);
-        if (ok) ok = mbar_wait(k_full(0), 0, a.error, 12);
-        ok = __all_sync(0xffffffffu, ok);
+        bool ok = mbar_wait_warp(q_full, 0, a.error, 12) && mbar_wait_warp(k_full(0), 0, a.error, 12);
         if (ok) {
             tc_fence_after();
             issue_s(0);
@@ -280,14 +278,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             const int s = j % AT_STAGES;
             // the scores of the NEXT tile are computed while the softmax warps work on this one
             if (j + 1 < n_tiles) {
-                ok = __all_sync(0xffffffffu, mbar_wait(k_full((j + 1) % AT_STAGES), ((j + 1) / AT_STAGES) & 1, a.error, 12));
+                ok = mbar_wait_warp(k_full((j + 1) % AT_STAGES), ((j + 1) / AT_STAGES) & 1, a.error, 12);
                 if (!ok) break;
                 tc_fence_after();
                 issue_s(j + 1);
             }
-            ok = mbar_wait(p_ready(j & 1), (j >> 1) & 1, a.error, 13);   // P is in tensor memory, where S of tile j was
-            if (ok) ok = mbar_wait(v_full(s), (j / AT_STAGES) & 1, a.error, 12);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = mbar_wait_warp(p_ready(j & 1), (j >> 1) & 1, a.error, 13) &&   // P is in tensor memory, where S of tile j was
+                 mbar_wait_warp(v_full(s), (j / AT_STAGES) & 1, a.error, 12);
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
@@ -315,7 +312,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
         bool ok = true;
         const float scale = CAPPED ? 1.0f : a.scale_log2e;
         for (int j = 0; j < n_tiles && ok; ++j) {
-            ok = mbar_wait(s_full(j & 1), (j >> 1) & 1, a.error, 15);
+            ok = mbar_wait_warp(s_full(j & 1), (j >> 1) & 1, a.error, 15);
             tc_fence_after();
             if (!ok) break;
             float s[AT_BN];
@@ -411,7 +408,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             // which nothing reads any more: no wait for that)
             const bool touch_o = __any_sync(0xffffffffu, rescale != 1.0f) && j > 0;
             if (touch_o) {
-                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
+                ok = mbar_wait_warp(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
                 tc_fence_after();
                 if (!ok) break;
 #pragma unroll
@@ -433,12 +430,12 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             // tell "two behind" from "done").  Here it costs nothing: P has been handed over, and the product
             // waited for was issued a whole tile ago.
             if (j > 0 && !touch_o) {
-                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
+                ok = mbar_wait_warp(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, a.error, 16);
                 tc_fence_after();
             }
         }
         if (ok) {
-            ok = mbar_wait(o_done((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, a.error, 17);
+            ok = mbar_wait_warp(o_done((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, a.error, 17);
             tc_fence_after();
         }
         if (ok) {

@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             if (!tl.valid) continue;
             const int buf = lt & 1;
             const int m = tl.row0 + (int)rank * TC_BM + row, n0 = tl.n0;
-            ok = mbar_wait(acc_full(buf), (lt >> 1) & 1, a.error, 3);
+            ok = mbar_wait_warp(acc_full(buf), (lt >> 1) & 1, a.error, 3);
             tc_fence_after();
             if (!ok) break;
             const uint32_t trow = tmem_base + buf * TC_BN + ((uint32_t)(quad * 32) << 16);

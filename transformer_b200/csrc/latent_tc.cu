@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
         int it = 0, slot = 0;
         uint32_t used = 1;                                // parity of the slot's last use
         auto box = [&](int x, int row) {
-            if (it >= LT_RING) ok = __all_sync(0xffffffffu, mbar_wait(empty(slot), used, g.error, 42));
+            if (it >= LT_RING) ok = mbar_wait_warp(empty(slot), used, g.error, 42);
             if (!ok) return;
             if (elect_one()) {
                 mbar_expect_tx(full(slot), LT_BOX_BYTES);
@@ -167,11 +167,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
         const uint32_t idesc_s = umma_idesc(LT_ROWS, LT_KEYS), idesc_o = umma_idesc(LT_ROWS, 64) | (1u << 16);
         int slot = 0;
         uint32_t use = 0;
-        bool ok = mbar_wait(q_full, 0, g.error, 44);
-        if (ok) ok = mbar_wait(q_turned, 0, g.error, 44);
-        ok = __all_sync(0xffffffffu, ok);
+        bool ok = mbar_wait_warp(q_full, 0, g.error, 44) && mbar_wait_warp(q_turned, 0, g.error, 44);
         auto arrived = [&]() {
-            ok = __all_sync(0xffffffffu, mbar_wait(full(slot), use, g.error, 44));
+            ok = mbar_wait_warp(full(slot), use, g.error, 44);
             tc_fence_after();
             return ok;
         };
@@ -201,7 +199,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
         for (int j = 0; j < pages && ok; ++j) {
             if (j + 1 < pages) scores(j + 1);             // while the softmax warps work on page j
             if (!ok) break;
-            ok = __all_sync(0xffffffffu, mbar_wait(p_ready(j & 1), (j >> 1) & 1, g.error, 45));
+            ok = mbar_wait_warp(p_ready(j & 1), (j >> 1) & 1, g.error, 45);
             if (!ok) break;
             tc_fence_after();
             for (int b = 0; b < LT_COLS / 64; ++b) {
@@ -262,7 +260,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
         float mx = -INFINITY, sum = 0.f;
         bool ok = true;
         for (int j = 0; j < pages && ok; ++j) {
-            ok = mbar_wait(s_full(j & 1), (j >> 1) & 1, g.error, 46);
+            ok = mbar_wait_warp(s_full(j & 1), (j >> 1) & 1, g.error, 46);
             tc_fence_after();
             if (!ok) break;
             const uint32_t ts = tmem_s + (j & 1) * 128 + lane_sel;
@@ -306,7 +304,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
             sum = sum * corr + v[0];
             const bool move = j > 0 && __any_sync(0xffffffffu, corr != 1.f);
             if (move) {         // O is touched once the previous page's product is done
-                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, g.error, 47);
+                ok = mbar_wait_warp(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, g.error, 47);
                 tc_fence_after();
                 if (!ok) break;
 #pragma unroll
@@ -331,12 +329,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(p_ready(j & 1)) : "memory");
             // keep in step with the products, phase by phase
             if (j > 0 && !move) {
-                ok = mbar_wait(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, g.error, 47);
+                ok = mbar_wait_warp(o_done((j - 1) & 1), ((j - 1) >> 1) & 1, g.error, 47);
                 tc_fence_after();
             }
         }
         if (ok) {
-            ok = mbar_wait(o_done((pages - 1) & 1), ((pages - 1) >> 1) & 1, g.error, 48);
+            ok = mbar_wait_warp(o_done((pages - 1) & 1), ((pages - 1) >> 1) & 1, g.error, 48);
             tc_fence_after();
         }
         if (ok) {

@@ -43,6 +43,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
     atomicCAS(error, 0, code);
     return false;
 }
+// The same by a whole warp: all lanes have the same answer.  A lane that gives up by itself would leave the others at the next vote,
+// shuffle or tcgen05 load of the whole warp, with no bound on their wait.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* error, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, error, code));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
