@@ -1,6 +1,6 @@
 """The windowed form of the tcgen05 prompt attention at the edges of tiles, pages, windows and chunks, against float64.
 
-Tolerance: the weights are rounded to bfloat16 (2^-9 of each, against a sum of unrounded ones) and so is the result:
+Tolerance of the first: the weights are rounded to bfloat16 (2^-9 of each, against a sum of unrounded ones) and so is the result:
 2^-8 of the largest |value|.  The products and exponentials in 32 bits add some 1e-6; 1e-3 covers the gate's and the
 cap's approximate divisions as well."""
 import pytest
@@ -81,3 +81,37 @@ def test_windowed_form(nh, nkvh, dh, window, keep, chunk, cap, more):
         err = float((out[at:at + n, :nh * dh].reshape(n, nh, dh).double() - want).abs().max())
         assert err <= 2.0 ** -8 * float(vc.abs().max()) + 1e-3, (b, err)
         at += n
+
+
+@pytest.mark.parametrize("nh,nkvh,dh,window,keep,chunk,cap,more", [
+    (8, 2, 128, 100, 4, 0, 30.0, "gate"), (4, 4, 64, 64, 0, 0, 0.0, "sinks"), (6, 2, 64, 65, 70, 0, 5.0, "heads"),
+    (5, 1, 128, 1 << 30, 0, 96, 0.0, "gate"), (4, 2, 128, 1 << 30, 0, 0, 0.0, ""), (16, 1, 64, 200, 3, 0, 20.0, "")])
+def test_bits_of_the_mma_form(nh, nkvh, dh, window, keep, chunk, cap, more):
+    """The mma.sync kernel without slices: the same weights (against the row's true maximum) and sums in the same order, so the same
+    bits, whichever of the two a step takes."""
+    from transformer_b200.csrc import lib
+    g = torch.Generator().manual_seed(nh + dh + window % 1000)
+    c = _batch(g)
+    bf = lambda *shape: torch.randn(*shape, generator=g).bfloat16().cuda()
+    nt, mma = c["nt"], lib.attention_window_mma_tile_tokens(nh, nkvh)
+    kc, vc, z = bf(c["n_pages"], nkvh, 64, dh), bf(c["n_pages"], nkvh, 64, dh), bf(nt, 2 * nh * dh)
+    z[:, :nh * dh] *= 2
+    gate, per_head, mult = (z[:, nh * dh:], 0, 1.0) if more == "gate" else (bf(nt, nh), 1, 0.7) if more == "heads" else (None, 0, 1.0)
+    sinks = torch.randn(nh, generator=g).cuda() * 2 if more == "sinks" else None
+    I = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    seq, t0, nq, at = [], [], [], 0
+    for b, n in enumerate(NEW):
+        for off in range(0, n, mma):
+            seq.append(b), t0.append(at + off), nq.append(min(mma, n - off))
+        at += n
+    seq, t0, nq = I(seq), I(t0), I(nq)
+    got, want = (torch.empty(nt, nh * dh, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    data = lambda out: (lib.ptr(z), lib.ptr(out), lib.ptr(kc), lib.ptr(vc), lib.ptr(gate))
+    rows = (nt, c["max_pages"], z.stride(0), 0 if gate is None else gate.stride(0), nh, nkvh)
+    rule = (window, keep, dh ** -0.5, cap, chunk, lib.ptr(sinks))
+    lib.call("tb_attention_tc_window_bf16", *data(got), lib.ptr(c["seq"]), lib.ptr(c["t0"]), lib.ptr(c["nq"]), lib.ptr(c["pos"]),
+             lib.ptr(c["table"]), c["tiles"], *rows, dh, c["n_pages"], *rule, per_head, mult, nh * dh)
+    lib.call("tb_attention_window_mma_heads_bf16", *data(want), lib.ptr(seq), lib.ptr(t0), lib.ptr(nq), lib.ptr(c["pos"]),
+             lib.ptr(c["table"]), 0, len(seq), *rows, dh, dh, 1, *rule, 0, 0, per_head, mult, nh * dh)
+    assert lib.gemm_tc_status() == 0 and bool(torch.isfinite(want).all())
+    assert torch.equal(got, want)

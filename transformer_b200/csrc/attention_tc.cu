@@ -16,11 +16,12 @@
 //            (tcgen05.mma with A in tensor memory), so P never passes through shared memory; and at
 //            the end O / l to memory.
 //
-// The running maximum is only raised when it grows by more than 8 (in the exponent's log2 units):
+// Plain causal attention: the running maximum is only raised when it grows by more than 8 (in the exponent's log2 units):
 // then the row of O in TMEM is rescaled; otherwise P is simply computed against the older maximum
 // (it stays below 2^8, exact enough in bfloat16 and float), so the costly read-modify-write of O is
 // rare.  Windows, kept first tokens, chunks, sinks, gates and capped scores are forms of the one kernel (AT_WINDOW, AT_CAPPED; rule and
-// measurements in parts/attention.py).  Warps 0 and 1 run their loops whole and one elected lane issues (see elect_one): 2,048
+// measurements in parts/attention.py); these raise it wherever it grows and have the bits of attention_window_mma.cu (16 heads of 128 over 4
+// key heads, 2,039 tokens, capped: 63.6 us, 58.4 with the older maximum, 109 there).  Warps 0 and 1 run their loops whole and one elected lane issues (see elect_one): 2,048
 // tokens of 32 heads of 128 40.9 us where one thread's loops took 45.5, 8 x 1,024 101 (111), 600 behind 1,000 of 8 heads over 2
 // 20 (26).  Bound by the softmax warps' chain a tile.  Every wait on an mbarrier is bounded (see gemm_tc.cu); a wait that runs out sets the error
 // word that tb_gemm_tc_status() reports.
@@ -28,6 +29,7 @@
 // Head sizes 64 and 128.
 #include <cuda.h>
 
+#include "memory_common.cuh"            // two floats an instruction
 #include "tc_common.cuh"
 
 #define AT_BM 128
@@ -309,8 +311,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
         const int pos_r = pos_first + row;
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         float m_used = -INFINITY, l_run = 0.f;
+        F2 lw[2] = {};                                      // all but PLAIN: the sums of the weights at columns 2 t and 2 t + 1 of eight, t = 0..3
         bool ok = true;
-        const float scale = CAPPED ? 1.0f : a.scale_log2e;
         for (int j = 0; j < n_tiles && ok; ++j) {
             ok = mbar_wait_warp(s_full(j & 1), (j >> 1) & 1, a.error, 15);
             tc_fence_after();
@@ -341,6 +343,10 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                     s[i] = a.cap_l2 - __fdividef(2.0f * a.cap_l2, 1.0f + e);
                 }
             }
+            if constexpr (FORM == AT_WINDOW) {
+#pragma unroll
+                for (int i = 0; i < AT_BN; ++i) s[i] *= a.scale_log2e;
+            }
             if constexpr (PLAIN) {
                 if (key0 + AT_BN - 1 > pos_first) {             // uniform over the block: a tile on or past the diagonal
 #pragma unroll
@@ -369,41 +375,74 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                 asm("max.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(s[i]), "f"(s[i + 1]));
                 asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(s[i + 2]), "f"(s[i + 3]));
             }
-            mx = fmaxf(mx, mx1) * scale;
-            // raise the maximum only when it has grown by more than 8; then O must be rescaled
-            const bool raise = mx > m_used + 8.0f;          // also true for the first visible keys (m_used = -inf)
-            const float m_new = raise ? mx : m_used;
-            const float rescale = (raise && m_used != -INFINITY) ? exp2f(m_used - m_new) : 1.0f;
-            m_used = m_new;
-            const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
             // computed BEFORE waiting for the previous tile's P V: the exponentials overlap that product,
             // only the stores below come after it
+            float rescale;
             uint32_t pk[AT_BN / 2];
-            // two scores at a time through the packed forms of multiply-add and add (half the instructions)
-            const uint64_t sc2 = pack_f32x2(scale, scale), nm2 = pack_f32x2(neg_m, neg_m);
-            uint64_t psum_a = 0ull, psum_b = 0ull;              // two pairs of +0.0f
+            if constexpr (PLAIN) {
+                mx = fmaxf(mx, mx1) * a.scale_log2e;
+                // raise the maximum only when it has grown by more than 8; then O must be rescaled
+                const bool raise = mx > m_used + 8.0f;          // also true for the first visible keys (m_used = -inf)
+                const float m_new = raise ? mx : m_used;
+                rescale = (raise && m_used != -INFINITY) ? exp2f(m_used - m_new) : 1.0f;
+                m_used = m_new;
+                const float neg_m = (m_used == -INFINITY) ? 0.f : -m_used;
+                // two scores at a time through the packed forms of multiply-add and add (half the instructions)
+                const uint64_t sc2 = pack_f32x2(a.scale_log2e, a.scale_log2e), nm2 = pack_f32x2(neg_m, neg_m);
+                uint64_t psum_a = 0ull, psum_b = 0ull;              // two pairs of +0.0f
 #pragma unroll
-            for (int i = 0; i < AT_BN; i += 4) {
-                uint64_t t0, t1;
-                asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t0) : "l"(pack_f32x2(s[i], s[i + 1])), "l"(sc2), "l"(nm2));
-                asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t1) : "l"(pack_f32x2(s[i + 2], s[i + 3])), "l"(sc2), "l"(nm2));
-                float e0, e1, e2, e3, p0, p1, p2, p3;
-                unpack_f32x2(t0, e0, e1);
-                unpack_f32x2(t1, e2, e3);
-                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(e0));
-                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(e1));
-                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p2) : "f"(e2));
-                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p3) : "f"(e3));
-                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum_a) : "l"(pack_f32x2(p0, p1)));
-                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum_b) : "l"(pack_f32x2(p2, p3)));
-                __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
-                pk[i / 2] = *reinterpret_cast<uint32_t*>(&h0);
-                pk[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&h1);
+                for (int i = 0; i < AT_BN; i += 4) {
+                    uint64_t t0, t1;
+                    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t0) : "l"(pack_f32x2(s[i], s[i + 1])), "l"(sc2), "l"(nm2));
+                    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t1) : "l"(pack_f32x2(s[i + 2], s[i + 3])), "l"(sc2), "l"(nm2));
+                    float e0, e1, e2, e3, p0, p1, p2, p3;
+                    unpack_f32x2(t0, e0, e1);
+                    unpack_f32x2(t1, e2, e3);
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(e0));
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(e1));
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p2) : "f"(e2));
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p3) : "f"(e3));
+                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum_a) : "l"(pack_f32x2(p0, p1)));
+                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(psum_b) : "l"(pack_f32x2(p2, p3)));
+                    __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
+                    pk[i / 2] = *reinterpret_cast<uint32_t*>(&h0);
+                    pk[i / 2 + 1] = *reinterpret_cast<uint32_t*>(&h1);
+                }
+                float ps0, ps1, ps2, ps3;
+                unpack_f32x2(psum_a, ps0, ps1);
+                unpack_f32x2(psum_b, ps2, ps3);
+                l_run = l_run * rescale + ((ps0 + ps1) + (ps2 + ps3));
+            } else {
+                // Weights against the true maximum, as in attention_window_mma.cu, where the largest of a row is exactly 1: against an older
+                // maximum it is rounded like the others, and the results were 12 to 24 % farther from 64 bits (2.2e-3 of their
+                // norm for 1.9e-3).  The sums are added in that kernel's order too, so a result has its bits.
+                mx = fmaxf(m_used, fmaxf(mx, mx1));
+                const float ref = mx == -INFINITY ? 0.f : mx;
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(rescale) : "f"(m_used - ref));
+                if (m_used == -INFINITY) rescale = 1.0f;        // nothing but zeros so far
+                m_used = mx;
+                F2 neg, by;
+                neg.f = make_float2(-ref, -ref);
+                by.f = make_float2(rescale, rescale);
+                lw[0] = mul2(lw[0], by);
+                lw[1] = mul2(lw[1], by);
+#pragma unroll
+                for (int i = 0; i < AT_BN; i += 4) {
+                    F2 x[2], sum;
+                    x[0].f = make_float2(s[i], s[i + 1]);
+                    x[1].f = make_float2(s[i + 2], s[i + 3]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        x[e] = add2(x[e], neg);
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x[e].f.x));
+                        asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(x[e].f.y));
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(x[e].f.x, x[e].f.y);
+                        pk[i / 2 + e] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    sum.f = make_float2(x[0].f.x + x[0].f.y, x[1].f.x + x[1].f.y);
+                    lw[(i >> 2) & 1] = add2(lw[(i >> 2) & 1], sum);
+                }
             }
-            float ps0, ps1, ps2, ps3;
-            unpack_f32x2(psum_a, ps0, ps1);
-            unpack_f32x2(psum_b, ps2, ps3);
-            l_run = l_run * rescale + ((ps0 + ps1) + (ps2 + ps3));
             // O may only be touched once the previous tile's P V is done (P itself goes where this tile's S was,
             // which nothing reads any more: no wait for that)
             const bool touch_o = __any_sync(0xffffffffu, rescale != 1.0f) && j > 0;
@@ -439,6 +478,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             tc_fence_after();
         }
         if (ok) {
+            if constexpr (!PLAIN) l_run = (lw[0].f.x + lw[0].f.y) + (lw[1].f.x + lw[1].f.y);
             float inv = 1.0f / l_run;
             const int t = t0 + row;
             const __nv_bfloat16* gt = nullptr;
