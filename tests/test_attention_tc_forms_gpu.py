@@ -115,3 +115,48 @@ def test_bits_of_the_mma_form(nh, nkvh, dh, window, keep, chunk, cap, more):
              lib.ptr(c["table"]), 0, len(seq), *rows, dh, dh, 1, *rule, 0, 0, per_head, mult, nh * dh)
     assert lib.gemm_tc_status() == 0 and bool(torch.isfinite(want).all())
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("nh,nkvh,dh,window,keep,chunk,cap", [
+    (4, 2, 128, 100, 4, 0, 30.0), (4, 4, 64, 64, 0, 0, 0.0), (6, 2, 64, 1 << 30, 0, 96, 0.0), (3, 1, 128, 1 << 30, 0, 0, 20.0)])
+def test_what_is_no_number_stays_with_the_rows_that_see_it(nh, nkvh, dh, window, keep, chunk, cap):
+    """Values that are infinite or NaN at places before, in and behind the tiles (one of them in a page's rows that no sequence has
+    reached): the rows that do not see them keep their bits, the others too but in the columns of those values."""
+    from transformer_b200.csrc import lib
+    g = torch.Generator().manual_seed(7 * nh + dh)
+    c = _batch(g)
+    bf = lambda *shape: torch.randn(*shape, generator=g).bfloat16().cuda()
+    nt = c["nt"]
+    kc, vc, z = bf(c["n_pages"], nkvh, 64, dh), bf(c["n_pages"], nkvh, 64, dh), bf(nt, nh * dh)
+
+    def run():
+        out = torch.empty((nt, nh, dh), dtype=torch.bfloat16, device="cuda")
+        lib.call("tb_attention_tc_window_bf16", lib.ptr(z), lib.ptr(out), lib.ptr(kc), lib.ptr(vc), 0, lib.ptr(c["seq"]),
+                 lib.ptr(c["t0"]), lib.ptr(c["nq"]), lib.ptr(c["pos"]), lib.ptr(c["table"]), c["tiles"], nt, c["max_pages"], nh * dh,
+                 0, nh, nkvh, dh, c["n_pages"], window, keep, dh ** -0.5, cap, chunk, 0, 0, 1.0, nh * dh)
+        assert lib.gemm_tc_status() == 0
+        return out
+
+    good = run()
+    assert bool(torch.isfinite(good).all())
+    # (sequence, key, key head, column, value); the last is behind its sequence's end
+    bad = [(0, 250, 0, 3, float("nan")), (0, 0, nkvh - 1, dh - 1, float("inf")), (0, 130, 0, 40, float("-inf")), (2, 190, 0, 0, float("inf")),
+           (2, 328, nkvh - 1, 17, float("nan")), (4, 131, 0, 33, float("nan")), (5, 320, 0, dh // 2, float("inf")),
+           (1, 62, 0, 9, float("nan")), (0, 310, 0, 9, float("nan"))]
+    for b, key, head, col, value in bad:
+        vc[c["pages"][b][key // 64], head, key % 64, col] = value
+    got, want, at = run(), good.clone(), 0
+    for b, n in enumerate(NEW):
+        p = torch.arange(BEFORE[b], BEFORE[b] + n, device="cuda")
+        for _, key, head, col, value in (e for e in bad if e[0] == b):
+            see = (key <= p) & ((p - key < window) | (key < keep))
+            if chunk:
+                see &= p // chunk == key // chunk
+            heads = range(head * (nh // nkvh), (head + 1) * (nh // nkvh))
+            for h in heads:
+                hit = got[at:at + n, h, col][see]
+                assert not bool(torch.isfinite(hit).any()), (b, key, h)
+                want[at:at + n, h, col][see] = hit
+        at += n
+    same = (got == want) | (got.isnan() & want.isnan())
+    assert bool(same.all())

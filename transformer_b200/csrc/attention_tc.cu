@@ -55,6 +55,7 @@ struct AtArgs {
     float scale_log2e;
     unsigned v_lbo, v_sbo;    // descriptor strides of the MN-major V operand, in bytes
     // all but AT_PLAIN
+    const __nv_bfloat16* vc;      // the cache that V's tiles come from
     const float* sinks;           // [nh] or null
     const __nv_bfloat16* gate;    // [nt, gate_stride] or null
     int gate_stride, gate_per_head, window, keep_first, chunk;
@@ -130,6 +131,39 @@ __device__ __forceinline__ void tmem_st32_words(uint32_t taddr, const uint32_t (
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// What is no number stays with the rows that see it.  A key that a row does not see has the weight 0, and 0 times an infinite or NaN
+// value is NaN: with 128 tokens a tile it would reach as many as 127 tokens before the value's own.  So the windowed forms look
+// through V's entries in the pages that not every row sees whole, 16 keys a warp, make those that are no number 0 (for every row's
+// product) and set *found; the epilogue adds them to the rows that do see them.
+template <int KB>      // apart from the page loop: inlined it cost that 1 to 4 %
+__device__ __noinline__ void at_clear_row(uint8_t* row, volatile uint32_t* found) {
+    for (int i = 0; i < KB * 16; ++i) {
+        uint32_t* w = reinterpret_cast<uint32_t*>(row + (i >> 4) * (AT_BN * 128)) + (i & 15);
+        *w = finite_pair(*w);
+    }
+    *found = 1;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the product reads these writes
+}
+template <int KB>
+__device__ __forceinline__ void at_clear(uint8_t* v, int key, int half, volatile uint32_t* found) {
+    uint8_t* row = v + key * 128 + half * 64;             // two lanes a key; the swizzle moves pieces within a row only
+    const __nv_bfloat162 zero = __float2bfloat162_rn(0.f);
+    __nv_bfloat162 sum[4] = {zero, zero, zero, zero};     // of 0 times the entries: 0, or NaN
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 x = *reinterpret_cast<const uint4*>(row + kb * (AT_BN * 128) + ((i ^ (key & 3)) << 4));
+            const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[e] = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]), zero, sum[e]);
+        }
+    sum[0] = __hadd2(__hadd2(sum[0], sum[1]), __hadd2(sum[2], sum[3]));
+    const bool bad = (*reinterpret_cast<const uint32_t*>(&sum[0]) & 0x7fff7fffu) != 0;
+    if (bad) at_clear_row<KB>(row, found);
+    __syncwarp();
+}
+
 // KB: 64-wide column boxes of a head; FORM: see AT_PLAIN.
 template <int KB, int FORM>
 __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -150,6 +184,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
     const uint32_t sq = smem_base, skv = sq + Q_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Q_BYTES + AT_STAGES * STAGE_BYTES);
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + AT_BARS);
+    volatile uint32_t* cleared = &tmem_slot + 1;          // not zero: see at_clear
     const int warp = warp_number(), lane = threadIdx.x & 31;
     if (smem_base & 1023u) {                              // never expected; refuse rather than compute garbage
         if (threadIdx.x == 0) atomicCAS(a.error, 0, 19);
@@ -192,6 +227,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
     auto p_ready = [&](int i) { return q_full + 24 + 8u * i; };
     auto o_done = [&](int i) { return q_full + 40 + 8u * i; };
     if (threadIdx.x == 0) {
+        *cleared = 0;
         for (int s = 0; s < AT_STAGES; ++s) {
             mbar_init(k_full(s), 1);
             mbar_init(k_empty(s), 1);
@@ -313,6 +349,14 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
         float m_used = -INFINITY, l_run = 0.f;
         F2 lw[2] = {};                                      // all but PLAIN: the sums of the weights at columns 2 t and 2 t + 1 of eight, t = 0..3
         bool ok = true;
+        // every key of a page visible to every row: not later than the first row's token, inside the last row's window
+        // or among the kept, in the last row's chunk (uniform over the block); and what this row sees of any other page
+        auto open_page = [&](int key0) {
+            return key0 + AT_BN - 1 <= pos_first && (pos_last - key0 < a.window || key0 + AT_BN - 1 < a.keep_first) &&
+                   (a.chunk <= 0 || key0 / a.chunk == pos_last / a.chunk);
+        };
+        const int near = pos_r - a.window, from = !PLAIN && a.chunk > 0 ? pos_r / a.chunk * a.chunk : 0;
+        auto sees = [&](int key) { return key <= pos_r && key >= from && (key > near || key < a.keep_first); };
         for (int j = 0; j < n_tiles && ok; ++j) {
             ok = mbar_wait_warp(s_full(j & 1), (j >> 1) & 1, a.error, 15);
             tc_fence_after();
@@ -354,18 +398,10 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                         if (key0 + i > pos_r) s[i] = -INFINITY;
                 }
             } else {
-                // every key visible to every row: not later than the first row's token, inside the last row's window
-                // or among the kept, in the last row's chunk (uniform over the block)
-                const bool open = key0 + AT_BN - 1 <= pos_first &&
-                                  (pos_last - key0 < a.window || key0 + AT_BN - 1 < a.keep_first) &&
-                                  (a.chunk <= 0 || key0 / a.chunk == pos_last / a.chunk);
-                if (!open) {
-                    const int near = pos_r - a.window, from = a.chunk > 0 ? pos_r / a.chunk * a.chunk : 0;
+                if (!open_page(key0)) {
 #pragma unroll
-                    for (int i = 0; i < AT_BN; ++i) {
-                        const int key = key0 + i;
-                        if (key > pos_r || key < from || !(key > near || key < a.keep_first)) s[i] = -INFINITY;
-                    }
+                    for (int i = 0; i < AT_BN; ++i)
+                        if (!sees(key0 + i)) s[i] = -INFINITY;
                 }
             }
             // two chains of three-input maxima: 32 instructions for the 64 scores
@@ -443,6 +479,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
                     lw[(i >> 2) & 1] = add2(lw[(i >> 2) & 1], sum);
                 }
             }
+            if constexpr (!PLAIN) {
+                if (!open_page(key0)) {
+                    ok = mbar_wait_warp(v_full(j % AT_STAGES), (j / AT_STAGES) & 1, a.error, 18);
+                    if (!ok) break;
+                    at_clear<KB>(smem_raw + Q_BYTES + (j % AT_STAGES) * STAGE_BYTES + KV_BYTES, quad * 16 + (lane >> 1), lane & 1, cleared);
+                }
+            }
             // O may only be touched once the previous tile's P V is done (P itself goes where this tile's S was,
             // which nothing reads any more: no wait for that)
             const bool touch_o = __any_sync(0xffffffffu, rescale != 1.0f) && j > 0;
@@ -477,6 +520,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             ok = mbar_wait_warp(o_done((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, a.error, 17);
             tc_fence_after();
         }
+        if constexpr (!PLAIN) asm volatile("bar.sync 1, 128;" ::: "memory");      // *cleared, as any of the four warps left it
         if (ok) {
             if constexpr (!PLAIN) l_run = (lw[0].f.x + lw[0].f.y) + (lw[1].f.x + lw[1].f.y);
             float inv = 1.0f / l_run;
@@ -499,6 +543,26 @@ __global__ void __launch_bounds__(AT_THREADS, 2) attention_tc_kernel(const __gri
             for (int c0 = 0; c0 < DH; c0 += 32) {
                 float o[32];
                 tmem_ld32(tmem_o + lane_sel + c0, o);       // warp-collective: rows past nq take part, store nothing
+                if constexpr (!PLAIN) {
+                    if (*cleared && row < nq) {
+                        for (int j = 0; j < n_tiles; ++j) {
+                            const int page = page_of(j), key0 = page * AT_BN;
+                            if (open_page(key0)) continue;
+                            const __nv_bfloat16* vp = a.vc + ((size_t)pt[page] * a.nkvh + g) * (TB_PAGE * DH) + c0;
+                            for (int k = 0; k < AT_BN; ++k) {
+                                if (!sees(key0 + k)) continue;
+#pragma unroll
+                                for (int i = 0; i < 32; i += 8) {
+                                    float v8[8];
+                                    load8(vp + k * DH + i, v8);
+#pragma unroll
+                                    for (int e = 0; e < 8; ++e)
+                                        if (!(fabsf(v8[e]) < INFINITY)) o[i + e] += v8[e];
+                                }
+                            }
+                        }
+                    }
+                }
                 if (row < nq) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
@@ -552,6 +616,7 @@ static int at_paged(const void* q, void* out, const void* kc, const void* vc, co
     rc = make_map(&mv, vc, rows, dh, dh, AT_BN);
     if (rc) return rc;
     a.out = (__nv_bfloat16*)out;
+    a.vc = (const __nv_bfloat16*)vc;
     a.tile_seq = tile_seq;
     a.tile_t0 = tile_t0;
     a.tile_nq = tile_nq;

@@ -48,6 +48,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* error, int code) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, error, code));
 }
+// Two bfloat16: a bit at the place of each sign (0x80008000) where it is infinite or NaN (an exponent of all ones carries into the
+// cleared sign); the other bits say nothing.  And the pair with zeros in their place.
+__device__ __forceinline__ uint32_t not_finite_pair(uint32_t w) { return (w & 0x7fff7fffu) + 0x00800080u; }
+__device__ __forceinline__ uint32_t finite_pair(uint32_t w) { return w & ~(((not_finite_pair(w) >> 15) & 0x00010001u) * 0xffffu); }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
