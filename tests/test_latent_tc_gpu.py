@@ -2,16 +2,16 @@
 
 Tiles of 128 rows that no sequence fills, windows that begin and end inside a page, heads that do not divide 128, one and two
 blocks a tile, rotated parts of 0, 32 and 64 entries of which not all turn."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("H,rank,rot,rdims,window,pitch", [
-    (16, 512, 64, 64, 1 << 30, 16), (8, 256, 32, 32, 100, 16), (20, 256, 64, 32, 64, 16), (3, 256, 0, 0, 200, 16),
-    (16, 512, 64, 20, 70, 12), (128, 512, 32, 16, 300, 16), (1, 256, 64, 64, 1, 16), (5, 512, 0, 0, 65, 3)])
-def test_same_bits(H, rank, rot, rdims, window, pitch):
+def _latents(H, rank, rot, rdims, window, pitch):
+    """The sequences' caches and queries, and a function that runs a kernel over them."""
     from transformer_b200.csrc import lib
     g = torch.Generator().manual_seed(rank + rot + H)
     tile = lib.latent_tc_tile_tokens(H, rank, rot)
@@ -49,7 +49,39 @@ def test_same_bits(H, rank, rot, rdims, window, pitch):
         assert lib.gemm_tc_status() == 0
         return out
 
-    for sink, gates in ((None, None), (sinks, gate)):
-        want = run("mma", lib.latent_attention_tile_tokens(H), (0,), (), sink, gates)
+    return SimpleNamespace(run=run, tile=tile, cache=cache, table=table, before=before, new=new, sinks=sinks, gate=gate,
+                           mma_tile=lib.latent_attention_tile_tokens(H))
+
+
+@pytest.mark.parametrize("H,rank,rot,rdims,window,pitch", [
+    (16, 512, 64, 64, 1 << 30, 16), (8, 256, 32, 32, 100, 16), (20, 256, 64, 32, 64, 16), (3, 256, 0, 0, 200, 16),
+    (16, 512, 64, 20, 70, 12), (128, 512, 32, 16, 300, 16), (1, 256, 64, 64, 1, 16), (5, 512, 0, 0, 65, 3)])
+def test_same_bits(H, rank, rot, rdims, window, pitch):
+    c = _latents(H, rank, rot, rdims, window, pitch)
+    for sink, gates in ((None, None), (c.sinks, c.gate)):
+        want = c.run("mma", c.mma_tile, (0,), (), sink, gates)
         assert bool(torch.isfinite(want).all()) and float(want.abs().mean()) > 1e-3
-        assert torch.equal(run("tc", tile, (), (cache.shape[0],), sink, gates), want)
+        assert torch.equal(c.run("tc", c.tile, (), (c.cache.shape[0],), sink, gates), want)
+
+
+@pytest.mark.parametrize("H,rank,rot,rdims,window,pitch", [
+    (16, 512, 64, 64, 1 << 30, 16), (8, 256, 32, 32, 100, 16), (3, 256, 0, 0, 70, 16), (1, 256, 64, 64, 1 << 30, 16)])
+def test_what_is_no_number_stays_with_the_rows_that_see_it(H, rank, rot, rdims, window, pitch):
+    """Entries that are infinite or NaN: the rows that do not see their tokens keep their bits, the others have no number there."""
+    c = _latents(H, rank, rot, rdims, window, pitch)
+    good = c.run("tc", c.tile, (), (c.cache.shape[0],))
+    # (sequence, key, column, value): one in the middle of a page, at a page's border, of three tokens, behind a sequence's end
+    bad = [(0, 250, 3, float("nan")), (0, 128, rank - 1, float("inf")), (1, 62, 0, float("-inf")), (0, 310, 70, float("nan")),
+           (5, 64 + 3 * c.tile, 200, float("inf")), (2, 200, 5, float("nan"))]
+    for b, key, col, value in bad:
+        c.cache[int(c.table[b, key // 64]), key % 64, col] = value
+    got, want, at = c.run("tc", c.tile, (), (c.cache.shape[0],)), good.clone(), 0
+    for b, n in enumerate(c.new):
+        p = torch.arange(c.before[b], c.before[b] + n, device="cuda")
+        for _, key, col, value in (e for e in bad if e[0] == b):
+            see = (key <= p) & (p - key < window)
+            assert not bool(torch.isfinite(got[at:at + n][see][:, :, col]).any())
+            want[at:at + n][see] = got[at:at + n][see]
+        at += n
+    same = (got == want) | (got.isnan() & want.isnan())
+    assert bool(same.all())

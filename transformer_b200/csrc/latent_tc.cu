@@ -83,6 +83,11 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
     const uint32_t sq = smem_base, ring = sq + boxes * LT_QBOX_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_lt + boxes * LT_QBOX_BYTES + LT_RING * LT_BOX_BYTES);
     uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + LT_BARS);
+    // What is no number stays with the rows that see it: a key that a row does not see has the weight 0, and 0 times an infinite or NaN
+    // value is NaN.  A key with such an entry has no finite score for any row, so a row that meets one at a masked place says so
+    // (suspect, by the page's parity, = the page's number + 1; suspect[2]: any page), the products' warp makes those entries of the
+    // page's values 0 before it multiplies them, and the epilogue adds them to the rows that do see them.
+    volatile uint32_t* suspect = &tmem_slot + 1;
     const int warp = warp_number(), lane = threadIdx.x & 31;
     if (smem_base & 1023u) {                              // never expected; refuse rather than compute garbage
         if (threadIdx.x == 0) atomicCAS(g.error, 0, 41);
@@ -104,6 +109,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
     auto p_ready = [&](int i) { return q_full + 32 + 8u * i; };
     auto o_done = [&](int i) { return q_full + 48 + 8u * i; };
     if (threadIdx.x == 0) {
+        suspect[0] = suspect[1] = suspect[2] = 0;
         for (int s = 0; s < LT_RING; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
@@ -121,6 +127,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // a page that not every row of the block sees whole
+    auto masked_page = [&](int key0) { return key0 + LT_KEYS - 1 > p_first || p_last - key0 >= a.window; };
     const uint32_t tmem_o = tmem_slot, tmem_s = tmem_slot + LT_COLS;      // page j: even sums at tmem_s + (j & 1) * 128, odd ones 64 further
 
     if (warp == 0) {
@@ -202,8 +210,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
             ok = mbar_wait_warp(p_ready(j & 1), (j >> 1) & 1, g.error, 45);
             if (!ok) break;
             tc_fence_after();
+            const bool look = suspect[j & 1] == (uint32_t)j + 1;
             for (int b = 0; b < LT_COLS / 64; ++b) {
                 if (!arrived()) break;
+                if (look) {
+                    uint32_t* box = reinterpret_cast<uint32_t*>(smem_lt + (ring - smem_base) + slot * LT_BOX_BYTES);
+                    for (int i = lane; i < LT_BOX_BYTES / 4; i += 32)
+                        if (not_finite_pair(box[i]) & 0x80008000u) box[i] = finite_pair(box[i]);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the product reads these writes
+                    __syncwarp();
+                }
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < LT_KEYS / 16; ++k)
@@ -275,11 +291,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
                 for (int i = 0; i < 32; ++i) v[half * 32 + i] = __fmul_rn(__uint_as_float(e[i]) + __uint_as_float(o[i]), a.scale);
             }
             const int key0 = (pg0 + j) * LT_KEYS;
-            // a page that not every row of the block sees whole
-            if (key0 + LT_KEYS - 1 > p_first || p_last - key0 >= a.window || !live) {
+            const bool masked = masked_page(key0);
+            if (masked || !live) {
+                bool odd = false;
 #pragma unroll
                 for (int i = 0; i < LT_KEYS; ++i)
-                    if (key0 + i > pos || pos - (key0 + i) >= a.window) v[i] = -INFINITY;
+                    if (key0 + i > pos || pos - (key0 + i) >= a.window) {
+                        odd |= !(fabsf(v[i]) < INFINITY);
+                        v[i] = -INFINITY;
+                    }
+                if (masked && odd) suspect[j & 1] = suspect[2] = j + 1;
             }
             float top = -INFINITY;
 #pragma unroll
@@ -337,6 +358,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
             ok = mbar_wait_warp(o_done((pages - 1) & 1), ((pages - 1) >> 1) & 1, g.error, 48);
             tc_fence_after();
         }
+        asm volatile("bar.sync 1, 128;" ::: "memory");      // suspect[2], as any of the four warps left it
         if (ok) {
             const float inv = live ? lm_finish(mx, sum, a.sinks, a.gate, a.ldg, t, h) : 0.f;
             __nv_bfloat16* out = a.out + ((size_t)t * a.H + h) * a.rank + part * LT_COLS;
@@ -345,6 +367,19 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_tc_kernel(const __grid_c
                 uint32_t x[32];
                 lt_ld32(tmem_o + lane_sel + c, x);        // warp-collective: rows without a query store nothing
                 lt_wait_ld();
+                if (live && suspect[2]) {
+                    for (int j = 0; j < pages; ++j) {
+                        const int key0 = (pg0 + j) * LT_KEYS;
+                        if (!masked_page(key0)) continue;
+                        const __nv_bfloat16* page = a.cache + (size_t)table[pg0 + j] * LT_KEYS * DK + part * LT_COLS + c;
+                        for (int k = max(0, pos - a.window + 1 - key0); k < LT_KEYS && key0 + k <= pos; ++k)
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                const float y = __bfloat162float(page[(size_t)k * DK + i]);
+                                if (!(fabsf(y) < INFINITY)) x[i] = __float_as_uint(__uint_as_float(x[i]) + y);
+                            }
+                    }
+                }
                 if (live) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
@@ -394,7 +429,7 @@ int tb_latent_attention_tc_bf16(const void* qa, const void* q, void* out, const 
                    err, tiles, rank / LT_COLS,
                    rdims % 16 == 0 && ldq % 8 == 0 && q_head % 8 == 0 && (q_head - rot) % 8 == 0 &&
                        !(((uintptr_t)q | (uintptr_t)cosT | (uintptr_t)sinT) & 15)};
-    const size_t smem = (size_t)((DK + 63) / 64) * LT_QBOX_BYTES + LT_RING * LT_BOX_BYTES + (LT_BARS + 1) * 8;
+    const size_t smem = (size_t)((DK + 63) / 64) * LT_QBOX_BYTES + LT_RING * LT_BOX_BYTES + (LT_BARS + 2) * 8;
     static PerDevice raised;
     tb_allow_smem(raised, (const void*)latent_tc_kernel, 227 * 1024);
     TB_LAUNCH((latent_tc_kernel), tiles * g.cols, LT_THREADS, smem, s, mq, mc, g);
