@@ -114,8 +114,8 @@ def test_chunks(dtype, G, H, dim, vdim, per_head, steep):
 
 @pytest.mark.parametrize("H,vdim,copies", [(4, 128, 5), (3, 32, 25), (3, 48, 17), (1, 256, 9), (1, 256, 10)])
 def test_scan_of_many_columns(H, vdim, copies):
-    """More blocks of 16 columns than SMs, where the scan takes 32 columns a block (not with 48), and just fewer (9 x 256): lengths
-    around a chunk's edges and an empty sequence.  The bound is that of `test_chunks`."""
+    """Many columns, with 16 and, where they come in 32s, with 32 of them a block, which give the same bits: lengths around a chunk's
+    edges and an empty sequence.  The bound is that of `test_chunks`."""
     from transformer_b200.csrc import lib
     gen, dim = torch.Generator().manual_seed(vdim + copies), 128
     lens = [(1, 15, 0, 16, 33, 50, 17)[i % 7] for i in range(copies)]
@@ -130,7 +130,12 @@ def test_scan_of_many_columns(H, vdim, copies):
     where = (lib.ptr(d[6]), lib.ptr(slots), nt, B, H, H, dim, vdim, 4, chunks)
     lib.call("tb_delta_chunk_f32", lib.ptr(d[0]), C, lib.ptr(d[1]), lib.ptr(state), *(lib.ptr(t) for t in d[2:6]), lib.ptr(rec), *where,
              H * dim, H, 0)
+    before, wide = state.clone(), vdim % 32 == 0
+    assert lib.try_call("tb_delta_chunk_scan_wide", lib.ptr(rec), lib.ptr(before), lib.ptr(o), *where) is wide
+    first = o.clone()
     lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where)
+    if wide:
+        assert torch.equal(o, first) and torch.equal(state, before)
     got = o.cpu().double().split(lens)
     assert not lib.library().tb_gemm_tc_status()
     for i, (xi, ai, bi) in enumerate(zip(x.split(lens), a.split(lens), bz.split(lens))):

@@ -13,12 +13,13 @@
 //                             solutions, one record for the scan
 //   delta_chunk_scan_kernel   a block = a sequence x a head x 16 or 32 columns of S
 // Measured with 16 heads of 128 x 128 (both kernels; before: records and scan token by token): one prompt of 2,048 tokens
-// 329 us (812), two of 1,500 353 (837), eight of 1,024 777 (1,770).  The first kernel is bound by instruction issue
+// 310 us (812), two of 1,500 351 (837), eight of 1,024 784 (1,770).  The first kernel is bound by instruction issue
 // and shared-memory reads in equal parts (34 KB and 64 registers a thread leave four blocks an SM); a warp leaves out the
-// tokens before its first key (136 to 128 us for two prompts of 1,500 tokens).  The scan of few sequences is bound by the
-// chain of a chunk (1.8 us; one block an SM), that of many by what goes through shared memory: a piece of a record that a
+// tokens before its first key (135 to 126 us for two prompts of 1,500 tokens).  The scan of few sequences is bound by the
+// chain of a chunk (1.7 us; one block an SM), that of many by what goes through shared memory: a piece of a record that a
 // lane loads serves its four columns, and 16 lanes to a column instead of 32 halve the exchange of the sums: eight
-// prompts 451 us (569 with 32 lanes), four of 600 142 (191), two of 1,500 226 (234).  Eight lanes to a column: 481 and 163.
+// prompts 465 us (563 with 32 lanes), four of 600 143 (188).  Eight lanes to a column: 481 and 163.  All forms add in one order and
+// have the same bits.
 #include "channel_delta.cuh"
 #include "memory_common.cuh"            // fma2, mul2
 #include "tc_common.cuh"                // bulk copies, barriers with bounded waits
@@ -28,7 +29,6 @@
 #define DC_BP 20            // pitch of B's rows: the 16 lanes that read a row each start in different banks
 #define DC_COLS 16          // columns of the state per scan block
 #define DC_STAGES 3
-#define DC_SMS 148          // of a B200
 
 // A record of one (head, chunk):  W | G q | G_last / G_j k, [16][dim] each | G_last [dim] | B [16][DC_BP], then
 // U0 as [vdim / 16][16 tokens][16 columns], so that a scan block's share is one piece.
@@ -218,10 +218,12 @@ struct DeltaChunkScanArgs {
 // 128 threads: LANES lanes share C columns and split the rows (DIM / LANES each, in registers, pieces of four
 // interleaved).  Per chunk: the sums over S for W and G q (16 tokens x C columns each), scattered so that every lane ends
 // with one token's sums for C or, of 32 lanes, C / 2 columns; u through shared memory to all lanes of the columns; the
-// update.  A lane takes the tokens in an order of its own (place t holds token t ^ its number), so the half that it gives
-// away is at the same places in every lane and nothing is selected.  The records come by bulk copy, two chunks ahead,
-// with bounded waits.
-template <int DIM, int LANES, int C>
+// update.  OWN: a lane takes the tokens in an order of its own (place t holds token t ^ its number), so the half that it gives
+// away is at the same places in every lane and nothing is selected.  With two rows' pieces a lane that is the faster way;
+// with one, where the chain of a chunk counts, the addresses that the lane's number enters cost more than the selects (one prompt of 2,048
+// tokens 235 us and 221; heads of 64: 179 and 157).  A lane's two pieces are summed apart and then together, as the
+// first exchange of 32 lanes has them.  The records come by bulk copy, two chunks ahead, with bounded waits.
+template <int DIM, int LANES, int C, bool OWN>
 __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkScanArgs a) {
     pdl_sync();
     constexpr int R4 = DIM / (4 * LANES), CB = LANES / DC_TOK, OUT = C / CB, COLS = 128 / LANES * C;
@@ -269,37 +271,43 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
         bulk_load(to + MAIN * sizeof(float), from + MAIN + (size_t)blockIdx.z * (DC_TOK * COLS), DC_TOK * COLS * sizeof(float), bar);
     };
     union Four { float4 f; F2 p[2]; };
-    // this lane's part of the sums over S for 16 rows of a record, then the lane's own sums
-    auto sums = [&](const float* rows, float (&mine)[OUT]) {
-        F2 sum[DC_TOK][C / 2];
+    // this lane's part of the sums over S for 16 rows of a record, [token][pair of columns]
+    auto sums = [&](const float* rows, F2 (&sum)[DC_TOK][C / 2]) {
 #pragma unroll
         for (int t = 0; t < DC_TOK; ++t) {
-            const float* row = rows + (t ^ my_tok) * DIM + part * 4;
-            F2 acc[C];
+            const float* row = rows + (OWN ? t ^ my_tok : t) * DIM + part * 4;
 #pragma unroll
             for (int r = 0; r < R4; ++r) {
                 Four w;
+                F2 acc[C];
                 w.f = *reinterpret_cast<const float4*>(row + r * (4 * LANES));
 #pragma unroll
-                for (int c = 0; c < C; ++c)
+                for (int c = 0; c < C; ++c) acc[c] = fma2(w.p[1], s[c][r * 2 + 1], mul2(w.p[0], s[c][r * 2]));
 #pragma unroll
-                    for (int e = 0; e < 2; ++e)
-                        acc[c] = r == 0 && e == 0 ? mul2(w.p[e], s[c][r * 2 + e]) : fma2(w.p[e], s[c][r * 2 + e], acc[c]);
+                for (int c = 0; c < C; c += 2) {
+                    F2 two;
+                    two.f = make_float2(acc[c].f.x + acc[c].f.y, acc[c + 1].f.x + acc[c + 1].f.y);
+                    sum[t][c / 2] = r == 0 ? two : add2(sum[t][c / 2], two);
+                }
             }
-#pragma unroll
-            for (int c = 0; c < C; c += 2) sum[t][c / 2].f = make_float2(acc[c].f.x + acc[c].f.y, acc[c + 1].f.x + acc[c + 1].f.y);
         }
+    };
+    // the lanes' parts together: every lane ends with its own token's columns (the same pairs of lanes are added in both forms)
+    auto meet = [&](F2 (&sum)[DC_TOK][C / 2], float (&mine)[OUT]) {
 #pragma unroll
-        for (int half = DC_TOK / 2; half > 0; half >>= 1)
+        for (int half = DC_TOK / 2; half > 0; half >>= 1) {
+            const bool up = my_tok & half;
 #pragma unroll
             for (int t = 0; t < half; ++t)
 #pragma unroll
                 for (int c = 0; c < C / 2; ++c) {
+                    const F2 keep = !OWN && up ? sum[t + half][c] : sum[t][c], give = !OWN && up ? sum[t][c] : sum[t + half][c];
                     F2 in;
-                    in.f.x = __shfl_xor_sync(0xffffffffu, sum[t + half][c].f.x, half * CB);
-                    in.f.y = __shfl_xor_sync(0xffffffffu, sum[t + half][c].f.y, half * CB);
-                    sum[t][c] = add2(sum[t][c], in);
+                    in.f.x = __shfl_xor_sync(0xffffffffu, give.f.x, half * CB);
+                    in.f.y = __shfl_xor_sync(0xffffffffu, give.f.y, half * CB);
+                    sum[t][c] = add2(keep, in);
                 }
+        }
 #pragma unroll
         for (int c = 0; c < OUT / 2; ++c) {
             F2 keep = sum[0][c];
@@ -328,7 +336,9 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
         const float* W = dc_sm + (size_t)(ch % DC_STAGES) * STAGE;
         const float* G = W + 3 * DC_TOK * DIM;
         float su[OUT], o[OUT];
-        sums(W, su);
+        F2 sw[DC_TOK][C / 2], sg[DC_TOK][C / 2];
+        sums(W, sw);
+        meet(sw, su);
         const int lc = group * C + my_col;
         const float* u0 = W + MAIN + lc / DC_COLS * (DC_TOK * DC_COLS) + my_tok * DC_COLS + lc % DC_COLS;
 #pragma unroll
@@ -336,8 +346,9 @@ __global__ void __launch_bounds__(128) delta_chunk_scan_kernel(const DeltaChunkS
             const float2 x = *reinterpret_cast<const float2*>(u0 + c);
             *reinterpret_cast<float2*>(&us[group][my_tok][my_col + c]) = make_float2(x.x - su[c], x.y - su[c + 1]);
         }
-        sums(W + DC_TOK * DIM, o);
+        sums(W + DC_TOK * DIM, sg);
         __syncwarp();           // the lanes of a group of columns are lanes of one warp
+        meet(sg, o);            // behind the hand-over of u: nothing in the update waits for it
 #pragma unroll
         for (int r = 0; r < R4; ++r) {
             Four gl;
@@ -411,15 +422,30 @@ static int delta_chunk_go(const DeltaPrepArgs& p, int nt, int B, int max_chunks,
     return tb_last_error();
 }
 
-template <int DIM, int LANES, int C>
+template <int DIM, int LANES, int C, bool OWN>
 static int delta_chunk_scan_go(const DeltaChunkScanArgs& a, int B, cudaStream_t s) {
     constexpr int COLS = 128 / LANES * C;
     constexpr size_t smem = (size_t)DC_STAGES * ((3 * DC_TOK + 1) * DIM + DC_TOK * DC_BP + DC_TOK * COLS) * sizeof(float);
     static PerDevice raised;
-    tb_allow_smem(raised, (const void*)delta_chunk_scan_kernel<DIM, LANES, C>, smem);
+    tb_allow_smem(raised, (const void*)delta_chunk_scan_kernel<DIM, LANES, C, OWN>, smem);
     // the blocks run for the whole sequence and want an SM each (see tb_launch_plain)
-    tb_launch_plain(delta_chunk_scan_kernel<DIM, LANES, C>, dim3(B, a.H, a.vdim / COLS), dim3(128), smem, s, a);
+    tb_launch_plain(delta_chunk_scan_kernel<DIM, LANES, C, OWN>, dim3(B, a.H, a.vdim / COLS), dim3(128), smem, s, a);
     return tb_last_error();
+}
+
+static int delta_chunk_scan_entry(const float* rec, float* state, float* out, const int* seq_start, const int* slots, int nt, int B,
+                                  int G, int H, int dim, int vdim, int taps, int max_chunks, bool wide, cudaStream_t s) {
+    if (nt < 0 || B < 0 || G <= 0 || H <= 0 || max_chunks < 0) return TB_ERR_ARG;
+    if (!delta_chunk_takes(dim, vdim, taps) || (wide && (dim != 128 || vdim % 32))) return TB_ERR_UNSUPPORTED;
+    if (((uintptr_t)rec & 15) || (((uintptr_t)state | (uintptr_t)out) & 7)) return TB_ERR_ARG;
+    if (nt == 0 || B == 0) return 0;
+    if (max_chunks < nt / DC_TOK + (B < nt ? B : nt)) return TB_ERR_ARG;
+    const long long per = (long long)H * dim * vdim + (taps - 1) * (2LL * G * dim + H * vdim);
+    if (per % 2) return TB_ERR_ARG;
+    DeltaChunkScanArgs a{rec, state, tc_error_ptr(), out, seq_start, slots, per, max_chunks, H, vdim};
+    if (!a.error) return tb_last_error();
+    if (wide) return delta_chunk_scan_go<128, 16, 4, true>(a, B, s);
+    return dim == 64 ? delta_chunk_scan_go<64, 16, 2, false>(a, B, s) : delta_chunk_scan_go<128, 32, 4, false>(a, B, s);
 }
 
 extern "C" {
@@ -453,19 +479,12 @@ TB_DELTA_CHUNK(bf16, __nv_bfloat16)
 
 int tb_delta_chunk_scan(const float* rec, float* state, float* out, const int* seq_start, const int* slots, int nt, int B,
                         int G, int H, int dim, int vdim, int taps, int max_chunks, cudaStream_t s) {
-    if (nt < 0 || B < 0 || G <= 0 || H <= 0 || max_chunks < 0) return TB_ERR_ARG;
-    if (!delta_chunk_takes(dim, vdim, taps)) return TB_ERR_UNSUPPORTED;
-    if (((uintptr_t)rec & 15) || (((uintptr_t)state | (uintptr_t)out) & 7)) return TB_ERR_ARG;
-    if (nt == 0 || B == 0) return 0;
-    if (max_chunks < nt / DC_TOK + (B < nt ? B : nt)) return TB_ERR_ARG;
-    const long long per = (long long)H * dim * vdim + (taps - 1) * (2LL * G * dim + H * vdim);
-    if (per % 2) return TB_ERR_ARG;
-    DeltaChunkScanArgs a{rec, state, tc_error_ptr(), out, seq_start, slots, per, max_chunks, H, vdim};
-    if (!a.error) return tb_last_error();
-    if (dim == 64) return delta_chunk_scan_go<64, 16, 2>(a, B, s);
-    // More than one block an SM: blocks of 32 columns.  Fewer leave SMs without one (one prompt of 2,048 tokens: 304 us, 237 so).
-    if (vdim % 32 == 0 && (long long)B * H * (vdim / DC_COLS) > DC_SMS) return delta_chunk_scan_go<128, 16, 4>(a, B, s);
-    return delta_chunk_scan_go<128, 32, 4>(a, B, s);
+    return delta_chunk_scan_entry(rec, state, out, seq_start, slots, nt, B, G, H, dim, vdim, taps, max_chunks, false, s);
+}
+// The same, to the bit, with 32 columns a block (see wide_scan_pays in parts/channel_delta.py); heads of 128, vdim a multiple of 32.
+int tb_delta_chunk_scan_wide(const float* rec, float* state, float* out, const int* seq_start, const int* slots, int nt, int B,
+                             int G, int H, int dim, int vdim, int taps, int max_chunks, cudaStream_t s) {
+    return delta_chunk_scan_entry(rec, state, out, seq_start, slots, nt, B, G, H, dim, vdim, taps, max_chunks, true, s);
 }
 }
 
@@ -473,3 +492,4 @@ int tb_delta_chunk_scan(const float* rec, float* state, float* out, const int* s
 TB_TAPE_REGISTER(tb_delta_chunk_f32)
 TB_TAPE_REGISTER(tb_delta_chunk_bf16)
 TB_TAPE_REGISTER(tb_delta_chunk_scan)
+TB_TAPE_REGISTER(tb_delta_chunk_scan_wide)

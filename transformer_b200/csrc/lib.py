@@ -77,7 +77,7 @@ _SIGNATURES: Dict[str, str] = {
     "tb_delta_prep_bf16": "pipppppppppppiiiiiiiiiii",
     "tb_delta_scan": "ppppppiiiiiii",
     "tb_delta_chunk_f32": "pipppppppppiiiiiiiiiii", "tb_delta_chunk_bf16": "pipppppppppiiiiiiiiiii",
-    "tb_delta_chunk_scan": "pppppiiiiiiii",
+    "tb_delta_chunk_scan": "pppppiiiiiiii", "tb_delta_chunk_scan_wide": "pppppiiiiiiii",
     "tb_gemm_tc_bias_glu_bf16": "ppppiiiiiii", "tb_gemm_skinny_bias_glu_bf16": "ppppiiiiiii",
     "tb_bias_glu_f32": "pppiii", "tb_bias_glu_bf16": "pppiii",
     "tb_router_sigmoid_f32": "ppppppppiiii", "tb_router_sigmoid_bf16": "ppppppppiiii",

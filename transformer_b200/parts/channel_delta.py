@@ -31,10 +31,19 @@ from .linear import matmul_nt
 # A step of more tokens than this a sequence, on average, takes 16 tokens at a time (csrc/channel_delta_chunk.cu), where that
 # kernel takes the heads.  It is the faster form from some 20 tokens a sequence on (16 heads of 128, both kernels, us: 16 x 8
 # tokens 65 there and 63 token by token, 1 x 64 32 and 46, 8 x 70 91 and 145, 1 x 320 a tenth of a millisecond apart, 1 x 2,048
-# 294 and 812); the line is kept where it is because the forms round differently (both in float: 1e-5 of the largest value
+# 310 and 812); the line is kept where it is because the forms round differently (both in float: 1e-5 of the largest value
 # from the 64-bit recurrence) and a request's short prompts keep the bits they had.  The average is the step's: which form a
 # prompt takes, and so its last bits, depends on the sequences that share its step and on where a step is cut.
 CHUNK_MEAN = 320
+
+
+def wide_scan_pays(lens, H: int, dim: int, vdim: int, sms: int) -> bool:
+    """Whether the scan of such chunks is faster with 32 columns a block (16 lanes to a column) than with 16 (32 lanes): where every SM has
+    so many columns that the longest sequence's chain, longer there, does not end last.  The same bits.  us, 16 heads of 128 x 128,
+    16 and 32 columns: 3 x 700 tokens 181 and 165, 4 x 600 185 and 143, 8 x 1,024 551 and 465, 1,000 + 900 + 400 + 300 260 and 233, of 2,000
+    and shorter ones to 300 (eight) 619 and 580; not taken: 2,048 222 and 314, 2 x 1,500 225 and 232, 600 + 1,000 + 400 201 and 233,
+    1,800 + 3 x 200 303 and 410."""
+    return dim == 128 and vdim % 32 == 0 and 2 * max(lens) * sms <= sum(lens) * H * (vdim // 16)
 
 
 @MIXERS.register("channel_delta")
@@ -132,7 +141,10 @@ class ChannelDelta(Mixer):
             lib.call("tb_delta_chunk_" + sfx, lib.ptr(z), self.z_width, lib.ptr(w["conv"]), lib.ptr(state), lib.ptr(a),
                      lib.ptr(w["dt_bias"]), lib.ptr(w["A_log"]), lib.ptr(bz), lib.ptr(rec), *where, chunks, a.stride(0),
                      bz.stride(0), per_head)
-            lib.call("tb_delta_chunk_scan", lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where, chunks)
+            key = ("delta_scan", H, self.dim, self.vdim)
+            if key not in ctx.plans:
+                ctx.plans[key] = "_wide" if wide_scan_pays(ctx.h_lens, *key[1:], ctx.engine.sm_count) else ""
+            lib.call("tb_delta_chunk_scan" + ctx.plans[key], lib.ptr(rec), lib.ptr(state), lib.ptr(o), *where, chunks)
         else:
             # what enters the recurrence, float: one record per (token, head) [q | k | decay | beta, k.q], and the values
             rec = ctx.scratch("delta.rec", (nt, H, lib.delta_record_size(self.dim)), torch.float32)
