@@ -12,7 +12,7 @@ import torch
 from ..csrc import lib
 from .base import FEED_FORWARDS, FeedForward, NormTail, ParamDecl, WeightedRows
 from . import linear
-from .linear import bias_glu_matmul, gemm_skinny, grouped_matmul, matmul_nt
+from .linear import bias_glu_matmul, bias_glu_pays, gemm_skinny, grouped_matmul, matmul_nt
 
 ROUTER_ROWS_FROM = 256      # above this many tokens the router works on tiles of 16 tokens (tensor cores)
 ROUTER_TAIL_ROWS = 256      # up to this many tokens the norm before the experts also routes
@@ -24,7 +24,7 @@ class DenseSwiGLU(FeedForward):
     out = h Wd^T (compute.rs:278-292).  With ``bias`` all three projections have one: ``bgu`` (gate's, then up's)
     and ``bd``, float.  The down projection's bias rides inside its product: the bound weight gets the bias as one
     more column (and zeros up to a multiple of eight), and the kernel that applies the pair's biases and the
-    activation (in bfloat16 the product's epilogue) writes a one into that column of ``h``.  ``glu_limit`` (with ``glu_alpha``, default 1): the pair
+    activation (in bfloat16 the product's epilogue, where that is faster) writes a one into that column of ``h``.  ``glu_limit`` (with ``glu_alpha``, default 1): the pair
     becomes g' * sigmoid(alpha g') * (u' + 1) with g' = min(g, limit), u' = clamp(u, -limit, limit) instead of
     silu(g) * u, in the product's epilogue.  ``act`` = "gelu_tanh": gelu(g) * u with the tanh form of gelu, there too."""
     graph_safe = True
@@ -66,7 +66,7 @@ class DenseSwiGLU(FeedForward):
         if self.bias:
             wide = self.weights["wd"].shape[1]
             h = ctx.scratch("ff.h1", (nt, wide), self.dtype)
-            if bias_glu_matmul(x1, self.weights["wgu"], self.weights["bgu"], h):
+            if bias_glu_pays(nt, self.di, x1.shape[1]) and bias_glu_matmul(x1, self.weights["wgu"], self.weights["bgu"], h):
                 matmul_nt(h, self.weights["wd"], out)
                 return
             gu = ctx.scratch("ff.gu", (nt, 2 * self.di), self.dtype)

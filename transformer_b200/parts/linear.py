@@ -128,6 +128,20 @@ def matmul_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, w_is_weigh
         torch.mm(a, w.t(), out=out)
 
 
+def bias_glu_pays(M: int, n: int, K: int) -> bool:
+    """Whether :func:`bias_glu_matmul` is faster than the product and the pass over it (bfloat16; the same bits).  us, the two launches and
+    the one kernel (n x K):
+      few rows, the streaming kernel both times: 1 row 2,816 x 1,024 7.2 and 4.3, 5,632 x 2,048 12.7 and 11.4, 8 rows 13.8 and 11.8; not
+        taken: 11,008 x 4,096 31.0 and 34.0 (the two matrices side by side in a block), 16 rows of 5,632 x 2,048 16.4 and 17.3
+      more rows, library product and pass against tcgen05: 1,500 rows of 5,632 x 2,048 63 and 57, 2,048 90 and 71, 3,000 124 and 104,
+        2,048 of 5,632 x 1,024 60 and 55, 4,096 of 2,816 x 1,024 58 and 55, 3,000 of 11,008 x 4,096 429 and 432; not taken: 17 rows of 2,816 x
+        1,024 7.2 and 16.3, 100 of 5,632 x 2,048 14.0 and 24.4, 512 27 and 33, 850 38 and 43, 1,000 of 11,008 x 4,096 149 and 155,
+        1,200 of 2,816 x 4,096 45 and 51, 2,048 of 2,816 x 1,024 31 and 36."""
+    if M <= SKINNY_MAX_ROWS:
+        return n * K <= (20_000_000 if M <= 8 else 8_000_000)
+    return M >= 1500 and M * n * K >= 10 ** 10
+
+
 def bias_glu_matmul(a, w, bias, h) -> bool:
     """h[:, :n] = silu(gate + bias[:n]) * (up + bias[n:]), (gate, up) = a @ w.T with w [2 n, K]; a one and zeros in what columns h has
     behind.  The bits of the product stored in bfloat16 and a pass over it.  False (and nothing done) where no kernel takes it."""
