@@ -56,8 +56,8 @@ struct SkinnyArgs {
     int by_row;
     GluRule glu;            // DUAL: how the (gate, up) pair becomes one value
     // One weight matrix with short rows (K < 2,048): what a thread's registers do not take before the wait is asked into L2.  Steps of one
-    // sequence of width 1,024, 8 layers, vocabulary 32,000: 1,042 to 1,018 us for four.  Longer rows lose: K 4,096, 32 layers of one
-    // sequence +3 % (the kernel before still reads from memory).
+    // sequence of width 1,024, 8 layers, vocabulary 32,000: 950 to 942 us for four, both in one run whose repeats agree within 1 us.  Longer
+    // rows lose: K 4,096, 32 layers of one sequence +3 % (the kernel before still reads from memory).
     int ahead;
 };
 

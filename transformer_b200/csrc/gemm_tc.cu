@@ -73,7 +73,6 @@ struct TcArgs {
     int tiles_m;        // row tiles (with groups: an upper bound; tiles past the last group are skipped)
     int n_tile;         // rows of B in a tile: a multiple of 16 up to TC_BN (fewer when that fills the SMs better)
     GluRule glu;        // dual: how the (gate, up) pair becomes one value
-    int ahead;          // k-blocks of weights that are asked into L2 before the kernel's wait
 };
 
 // ---- the kernel ----------------------------------------------------------------------------
@@ -134,16 +133,6 @@ template <int CTAS, int EPI>
 __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                             const __grid_constant__ CUtensorMap map_b,
                                                             const TcArgs a) {
-    if (CTAS == 1 && a.ahead && threadIdx.x == 0) {
-        // Which weights the block's first tile needs is known before the rows' offsets are, if no group has more than a tile of
-        // rows and none is empty: they are asked into L2 while the kernels before this one end.  A wrong guess costs its bytes.
-        const int n_out = a.dual ? a.n_tile / 2 : a.n_tile, tiles_n = (a.N + n_out - 1) / n_out, g = (int)blockIdx.x / tiles_n;
-        const int row = g * a.b_group_rows + ((int)blockIdx.x - g * tiles_n) * n_out, n = min(a.ahead, (a.K + TC_BK - 1) / TC_BK);
-        for (int kb = 0; kb < n && g < a.G; ++kb) {
-            tma_prefetch_2d(&map_b, kb * TC_BK, row);
-            tma_prefetch_2d(&map_b, kb * TC_BK, row + (a.dual ? a.N : a.n_tile / 2));
-        }
-    }
     pdl_sync();
     extern __shared__ uint8_t smem_raw[];
     constexpr int TC_STAGES = TcShape<CTAS>::STAGES, TC_STAGE_BYTES = TcShape<CTAS>::STAGE_BYTES;
@@ -615,10 +604,7 @@ static int gemm_tc_entry(const void* A, const void* B, void* C, const int* group
     if (rc) return rc;
     int* err_ptr = tc_error_ptr();
     if (!err_ptr) return tb_last_error();
-    TcArgs a{C, group_offsets, err_ptr, ldc, M, N, K, G, rows_b, dual, 0, n_tile, glu,
-             // at most a tile of rows a group, on average: 8 of them (a prompt of 131 tokens through 8 layers of 16 experts 1,268 us
-             // without, 1,246 with 4 or 8, 1,253 with 16, 1,288 with 64)
-             (long long)M <= (long long)TC_BM * G ? 8 : 0};
+    TcArgs a{C, group_offsets, err_ptr, ldc, M, N, K, G, rows_b, dual, 0, n_tile, glu};
     if (glu.bias) {
         rc = pair ? tc_launch<2, TC_EPI_BIASED>(ma, mb, a, s) : TB_ERR_UNSUPPORTED;
         if (rc == TB_ERR_UNSUPPORTED) rc = tc_launch<1, TC_EPI_BIASED>(ma, mb, a, s);
