@@ -1,5 +1,6 @@
 """Products by pairs of blocks on the tensor cores, at sizes around the rule that chooses them: the bits of the same product made in pieces
 of at most 128 rows (which single blocks take: a tcgen05 product adds along K in one order), and a few columns against 64 bits.
+Which form a product takes is asked of the rule itself, so a case says where it lies.
 
 The bound of the second: float sums of K products of bfloat16 values, error at most K 2^-24 of the sum of their absolute values,
 and one rounding to bfloat16 (2^-9 of the value), through the pair's silu(g) u (slope at most 1.1) at most doubled.  With biases both
@@ -7,7 +8,12 @@ products are rounded to bfloat16 before these are added: 2^-9 of either product,
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
+SMS = 148       # of the GPU that the rule was measured on
+
+
+def _takes_pairs(rows, N, K, kind, sms=SMS):
+    from transformer_b200.csrc import lib
+    return bool(lib.library().tb_gemm_tc_takes_pairs(sum(rows), N, K, len(rows), int(len(rows) > 1), min(kind, 2), sms))
 
 
 def _call(a, w, out, offsets, N, kind, bias=None):
@@ -20,12 +26,28 @@ def _call(a, w, out, offsets, N, kind, bias=None):
                  M, N, K, w.shape[0], kind)
 
 
-@pytest.mark.parametrize("rows,N,K,kind", [
-    ([1300], 2000, 1032, 2), ([1299], 2008, 1024, 3), ([385], 20000, 1032, 1), ([1025], 4104, 2048, 0), ([300], 5632, 1024, 2), ([512], 18944, 1024, 1),
-    ([0, 257, 1, 700, 256, 255, 511, 3, 129, 900, 0, 40, 513, 300, 128, 600], 688, 1024, 2),
-    ([600, 1, 2047, 300, 1000, 260, 512, 0], 2056, 520, 0), ([600, 0, 700, 500], 4096, 688, 0)])
-def test_pairs(rows, N, K, kind):
+@pytest.mark.parametrize("rows,N,K,kind,pairs", [
+    ([3000], 2048, 128, 0, False), ([3000], 2048, 504, 0, False), ([3000], 2048, 512, 0, True), ([128], 32000, 2048, 1, False), ([129], 32000, 2048, 1, True),
+    ([200], 5632, 4096, 2, False), ([128] * 16, 688, 4096, 2, False), ([129] * 16, 688, 4096, 2, True), ([512] * 16, 688, 4096, 2, False),
+    ([640] * 16, 688, 4096, 2, True), ([512] * 8, 14336, 4096, 2, False), ([1024] * 8, 14336, 4096, 2, True), ([512] * 8, 4096, 14336, 0, False), ([511] * 16, 4096, 688, 0, False),
+    ([512] * 16, 4096, 688, 0, True)])
+def test_sides_of_the_line(rows, N, K, kind, pairs):
+    assert _takes_pairs(rows, N, K, kind) is pairs
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,N,K,kind,pairs", [
+    ([1300], 2000, 1032, 2, True), ([1299], 2008, 1024, 3, True), ([385], 20000, 1032, 1, True), ([1025], 4104, 2048, 0, True),
+    ([300], 5632, 1024, 2, False), ([512], 18944, 1024, 1, True), ([3000], 2048, 504, 0, False), ([3000], 2048, 520, 0, True),
+    ([0, 257, 1, 700, 256, 255, 511, 3, 129, 900, 0, 40, 513, 300, 128, 600], 688, 1024, 2, False),
+    ([384, 0, 500, 257, 1, 768, 129, 600, 450, 300, 420, 512, 380, 700, 390, 353], 688, 1032, 2, True),
+    ([0, 257, 1, 1500, 256, 755, 511, 3, 129, 2100, 0, 740, 513, 1300, 828, 1400], 688, 1024, 2, True),
+    ([700, 0, 640, 1, 900, 129, 257, 1030], 1408, 1032, 2, True),
+    ([600, 1, 2047, 300, 1000, 260, 512, 0], 2056, 520, 0, True), ([600, 0, 700, 500], 4096, 688, 0, False)])
+def test_pairs(rows, N, K, kind, pairs):
     from transformer_b200.csrc import lib
+    if torch.cuda.get_device_properties(0).multi_processor_count == SMS:
+        assert _takes_pairs(rows, N, K, kind, 0) is pairs
     gen = torch.Generator(device="cuda").manual_seed(N + K)
     M, G, dual = sum(rows), len(rows), kind >= 2
     a = torch.randn(M, K, device="cuda", generator=gen).bfloat16()

@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer: the leader's one thread, for the pair ----------------
+        // ---------------- MMA issuer: one thread, or of a pair the leader's warp for both blocks ----------------
         if ((PAIR || lane == 0) && rank == 0) {
             const uint32_t idesc = umma_idesc(TcShape<CTAS>::ROWS, a.n_tile);
             bool ok = true;
@@ -356,8 +356,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                     continue;
                 }
                 if (FLOAT && wide_float) {
-                    // the same for floats: a chunk's 32 columns are a whole line.  (Logits of 1,000 rows, K 2,048, N 32,000: 290 us
-                    // row by row, 150 so.)
+                    // the same for floats: a chunk's 32 columns are a whole line.  (Logits of 1,000 rows, K 2,048, N 32,000, single blocks: 290 us
+                    // row by row, 174 so.)
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         *reinterpret_cast<float4*>(strip + lane * 128 + ((j ^ (lane & 7)) << 4)) =
@@ -547,6 +547,28 @@ static int tc_sms() {
     return sms;
 }
 
+static int tc_tiles_n(int N, bool dual) { return (N + (dual ? TC_BN / 2 : TC_BN) - 1) / (dual ? TC_BN / 2 : TC_BN); }
+
+// Pairs of blocks, where they take at most a seventh more rounds over the SMs than single blocks would (a round of theirs takes about 7/8 of the
+// time: B is staged once for 256 rows), counting half a tile of padding a group.  What fits one round stays with single blocks, and so does
+// a short K (below 512, or 1,024 with fewer than 512 rows a group), whose start counts.  Products of a millisecond and more run at the power
+// limit, where what is computed counts, padding with it: from 16 rounds on with K from 4,096 a fourteenth more.  Single blocks / pairs, us
+// (many launches between two events, weights from memory; profiles/gemm_tc_pairs.md has more):
+//   (gate, up) 5,632 wide, K 2,048: 520 rows 29.5 / 27.0, 1,000 45 / 40, 2,048 79 / 69, 4,096 158 / 135; 300 rows 18.0 / 25.6 (1 round, 2)
+//   logits of 32,000 tokens, K 2,048: 200 rows 48 / 35, 500 94 / 67, 1,000 179 / 123; 64 rows 33 / 46
+//   16 experts, (gate, up) 688 wide, K 4,096: 200 rows each 60 / 56, 384 87 / 85, 640 130 / 116, 1,024 182 / 165; 512 99 / 112 (3 rounds, 4)
+//   their down product (4,096 wide, K 688): 512 rows each 62 / 57, 1,024 116 / 98, 2,048 198 / 171; 128 34 / 36
+//   8 experts 14,336 wide, K 4,096: 512 rows each 835 / 993 and 840 / 958 one after the other, 828 / 829 and 777 / 803 in turn (28 rounds,
+//   31), 768 1,240 / 1,169, 1,024 1,544 to 1,703 / 1,338 to 1,606, 2,048 2,904 to 3,088 / 2,538 to 2,995
+//   2,048 wide, K 128: 3,000 rows 6.8 / 7.5
+static bool tc_takes_pairs(int M, int N, int K, int G, bool grouped, bool dual, int sms) {
+    if (M <= TC_BM * (long long)G || K < (M >= 512ll * G ? 512 : 1024)) return false;
+    const long long pad = grouped ? G : 0, tiles_n = tc_tiles_n(N, dual);
+    const long long single = (((long long)M + TC_BM - 1) / TC_BM + pad / 2) * tiles_n, twos = (((long long)M + 2 * TC_BM - 1) / (2 * TC_BM) + pad / 2) * tiles_n;
+    const long long rounds = (single + sms - 1) / sms, pair_rounds = (twos + sms / 2 - 1) / (sms / 2);
+    return rounds >= 2 && (K >= 4096 && rounds >= 16 ? 13 * pair_rounds <= 14 * rounds : 7 * pair_rounds <= 8 * rounds);
+}
+
 // C[m] = A[m] . B[g(m)]^T.  A [M, K] (rows sorted by group), B [G, rows_b, K] with rows_b = N (or 2N when
 // out_kind == 2: gate rows then up rows).  out_kind: 0 bfloat16, 1 float, 2 swiglu (bfloat16).
 // Refuses (TB_ERR_UNSUPPORTED) what TMA cannot address: K or a pitch that is no multiple of 8,
@@ -561,21 +583,8 @@ static int gemm_tc_entry(const void* A, const void* B, void* C, const int* group
     const int rows_b = dual ? 2 * N : N;
     // Rows of B per tile: as many column tiles as the full width would need, but of equal widths (N = 688 with
     // swiglu: six tiles of 120 gate and 120 up rows instead of five of 128 and one of 48 padded to 128).
-    const int sms = tc_sms(), out_max = dual ? TC_BN / 2 : TC_BN, tiles_n = (N + out_max - 1) / out_max;
-    // Pairs of blocks, where their rounds over the SMs are not too many more than the single blocks' (a round of theirs takes 7/8 of the
-    // time: B is staged once for 256 rows), counting half a tile of padding a group.  What one round holds starts 2 us earlier in single
-    // blocks, and with a short K that start counts up to 512 rows a group.  Single blocks / pairs, us:
-    //   (gate, up) 5,632 wide, K 2,048: 520 rows 39.8 / 34.8, 1,000 51 / 45, 2,048 78 / 68, 3,451 124 / 109; 300 rows 28.7 / 33.7 (1 round, 2)
-    //   logits of 32,000 tokens, K 2,048: 200 rows 62 / 46, 500 100 / 72, 1,000 174 / 118; 64 rows 41 / 44
-    //   16 experts, (gate, up) 688 wide, K 4,096: 200 rows each 74 / 66, 384 96 / 84, 512 96 / 104 (3 rounds, 4), 1,024 166 / 148
-    //   their down product (4,096 wide, K 688): 512 rows each 64 / 59, 1,024 104 / 92, 2,048 197 / 163; 2,048 wide, K 704: 384 31 / 33
-    bool pair = false;
-    if (M > TC_BM * (long long)G && (K >= 1024 || M >= 512ll * G)) {
-        const long long pad = group_offsets ? G : 0;
-        const long long single = (((long long)M + TC_BM - 1) / TC_BM + pad / 2) * tiles_n, twos = (((long long)M + 2 * TC_BM - 1) / (2 * TC_BM) + pad / 2) * tiles_n;
-        const long long rounds = (single + sms - 1) / sms, pair_rounds = (twos + sms / 2 - 1) / (sms / 2);
-        pair = rounds >= 2 && 7 * pair_rounds <= 8 * rounds;
-    }
+    const int sms = tc_sms(), tiles_n = tc_tiles_n(N, dual);
+    const bool pair = tc_takes_pairs(M, N, K, G, group_offsets != nullptr, dual, sms);
     int n_tile;
     {
         const int unit = (pair ? 32 : 16) >> dual;      // a pair's B tile is a multiple of 32 rows
@@ -636,6 +645,11 @@ int tb_gemm_tc_bias_glu_bf16(const void* A, const void* B, const float* bias, vo
                              int fill, cudaStream_t s) {
     if (!bias || fill < 0 || ldc < N + fill) return TB_ERR_ARG;
     return gemm_tc_entry(A, B, C, nullptr, lda, ldb, ldc, M, N, K, 1, 2, GluRule{0, 0.f, 0.f, bias, fill}, s);
+}
+
+// Whether tb_gemm_tc_bf16 takes pairs of blocks on a GPU of so many SMs (0: on this one).
+int tb_gemm_tc_takes_pairs(int M, int N, int K, int G, int grouped, int out_kind, int sms) {
+    return tc_takes_pairs(M, N, K, G, grouped != 0, out_kind == 2, sms > 0 ? sms : tc_sms());
 }
 
 // Nonzero if any tensor-core product gave up on a wait since the last call (1 producer, 2 MMA,

@@ -134,7 +134,7 @@ class TapeMap(ctypes.Structure):
 
 _NO_STREAM = {"tb_decay_scan_rect_record_size": "ii", "tb_split_delta_record_size": "i",
               "tb_decay_state_size": "iii", "tb_decay_record_size": "i",
-              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_gates": "", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_latent_tc_tile_tokens": "iii", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
+              "tb_attention_window_mma_tile_tokens": "ii", "tb_delta_state_size": "iiiii", "tb_delta_record_size": "i", "tb_delta_scan_lanes": "i", "tb_delta_chunk_record_size": "iii", "tb_delta_chunk_tokens": "", "tb_delta_value_pitch": "i", "tb_mlstm_state_size": "ii", "tb_mlstm_parallel_size": "iiii", "tb_mlstm_parallel_gates": "", "tb_mlstm_parallel_tokens": "", "tb_latent_attention_tile_tokens": "i", "tb_latent_tc_tile_tokens": "iii", "tb_attention_tile_tokens": "ii", "tb_gemm_tc_takes_pairs": "iiiiiii", "tb_gemm_tc_status": "", "tb_attention_prefill_tile_tokens": "",
               "tb_attention_tc_tile_tokens": ""}
 
 _lock = threading.Lock()
