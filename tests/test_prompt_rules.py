@@ -3,6 +3,7 @@ from types import SimpleNamespace
 
 import pytest
 
+from transformer_b200.parts.attention import window_tcgen05_pays
 from transformer_b200.parts.channel_delta import wide_scan_pays
 from transformer_b200.parts.latent_attention import tc_pays
 
@@ -28,3 +29,14 @@ def test_delta_scan(lens, H, dim, vdim, pays):
 def test_latent_attention(heads, lens, before, pays):
     ctx, m = _step(lens, before), SimpleNamespace(tc_tile=128 // heads)
     assert tc_pays(ctx, m) is pays and tc_pays(ctx, m) is pays
+
+
+@pytest.mark.parametrize("nh,nkvh,dh,lens,before,window,chunk,pays", [
+    (16, 4, 128, [2048], [0], 2048, 0, True), (16, 4, 128, [600] * 2, [0] * 2, 2048, 0, True), (16, 4, 128, [300], [0], 2048, 0, True),
+    (16, 4, 128, [400] * 4, [1500] * 4, 2048, 0, True), (16, 16, 128, [2048], [0], 64, 0, True), (64, 1, 128, [512], [4000], 2048, 0, True),
+    (8, 8, 64, [600] * 2, [0] * 2, 2048, 0, True), (2, 1, 128, [2048], [0], 2048, 0, False), (4, 4, 128, [512], [512], 2048, 0, False),
+    (16, 4, 128, [300] * 4, [0] * 4, 64, 0, False), (16, 4, 128, [300] * 4, [0] * 4, 2048, 64, False), (64, 1, 128, [300] * 4, [0] * 4, 2048, 0, False),
+    (8, 1, 64, [600] * 2, [0] * 2, 64, 0, False), (16, 4, 128, [129] * 8, [0] * 8, 2048, 0, False), (16, 4, 64, [512], [4000], 2048, 0, False)])
+def test_windowed_attention(nh, nkvh, dh, lens, before, window, chunk, pays):
+    ctx, m = _step(lens, before), SimpleNamespace(tc_tile=128, nh=nh, nkvh=nkvh, dh=dh, chunk=chunk)
+    assert window_tcgen05_pays(ctx, m, window) is pays and window_tcgen05_pays(ctx, m, window) is pays

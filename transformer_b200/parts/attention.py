@@ -480,18 +480,25 @@ class Attention(Mixer):
                             ctx.max_pages, self.qkv_width, self.nh, self.nkvh, self.dh, splits, self.scale)
 
 
-def window_tcgen05_pays(ctx, m) -> bool:
+def window_tcgen05_pays(ctx, m, window) -> bool:
     """Whether a step's windowed attention is faster with 128 tokens of a head a block on the tcgen05 tensor cores than with the
-    mma.sync kernel's 64 rows of a head group, which can cut the keys into slices as well.  From 256 tokens a sequence on,
-    on average, if no sequence goes on behind more cached tokens than it brings or the blocks fill the SMs.  us, mma.sync and
-    tcgen05, 16 heads of 128 over 4 key heads, window 2,048, capped scores: 300 tokens 26 and 19, 2 x 600 42 and 28, 2,048 110
-    and 63 (uncapped 103 and 44), 4 x 400 behind 1,500 108 and 84; not taken: 8 x 129 20 and 23, 64 behind 2,000 33 and 60,
-    64 x 3 behind 500 26 and 95.  Heads of 64 from 80 blocks on: 8 heads, 2 x 600 25 and 23, 1,000 28 and 32."""
-    key = ("window_tc", m.tc_tile, m.nh, m.dh)
+    mma.sync kernel's 64 rows of a head group, which can cut the keys into slices as well.  From 256 tokens a sequence on, on average,
+    but where slices make few blocks' chains of pages shorter (below 40 blocks, or 80 with heads of 64), where the window is short and the tiles
+    not full (a tile of 128 tokens visits two pages more than one of 16), and where the tiles are a fifth empty and either heads of 64
+    or 64 heads on a key head, whose pages the other kernel reads once, have few pages to visit.  us, mma.sync and tcgen05, heads of
+    128, capped scores (840 shapes measured, none of those taken more than 4 % slower): 16 heads over 4, window 2,048: 2,048 tokens 110 and 67,
+    2 x 600 41 and 29, 300 25 and 20, 4 x 400 behind 1,500 108 and 90; 16 over 16, 2,048 tokens, window 64 43 and 28; 64 over 1, 512 behind
+    4,000 224 and 106; not taken: 2 over 1, 2,048 tokens 42 and 64; 4 over 4, 512 behind 512 26 and 39; 16 over 4, 4 x 300, window 64
+    24 and 27; 64 over 1, 4 x 300 62 and 68; 8 over 1, heads of 64, 2 x 600, window 64 12 and 13."""
+    reach = min(window, m.chunk) if m.chunk else window
+    key = ("window_tc", m.tc_tile, m.nh, m.nkvh, m.dh, reach)
     if key not in ctx.plans:
-        blocks = ctx.tiles(m.tc_tile).count * m.nh
-        fills = blocks >= ctx.engine.sm_count or all(b <= n for b, n in zip(ctx.h_pos0, ctx.h_lens))
-        ctx.plans[key] = ctx.nt >= 256 * ctx.B and fills and (m.dh != 64 or blocks >= 80)
+        tiles = ctx.tiles(m.tc_tile).count
+        blocks, full = tiles * m.nh, ctx.nt / max(1, tiles * m.tc_tile)
+        pages = max(min((b + n + 63) // 64, reach // 64 + 3) for b, n in zip(ctx.h_pos0, ctx.h_lens))
+        few = blocks < 8 or (blocks < 40 and (pages > 5 or reach < 256)) or (m.dh == 64 and blocks < 80 and pages > 8)
+        ctx.plans[key] = ctx.nt >= 256 * ctx.B and not few and \
+            (full >= 0.95 or (reach >= 256 and (full >= 0.8 or pages > 8 or (m.dh > 64 and m.nh < 64 * m.nkvh))))
     return ctx.plans[key]
 
 
@@ -510,7 +517,7 @@ def run_window_attention(ctx, m, z, o, gate, cache, table, nt, window, q_stride=
     q_stride = m.qkv_width if q_stride is None else q_stride
     g_stride = m.qkv_width if gate is None else gate.stride(0)
     if m.window_tile and USE_WINDOW_MMA:
-        if m.tc_tile and USE_TCGEN05 and not ctx.decode and ocos is None and dist_bias is None and window_tcgen05_pays(ctx, m):
+        if m.tc_tile and USE_TCGEN05 and not ctx.decode and ocos is None and dist_bias is None and window_tcgen05_pays(ctx, m, window):
             # prompts: S and O in tensor memory, K and V pages by TMA
             tiles = ctx.tiles(m.tc_tile)
             per_head, mult, ldo = heads or (0, 1.0, o.stride(0))
