@@ -39,7 +39,7 @@ def test_latent_prompts(monkeypatch, heads, rank, rot):
     assert bool(torch.isfinite(got).all()) and torch.equal(got, want)
 
 
-@pytest.mark.parametrize("heads,kv_heads,window,cap", [(8, 2, 200, 30.0), (4, 4, 4096, 0.0)])
+@pytest.mark.parametrize("heads,kv_heads,window,cap", [(8, 2, 300, 30.0), (4, 4, 4096, 0.0)])
 def test_windowed_prompts(monkeypatch, heads, kv_heads, window, cap):
     from transformer_b200.parts import attention
     att = {"heads": heads, "kv_heads": kv_heads, "dim": 128, "vdim": 128, "scale": 128 ** -0.5, "mask": {"size": window, "keep_first": 4},
