@@ -29,7 +29,7 @@ def _call(a, w, out, offsets, N, kind, bias=None):
 @pytest.mark.parametrize("rows,N,K,kind,pairs", [
     ([3000], 2048, 128, 0, False), ([3000], 2048, 504, 0, False), ([3000], 2048, 512, 0, True), ([128], 32000, 2048, 1, False), ([129], 32000, 2048, 1, True),
     ([200], 5632, 4096, 2, False), ([128] * 16, 688, 4096, 2, False), ([129] * 16, 688, 4096, 2, True), ([512] * 16, 688, 4096, 2, False),
-    ([640] * 16, 688, 4096, 2, True), ([512] * 8, 14336, 4096, 2, False), ([1024] * 8, 14336, 4096, 2, True), ([512] * 8, 4096, 14336, 0, False), ([511] * 16, 4096, 688, 0, False),
+    ([640] * 16, 688, 4096, 2, True), ([512] * 8, 14336, 4096, 2, True), ([512] * 8, 4096, 14336, 0, False), ([511] * 16, 4096, 688, 0, False),
     ([512] * 16, 4096, 688, 0, True)])
 def test_sides_of_the_line(rows, N, K, kind, pairs):
     assert _takes_pairs(rows, N, K, kind) is pairs

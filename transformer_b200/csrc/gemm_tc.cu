@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
                 }
                 if (FLOAT && wide_float) {
                     // the same for floats: a chunk's 32 columns are a whole line.  (Logits of 1,000 rows, K 2,048, N 32,000, single blocks: 290 us
-                    // row by row, 174 so.)
+                    // row by row, 172 so.)
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         *reinterpret_cast<float4*>(strip + lane * 128 + ((j ^ (lane & 7)) << 4)) =
@@ -551,22 +551,21 @@ static int tc_tiles_n(int N, bool dual) { return (N + (dual ? TC_BN / 2 : TC_BN)
 
 // Pairs of blocks, where they take at most a seventh more rounds over the SMs than single blocks would (a round of theirs takes about 7/8 of the
 // time: B is staged once for 256 rows), counting half a tile of padding a group.  What fits one round stays with single blocks, and so does
-// a short K (below 512, or 1,024 with fewer than 512 rows a group), whose start counts.  Products of a millisecond and more run at the power
-// limit, where what is computed counts, padding with it: from 16 rounds on with K from 4,096 a fourteenth more.  Single blocks / pairs, us
-// (many launches between two events, weights from memory; profiles/gemm_tc_pairs.md has more):
-//   (gate, up) 5,632 wide, K 2,048: 520 rows 29.5 / 27.0, 1,000 45 / 40, 2,048 79 / 69, 4,096 158 / 135; 300 rows 18.0 / 25.6 (1 round, 2)
-//   logits of 32,000 tokens, K 2,048: 200 rows 48 / 35, 500 94 / 67, 1,000 179 / 123; 64 rows 33 / 46
-//   16 experts, (gate, up) 688 wide, K 4,096: 200 rows each 60 / 56, 384 87 / 85, 640 130 / 116, 1,024 182 / 165; 512 99 / 112 (3 rounds, 4)
-//   their down product (4,096 wide, K 688): 512 rows each 62 / 57, 1,024 116 / 98, 2,048 198 / 171; 128 34 / 36
-//   8 experts 14,336 wide, K 4,096: 512 rows each 835 / 993 and 840 / 958 one after the other, 828 / 829 and 777 / 803 in turn (28 rounds,
-//   31), 768 1,240 / 1,169, 1,024 1,544 to 1,703 / 1,338 to 1,606, 2,048 2,904 to 3,088 / 2,538 to 2,995
+// a short K (below 512, or 1,024 with fewer than 512 rows a group), whose start counts.  Single blocks / pairs, us (many launches between two
+// events, weights from memory; profiles/gemm_tc_pairs.md has more):
+//   (gate, up) 5,632 wide, K 2,048: 520 rows 29.3 / 26.8, 1,000 42 / 38, 2,048 73 / 64, 4,096 162 / 137; 300 rows 17.9 / 25.4 (1 round, 2)
+//   logits of 32,000 tokens, K 2,048: 200 rows 49 / 36, 500 93 / 66, 1,000 172 / 128; 64 rows 33 / 41
+//   16 experts, (gate, up) 688 wide, K 4,096: 200 rows each 59 / 55, 384 84 / 80, 640 130 / 114, 1,024 169 / 165; 512 93 / 103 (3 rounds, 4)
+//   their down product (4,096 wide, K 688): 512 rows each 59 / 55, 1,024 113 / 95, 2,048 216 / 181; 128 31 / 33
+//   8 experts 14,336 wide, K 4,096, by themselves at the power limit, where two runs differ by a tenth: 512 rows each 828 / 829 and 777 / 803,
+//   768 1,240 / 1,169, 1,024 1,544 / 1,338, 2,048 2,904 / 2,538; in a model of 32 such layers 2,048 tokens take 56.0 ms / 54.1
 //   2,048 wide, K 128: 3,000 rows 6.8 / 7.5
 static bool tc_takes_pairs(int M, int N, int K, int G, bool grouped, bool dual, int sms) {
     if (M <= TC_BM * (long long)G || K < (M >= 512ll * G ? 512 : 1024)) return false;
     const long long pad = grouped ? G : 0, tiles_n = tc_tiles_n(N, dual);
     const long long single = (((long long)M + TC_BM - 1) / TC_BM + pad / 2) * tiles_n, twos = (((long long)M + 2 * TC_BM - 1) / (2 * TC_BM) + pad / 2) * tiles_n;
     const long long rounds = (single + sms - 1) / sms, pair_rounds = (twos + sms / 2 - 1) / (sms / 2);
-    return rounds >= 2 && (K >= 4096 && rounds >= 16 ? 13 * pair_rounds <= 14 * rounds : 7 * pair_rounds <= 8 * rounds);
+    return rounds >= 2 && 7 * pair_rounds <= 8 * rounds;
 }
 
 // C[m] = A[m] . B[g(m)]^T.  A [M, K] (rows sorted by group), B [G, rows_b, K] with rows_b = N (or 2N when
