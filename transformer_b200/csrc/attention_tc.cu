@@ -21,7 +21,7 @@
 // (it stays below 2^8, exact enough in bfloat16 and float), so the costly read-modify-write of O is
 // rare.  Windows, kept first tokens, chunks, sinks, gates and capped scores are forms of the one kernel (AT_WINDOW, AT_CAPPED; rule and
 // measurements in parts/attention.py); these raise it wherever it grows and have the bits of attention_window_mma.cu (16 heads of 128 over 4
-// key heads, 2,039 tokens, capped: 63.6 us, 58.4 with the older maximum, 109 there).  Warps 0 and 1 run their loops whole and one elected lane issues (see elect_one): 2,048
+// key heads, 2,039 tokens, capped: 66.0 us, 63.6 without at_clear, 58.4 with the older maximum as well, 109 there).  Warps 0 and 1 run their loops whole and one elected lane issues (see elect_one): 2,048
 // tokens of 32 heads of 128 40.9 us where one thread's loops took 45.5, 8 x 1,024 101 (111), 600 behind 1,000 of 8 heads over 2
 // 20 (26).  Bound by the softmax warps' chain a tile.  Every wait on an mbarrier is bounded (see gemm_tc.cu); a wait that runs out sets the error
 // word that tb_gemm_tc_status() reports.

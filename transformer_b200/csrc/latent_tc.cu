@@ -15,7 +15,7 @@
 //             from tensor memory, mask, maximum, weights (back into tensor memory, over the scores they came from), the sum, and
 //             O times the factor by which the maximum moved, where it moved for any row of the warp
 //
-// One prompt of 2,039 tokens, 16 heads, rank 512 + 64: 208 us, 440 with 64 rows a block and mma.sync.  A page takes a block some 7,000
+// One prompt of 2,039 tokens, 16 heads, rank 512 + 64: 212 us, 440 with 64 rows a block and mma.sync.  A page takes a block some 7,000
 // clocks; the products' share is 2,300 (a k-step of the scores reads 6 KB of shared memory for 128 x 64 x 16, 48 clocks), the
 // rest is the chain of the row's thread: scores out of tensor memory, 64 exponentials, 256 sums rescaled while the maximum still moves.
 #include "latent_common.cuh"

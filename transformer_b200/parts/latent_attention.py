@@ -66,8 +66,8 @@ def rows_pay(lens, before, window: int, tile: int, rank: int, blocks: int) -> bo
 def tc_pays(ctx, m) -> bool:
     """Whether a step without slices is faster on the tcgen05 tensor cores (latent_tc.cu) than with 16 or 64 rows a block: from a third
     of the tiles' rows in use on.  us, the faster of those two and tcgen05 (rank 512 + 64, 16 heads): one prompt of 2,039
-    tokens 440 and 208, 4 of 300 88 and 43, 16 of 100 82 and 42, 40 of 16 behind 1,000 244 and 115, 200 of 6 (0.75 in use) 54 and
-    34; not taken: 420 of 2 behind 2,000 (0.25) 574 and 615.  Rank 256 + 32, 8 heads: 2,039 tokens 159 and 76, 200 of 6 (0.38) 17 and 16;
+    tokens 440 and 212, 4 of 300 88 and 45, 16 of 100 82 and 44, 40 of 16 behind 1,000 244 and 118, 200 of 6 (0.75 in use) 54 and
+    36; not taken: 420 of 2 behind 2,000 (0.25) 574 and 615.  Rank 256 + 32, 8 heads: 2,039 tokens 159 and 81, 200 of 6 (0.38) 17 and 17;
     not taken: 420 of 2 behind 300 (0.12) 35 and 47."""
     key = ("latent_tc", m.tc_tile)
     if key not in ctx.plans:
